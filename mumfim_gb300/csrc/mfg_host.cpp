@@ -22,6 +22,7 @@
 
 #include <cuda_runtime.h>
 
+#include "mfg_exact.cuh"
 #include "mfg_internal.h"
 #include "mfg_metrics.h"
 #include "mfg_mixed.h"
@@ -582,7 +583,9 @@ static mfg_status batch_create_impl(const mfg_network* nets, const mfg_strategy*
   const int64_t nt = no, et = fo;
 
   // ---- pack ------------------------------------------------------------
-  std::vector<double> X(3 * nt), m(nt), l0(et);
+  // FP64 batches: 1 / m and m c follow the masses, 1 / l0 the lengths
+  const bool f64 = b->precision == MFG_PREC_F64;
+  std::vector<double> X(3 * nt), m(f64 ? 3 * nt : nt), l0(f64 ? 2 * et : et);
   std::vector<int2> conn(et);
   std::vector<int32_t> rowptr(ro), inc(io), bnd(std::max<int64_t>(bo, 1));
   parallel_for(n_rve, [&](int r) {
@@ -596,6 +599,14 @@ static mfg_status batch_create_impl(const mfg_network* nets, const mfg_strategy*
     std::memcpy(&l0[d.fiber_off], s.l0.data(), s.n_fibers * sizeof(double));
     std::memcpy(&rowptr[d.row_off], s.rowptr.data(), (N + 1) * sizeof(int32_t));
     std::memcpy(&inc[d.inc_off], s.inc.data(), 2 * s.n_fibers * sizeof(int32_t));
+    if (f64) {
+      for (int i = 0; i < N; ++i) {
+        m[nt + d.node_off + i] = mfg::exact_reciprocal(s.m[i]);
+        m[2 * nt + d.node_off + i] = s.m[i] * d.c;
+      }
+      for (int e = 0; e < s.n_fibers; ++e)
+        l0[et + d.fiber_off + e] = mfg::exact_reciprocal(s.l0[e]);
+    }
     if (!s.bnd_order.empty())
       std::memcpy(&bnd[d.bnd_off], s.bnd_order.data(), s.bnd_order.size() * sizeof(int32_t));
   });
@@ -654,8 +665,11 @@ static mfg_status batch_create_impl(const mfg_network* nets, const mfg_strategy*
   dv.u = b->d_u.p;
   dv.v = b->d_v.p;
   dv.m = b->d_m.p;
+  dv.rm = b->d_m.p + (f64 ? nt : 0);
+  dv.mc = b->d_m.p + (f64 ? 2 * nt : 0);
   dv.conn = b->d_conn.p;
   dv.l0 = b->d_l0.p;
+  dv.rl0 = b->d_l0.p + (f64 ? et : 0);
   dv.nrm = b->d_nrm.p;
   dv.fint = b->d_fint.p;
   dv.rowptr = b->d_rowptr.p;
@@ -1093,6 +1107,7 @@ struct PendingReq {
 // working set when used), for admission against the HBM budget.
 double batch_bytes(int64_t nt, int64_t et, int64_t nbt, int64_t R, bool mixed) {
   double b = nt * (5 * 3 * 8.0 + 8 + 4) + et * (8.0 + 8 + 24 + 8) + nbt * (48.0 + 4) + R * 200.0;
+  if (!mixed) b += nt * 16.0 + et * 8.0;  // 1 / m, m c, 1 / l0
   if (mixed)  // + node-centric incidences (about 2.3 per fiber, with the set-up fiber ids)
     b += nt * (24.0 + 12 + 8 + 4 + 4 + 8 + 8) + et * (16.0 + 16 + 16 + 8 + 8 + 4 + 64) + R * 20.0;
   return b;

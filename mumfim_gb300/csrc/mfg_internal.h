@@ -57,8 +57,11 @@ struct DevBatch {
   double* u;         // 3 * nt displacement
   double* v;         // 3 * nt velocity
   const double* m;   // nt lumped mass
+  const double* rm;  // nt 1 / mass for div_known(), and mass times damping (FP64 batches)
+  const double* mc;
   const int2* conn;  // et fiber end nodes (RVE-local ids)
   const double* l0;  // et reference lengths
+  const double* rl0; // et 1 / length for div_known() (FP64 batches)
   double* nrm;       // 3 * et per-fiber force vectors (scratch)
   double* fint;      // 3 * nt internal force (boundary rows used by the stress)
   const int32_t* rowptr;  // per RVE n_nodes + 1 offsets into that RVE's incidences

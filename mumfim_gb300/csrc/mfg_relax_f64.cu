@@ -8,7 +8,8 @@
 //
 // Bit-exactness with a serial run of the same algorithm:
 //  - this file is compiled with --fmad=false and every expression keeps the
-//    reference's operation order; division and sqrt are IEEE (nvcc default);
+//    reference's operation order; quotients and square roots are correctly
+//    rounded (mfg_exact.cuh, or the IEEE operations where it does not apply);
 //  - nodal forces are gathered node by node over a CSR list of incident
 //    fibers in ascending fiber id, which adds the per-fiber force vectors in
 //    exactly the order the serial scatter f_int[n1] -= t; f_int[n2] += t
@@ -26,12 +27,20 @@
 //   node pass  : f = gather(nrm); v += h_s f/m; v += h_{s+1} f/m; x += 2h_{s+1} v
 //   fiber pass : l = |x2 - x1|; T = law(l0, l); nrm = (x2 - x1) * (T / l)
 // giving two block barriers per step.
+//
+// What bounds it: the FP64 pipe, 2 lanes per clock and SM (82 % busy over 304
+// RVEs of 4,500 nodes). The general divisions and square root, a second
+// quotient h f / m for the trailing kick and a minimum no step needed made
+// 84 FP64 instructions a fiber and step; the forms of mfg_exact.cuh and one
+// quotient for both kicks leave 52, the same bits. 256 RVEs of 4,500 nodes:
+// 4.3e9 -> 7.8e9 fiber-steps/s.
 #include <cfloat>
 #include <climits>
 
 #include "mumfim_gpu.h"
 
 #include "mfg_common.cuh"
+#include "mfg_exact.cuh"
 #include "mfg_internal.h"
 
 namespace mfg {
@@ -39,49 +48,110 @@ namespace {
 
 constexpr int kThreadsF64 = 256;
 
-// BatchedFiberRVEAnalysisExplicitBase.h:155-172
-__device__ __forceinline__ double linear_force(double orig_length, double length, double E,
-                                               double A) {
-  double length_ratio = length / orig_length;
-  double green_strain = 1.0 / 2.0 * (length_ratio * length_ratio - 1);
-  return length_ratio * E * A * green_strain;
+// Reaction law of one RVE with everything that does not depend on the fiber
+// formed once, by the expressions the reference forms per fiber.
+//
+// Linear (BatchedFiberRVEAnalysisExplicitBase.h:155-172):
+//   T = lr E A g,  g = 1/2 (lr^2 - 1),  lr = l / l0
+// Nonlinear (NonlinearReaction::forceReaction().first, src/mumfim/microscale/
+// FiberReactions.cc:16-71; compressive transition ratio 1.0,
+// FiberNetworkIO_impl.h:35), with alpha = E A / B:
+//   toe        alpha lr (e^(B g) - 1)
+//   beyond it  m (lr - r) l0 + b at a transition ratio r (lt above, 1 below),
+//              m = alpha / l0 ((1 + r^2 B) e^(B g_r) - 1), b the toe's force at r
+struct LawF64 {
+  bool nonlinear;
+  bool exact;  // E A (half_E, below) and alpha (div_known) are far from underflow
+  double half_E, A;  // half_E = E / 2: the linear law's factor 1/2, moved to where it is exact
+  double alpha, B, lt, kt, bt, kc, bc;
+};
+
+__device__ __forceinline__ LawF64 make_law_f64(const RveDesc& d) {
+  LawF64 L;
+  L.nonlinear = d.law == 1;
+  L.half_E = 0.5 * d.E;
+  L.A = d.A;
+  L.alpha = L.B = L.lt = L.kt = L.bt = L.kc = L.bc = 0.0;
+  if (L.nonlinear) {
+    const double cmp = 1.0;
+    L.alpha = d.E * d.A / d.B;
+    L.B = d.B;
+    L.lt = d.lt;
+    const double gt = 1.0 / 2.0 * (d.lt * d.lt - 1);
+    const double gc = 1.0 / 2.0 * (cmp * cmp - 1);
+    L.kt = (1 + d.lt * d.lt * d.B) * exp(d.B * gt) - 1;
+    L.bt = L.alpha * d.lt * (exp(d.B * gt) - 1);
+    L.kc = (1 + cmp * cmp * d.B) * exp(d.B * gc) - 1;
+    L.bc = L.alpha * cmp * (exp(d.B * gc) - 1);
+  }
+  L.exact = in_range(d.E) && in_range(d.E * d.A) && (!L.nonlinear || in_range(L.alpha));
+  return L;
 }
 
-// NonlinearReaction::forceReaction().first (src/mumfim/microscale/FiberReactions.cc:16-71),
-// compressive transition ratio 1.0 (FiberNetworkIO_impl.h:35).
-__device__ __forceinline__ double nl_force(double alpha, double B, double lr, double gs) {
-  return alpha * lr * (exp(B * gs) - 1);
+// Force at length ratio lr of a fiber of reference length l0; alpha_l0 =
+// alpha / l0 (nonlinear law only).
+__device__ __forceinline__ double reaction_force(const LawF64& L, double lr, double l0,
+                                                 double alpha_l0) {
+  if (!L.nonlinear) return lr * L.half_E * L.A * (lr * lr - 1);
+  if (lr > L.lt) return alpha_l0 * L.kt * (lr - L.lt) * l0 + L.bt;
+  if (lr < 1.0) return alpha_l0 * L.kc * (lr - 1.0) * l0 + L.bc;
+  const double gs = 1.0 / 2.0 * (lr * lr - 1);
+  return L.alpha * lr * (exp(L.B * gs) - 1);
 }
-__device__ __forceinline__ double nl_deriv(double alpha, double B, double lr, double l0,
-                                           double gs) {
-  return alpha / l0 * ((1 + lr * lr * B) * exp(B * gs) - 1);
+
+// Force vector d T / l of one fiber with end-to-end vector d, by the general
+// operations: the numbers fiber_vector() does not take. Returns l.
+__device__ __noinline__ double fiber_vector_general(const LawF64& L, const double d[3], double l0,
+                                                    double n[3]) {
+  const double l = sqrt(d[0] * d[0] + d[1] * d[1] + d[2] * d[2]);
+  const double lr = l / l0;
+  const double T = L.nonlinear ? reaction_force(L, lr, l0, L.alpha / l0)
+                               : lr * (2.0 * L.half_E) * L.A * (0.5 * (lr * lr - 1));
+  const double q = T / l;
+  for (int k = 0; k < 3; ++k) n[k] = d[k] * q;
+  return l;
 }
-__device__ __forceinline__ double nonlinear_force(double orig_length, double length, double E,
-                                                  double A, double B, double lt) {
-  const double cmp = 1.0;
-  double length_ratio = length / orig_length;
-  double alpha = E * A / B;
-  if (length_ratio > lt) {
-    double gt = 1.0 / 2.0 * (lt * lt - 1);
-    double m = nl_deriv(alpha, B, lt, orig_length, gt);
-    double b = nl_force(alpha, B, lt, gt);
-    return m * (length_ratio - lt) * orig_length + b;
-  } else if (length_ratio < cmp) {
-    double gc = 1.0 / 2.0 * (cmp * cmp - 1);
-    double m = nl_deriv(alpha, B, cmp, orig_length, gc);
-    double b = nl_force(alpha, B, cmp, gc);
-    return m * (length_ratio - cmp) * orig_length + b;
+
+// The same, with the square root and the three quotients of mfg_exact.cuh
+// (rl0 = RN(1 / l0), or 0 to ask for the general operations): 33 FP64
+// instructions on the linear law instead of 45, the same bits.
+__device__ __forceinline__ double fiber_vector(const LawF64& L, const double d[3], double l0,
+                                               double rl0, double n[3]) {
+  const double s = d[0] * d[0] + d[1] * d[1] + d[2] * d[2];
+  double l, y;
+  sqrt_recip(s, rsqrt_start(s), l, y);
+  const double lr = div_known(l, l0, rl0);
+  const double T =
+      reaction_force(L, lr, l0, L.nonlinear ? div_known(L.alpha, l0, rl0) : 0.0);
+  if (L.exact && in_range(s) && hi_word(rl0) != 0 && !all_ones(l) && (in_range(T) || is_zero(T))) {
+    const double q = div_known(T, l, y);
+    n[0] = d[0] * q; n[1] = d[1] * q; n[2] = d[2] * q;
+    return l;
   }
-  double gs = 1.0 / 2.0 * (length_ratio * length_ratio - 1);
-  return nl_force(alpha, B, length_ratio, gs);
+  return fiber_vector_general(L, d, l0, n);
+}
+
+// x / m for a node's mass (rm = RN(1 / m), or 0): div_known() where it
+// applies. The general division is a call: inlined, the compiler runs it
+// ahead of the test on every node (12 FP64 instructions a fiber, measured).
+__device__ __noinline__ double general_quotient(double x, double m) { return x / m; }
+
+__device__ __forceinline__ double over_mass(double x, double m, double rm) {
+  if ((in_range(x) && hi_word(rm) != 0) || is_zero(x)) return div_known(x, m, rm);
+  return general_quotient(x, m);
+}
+
+// x with its sign flipped where `flip`; no FP64 instruction.
+__device__ __forceinline__ double flip_sign(double x, bool flip) {
+  return __hiloint2double(__double2hiint(x) ^ (flip ? 0x80000000 : 0), __double2loint(x));
 }
 
 struct RveView {
   const double *X0, *X1, *X2;
   double *x0, *x1, *x2, *u0, *u1, *u2, *v0, *v1, *v2;
-  const double* m;
+  const double *m, *rm, *mc;
   const int2* conn;
-  const double* l0;
+  const double *l0, *rl0;
   double *n0, *n1, *n2;
   double *fi0, *fi1, *fi2;
   const int32_t* rowptr;
@@ -97,9 +167,9 @@ __device__ __forceinline__ RveView make_view(const DevBatch& b, const RveDesc& d
   r.u0 = b.u + no; r.u1 = b.u + nt + no; r.u2 = b.u + 2 * nt + no;
   r.v0 = b.v + no; r.v1 = b.v + nt + no; r.v2 = b.v + 2 * nt + no;
   r.fi0 = b.fint + no; r.fi1 = b.fint + nt + no; r.fi2 = b.fint + 2 * nt + no;
-  r.m = b.m + no;
+  r.m = b.m + no; r.rm = b.rm + no; r.mc = b.mc + no;
   r.conn = b.conn + fo;
-  r.l0 = b.l0 + fo;
+  r.l0 = b.l0 + fo; r.rl0 = b.rl0 + fo;
   r.n0 = b.nrm + fo; r.n1 = b.nrm + et + fo; r.n2 = b.nrm + 2 * et + fo;
   r.rowptr = b.rowptr + d.row_off;
   r.inc = b.inc + d.inc_off;
@@ -109,49 +179,67 @@ __device__ __forceinline__ RveView make_view(const DevBatch& b, const RveDesc& d
 
 // f_int of node i: incident fiber vectors in ascending fiber id, subtracted at
 // the fiber's first node and added at its second
-// (BatchedFiberRVEAnalysisExplicitBase.h:246-251 in serial order).
+// (BatchedFiberRVEAnalysisExplicitBase.h:246-251 in serial order). The first
+// one is taken as it is: adding it to zero changes no bit but a zero's sign.
 __device__ __forceinline__ void gather_fint(const RveView& r, int i, double& a0, double& a1,
                                             double& a2) {
   a0 = 0.0; a1 = 0.0; a2 = 0.0;
-  const int pb = r.rowptr[i], pe = r.rowptr[i + 1];
-  for (int p = pb; p < pe; ++p) {
+  const int pb = __ldg(r.rowptr + i), pe = __ldg(r.rowptr + i + 1);
+  if (pb == pe) return;
+  {
+    const int code = __ldg(r.inc + pb);
+    const int e = code >> 1;
+    const bool neg = !(code & 1);
+    a0 = flip_sign(r.n0[e], neg); a1 = flip_sign(r.n1[e], neg); a2 = flip_sign(r.n2[e], neg);
+  }
+  for (int p = pb + 1; p < pe; ++p) {
     const int code = __ldg(r.inc + p);
     const int e = code >> 1;
-    const double t0 = r.n0[e], t1 = r.n1[e], t2 = r.n2[e];
-    if (code & 1) {
-      a0 = a0 + t0; a1 = a1 + t1; a2 = a2 + t2;
-    } else {
-      a0 = a0 - t0; a1 = a1 - t1; a2 = a2 - t2;
-    }
+    const bool neg = !(code & 1);
+    a0 = a0 + flip_sign(r.n0[e], neg);
+    a1 = a1 + flip_sign(r.n1[e], neg);
+    a2 = a2 + flip_sign(r.n2[e], neg);
   }
 }
 
 // Fiber pass: lengths, reaction force and per-fiber force vector
 // (TeamOuterLoop.h:53-82 and BatchedFiberRVEAnalysisExplicitBase.h:203-252).
-// Returns this thread's minimum length.
-__device__ __forceinline__ double fiber_pass(const RveView& r, const RveDesc& d) {
+// Returns this thread's minimum length when kLen (every 100th step; an FP64
+// minimum is an instruction of the pipe that bounds the kernel).
+template <bool kLen>
+__device__ __forceinline__ double fiber_pass(const RveView& r, const RveDesc& d, const LawF64& L) {
   double lmin = DBL_MAX;
   for (int e = threadIdx.x; e < d.n_fibers; e += kThreadsF64) {
     const int2 c = __ldg(r.conn + e);
-    const double d0 = r.x0[c.y] - r.x0[c.x];
-    const double d1 = r.x1[c.y] - r.x1[c.x];
-    const double d2 = r.x2[c.y] - r.x2[c.x];
-    const double l = sqrt(d0 * d0 + d1 * d1 + d2 * d2);
-    lmin = fmin(lmin, l);
-    const double l0 = __ldg(r.l0 + e);
-    const double frc = d.law == 1 ? nonlinear_force(l0, l, d.E, d.A, d.B, d.lt)
-                                  : linear_force(l0, l, d.E, d.A);
-    const double frc_ovr_l = frc / l;
-    r.n0[e] = d0 * frc_ovr_l;
-    r.n1[e] = d1 * frc_ovr_l;
-    r.n2[e] = d2 * frc_ovr_l;
+    const double dv[3] = {r.x0[c.y] - r.x0[c.x], r.x1[c.y] - r.x1[c.x], r.x2[c.y] - r.x2[c.x]};
+    double n[3];
+    const double l = fiber_vector(L, dv, __ldg(r.l0 + e), __ldg(r.rl0 + e), n);
+    if (kLen) lmin = fmin(lmin, l);
+    r.n0[e] = n[0];
+    r.n1[e] = n[1];
+    r.n2[e] = n[2];
   }
   return lmin;
+}
+
+// One node's trailing kick of the last step and leading kick of this one from
+// its internal force a, in place on the velocity w
+// (BatchedFiberRVEAnalysisExplicitBase.h:253-287, TeamOuterLoop.h:157-175).
+// Between refreshes of the time step both half kicks add the same quotient
+// h f / m, formed once
+// (`same`).
+__device__ __forceinline__ void kick(double a, double m, double rm, double mc, double h_prev,
+                                     double h, bool first, bool same, double& w) {
+  const double f = -(a + mc * w);  // f = -f_int - c m v
+  const double q = over_mass(h * f, m, rm);
+  if (!first) w += same ? q : over_mass(h_prev * f, m, rm);
+  w += q;
 }
 
 __device__ void solve_rve(const DevBatch& b, const RunArgs& a, int rve, double* red) {
   const RveDesc d = b.desc[rve];
   const RveView r = make_view(b, d);
+  const LawF64 L = make_law_f64(d);
   const int N = d.n_nodes, NF = d.n_free;
   const int tid = threadIdx.x;
   const double* F = a.F + 9 * (a.n_F > 1 ? rve : 0);
@@ -185,7 +273,7 @@ __device__ void solve_rve(const DevBatch& b, const RunArgs& a, int rve, double* 
   __syncthreads();
 
   // ---- RunInitialization: lengths, dt_crit, first forces -----------------
-  double dt_crit = block_min<kThreadsF64>(fiber_pass(r, d), red) / d.sound_speed;
+  double dt_crit = block_min<kThreadsF64>(fiber_pass<true>(r, d, L), red) / d.sound_speed;
 
   // ---- main loop ---------------------------------------------------------
   const int cap = d.max_steps;  // host resolves the default cap for RELAX
@@ -215,30 +303,21 @@ __device__ void solve_rve(const DevBatch& b, const RunArgs& a, int rve, double* 
     if (!ramp && res_step && !(residual > d.tol)) break;
     if (step >= cap) break;  // RAMP: exactly max_steps steps; RELAX: cap reached
     const double h = d.crit * dt_crit * 0.5;  // TeamOuterLoop.h:345
+    const double h2 = 2 * h;
+    const bool same = h == h_prev;
     // node pass: trailing kick of step-1, leading kick + drift of step
     for (int i = tid; i < NF; i += kThreadsF64) {
       double a0, a1, a2;
       gather_fint(r, i, a0, a1, a2);
-      const double mass = r.m[i];
-      const double mc = mass * d.c;
+      const double mass = __ldg(r.m + i), rm = __ldg(r.rm + i), mc = __ldg(r.mc + i);
       double w0 = r.v0[i], w1 = r.v1[i], w2 = r.v2[i];
-      // f = -f_int - c m v (BatchedFiberRVEAnalysisExplicitBase.h:253-274)
-      const double f0 = -a0 - mc * w0;
-      const double f1 = -a1 - mc * w1;
-      const double f2 = -a2 - mc * w2;
-      if (step > 0) {  // updateAccelVel (BatchedFiberRVEAnalysisExplicitBase.h:275-287)
-        w0 += h_prev * f0 / mass;
-        w1 += h_prev * f1 / mass;
-        w2 += h_prev * f2 / mass;
-      }
-      // updates (TeamOuterLoop.h:157-175)
-      w0 = w0 + h * f0 / mass;
-      w1 = w1 + h * f1 / mass;
-      w2 = w2 + h * f2 / mass;
+      kick(a0, mass, rm, mc, h_prev, h, step == 0, same, w0);
+      kick(a1, mass, rm, mc, h_prev, h, step == 0, same, w1);
+      kick(a2, mass, rm, mc, h_prev, h, step == 0, same, w2);
       r.v0[i] = w0; r.v1[i] = w1; r.v2[i] = w2;
-      r.x0[i] = r.x0[i] + 2 * h * w0;
-      r.x1[i] = r.x1[i] + 2 * h * w1;
-      r.x2[i] = r.x2[i] + 2 * h * w2;
+      r.x0[i] = r.x0[i] + h2 * w0;
+      r.x1[i] = r.x1[i] + h2 * w1;
+      r.x2[i] = r.x2[i] + h2 * w2;
     }
     if (ramp) {
       const double alpha = static_cast<double>(step + 1) / static_cast<double>(d.max_steps);
@@ -250,10 +329,10 @@ __device__ void solve_rve(const DevBatch& b, const RunArgs& a, int rve, double* 
       }
     }
     __syncthreads();
-    const double lmin = fiber_pass(r, d);
     if (step % kUpdateFreq == 0) {
-      dt_crit = block_min<kThreadsF64>(lmin, red) / d.sound_speed;
+      dt_crit = block_min<kThreadsF64>(fiber_pass<true>(r, d, L), red) / d.sound_speed;
     } else {
+      fiber_pass<false>(r, d, L);
       __syncthreads();
     }
     h_prev = h;

@@ -1,0 +1,95 @@
+// Checks mfg_exact.cuh on the host: div_known() and sqrt_recip() against the
+// general operations, on random operands and on operands next to a rounding
+// boundary (where an approximate correction would round the wrong way).
+//  - quotients x / d that lie k / (2^54 d) of an ulp from a midpoint, k odd and
+//    small: Q d + k = 2^54 x is solved for the 54-bit midpoint Q (d odd);
+//  - square roots next to a midpoint M + 1/2: M^2 + M + j = 0 mod 2^52 is
+//    solved for M by Newton's iteration in 2-adic integers, so that
+//    s = M^2 + M + j has 53 significant bits.
+// The start of sqrt_recip() is perturbed by up to 2^-19, the error it allows.
+// Prints "bad=0" and exits 0 when every result is the general operation's.
+#include <cstdint>
+#include <cstdio>
+#include <random>
+
+#include "mfg_exact.cuh"
+
+using namespace mfg;
+
+namespace {
+
+std::mt19937_64 rng(11);
+long bad = 0;
+
+uint64_t inverse(uint64_t a) {  // of an odd a, mod 2^64
+  uint64_t x = a;
+  for (int i = 0; i < 6; ++i) x *= 2 - a * x;
+  return x;
+}
+
+double significand() { return std::ldexp(static_cast<double>((rng() >> 11) | (1ull << 52)), -52); }
+
+void check_div(double x, double d) {
+  const double rd = exact_reciprocal(d);
+  if (rd == 0.0 || !in_range(x) || div_known(x, d, rd) != x / d) {
+    if (++bad <= 10) std::printf("div %a / %a\n", x, d);
+  }
+}
+
+void check_sqrt(double s) {
+  const double off = (static_cast<double>(rng() % 2001) - 1000.0) / 1000.0;
+  double l, y;
+  sqrt_recip(s, 1.0 / std::sqrt(s) * (1.0 + std::ldexp(off, -19)), l, y);
+  if (!in_range(s) || l != std::sqrt(s) || (!all_ones(l) && y != 1.0 / l)) {
+    if (++bad <= 10) std::printf("sqrt %a: %a, %a\n", s, l, y);
+  }
+}
+
+}  // namespace
+
+int main() {
+  long n = 0;
+  for (long t = 0; t < 4000000; ++t) {  // hard quotients
+    const uint64_t M = (rng() >> 11) | (1ull << 52) | 1;
+    const int64_t k = 2 * static_cast<int64_t>(rng() % 16) - 15;
+    const uint64_t Q = (0 - static_cast<uint64_t>(k)) * inverse(M) & ((1ull << 54) - 1);
+    if (!(Q >> 53)) continue;
+    const unsigned __int128 P = static_cast<unsigned __int128>(Q) * M + static_cast<__int128>(k);
+    const uint64_t X = static_cast<uint64_t>(P >> 54);
+    if (X == 0 || X >> 53) continue;
+    const int e = static_cast<int>(rng() % 140) - 70;
+    check_div(std::ldexp(static_cast<double>(X), e), static_cast<double>(M));
+    ++n;
+  }
+  for (int t = 0; t < 2000000; ++t) {
+    check_div(std::ldexp(significand(), static_cast<int>(rng() % 1500) - 750),
+              std::ldexp(significand(), static_cast<int>(rng() % 190) - 95));
+    check_sqrt(std::ldexp(significand(), static_cast<int>(rng() % 1500) - 750));
+  }
+  for (uint64_t k = 0; k < 2000; ++k) {  // next to powers of two
+    check_sqrt(1.0 + static_cast<double>(k) * 0x1p-52);
+    check_sqrt(2.0 - static_cast<double>(k + 1) * 0x1p-52);
+    check_sqrt(4.0 - static_cast<double>(k + 1) * 0x1p-51);
+    check_div(2.0 - static_cast<double>(k + 1) * 0x1p-52, 2.0 - 0x1p-52);
+    check_div(1.0 + static_cast<double>(k) * 0x1p-52, 2.0 - 0x1p-52);
+  }
+  for (int64_t j = -4000; j <= 4000; j += 2)  // hard square roots
+    for (uint64_t root = 0; root < 2; ++root) {
+      uint64_t M = root;
+      for (int i = 0; i < 8; ++i)
+        M -= (M * M + M + static_cast<uint64_t>(j)) * inverse(2 * M + 1);
+      for (int bits = 52; bits <= 53; ++bits) {
+        const uint64_t m = (M & ((1ull << bits) - 1)) | (bits == 52 ? 1ull << 52 : 0);
+        if (m < (1ull << 52) || m >= (1ull << 53)) continue;
+        unsigned __int128 S = static_cast<unsigned __int128>(m) * m + m + static_cast<__int128>(j);
+        int shift = 0;
+        while (!(S & 1)) S >>= 1, ++shift;
+        if (S >> 53) continue;
+        check_sqrt(std::ldexp(static_cast<double>(static_cast<uint64_t>(S)), shift));
+        check_sqrt(std::ldexp(static_cast<double>(static_cast<uint64_t>(S)), shift - 130));
+        ++n;
+      }
+    }
+  std::printf("hard cases %ld bad=%ld\n", n, bad);
+  return bad != 0 || n < 100000;
+}
