@@ -23,6 +23,7 @@
 #include <cuda_runtime.h>
 
 #include "mfg_exact.cuh"
+#include "mfg_f64_order.h"
 #include "mfg_internal.h"
 #include "mfg_metrics.h"
 #include "mfg_mixed.h"
@@ -333,6 +334,13 @@ struct mfg_batch {
   DevArray<int32_t> d_status, d_steps;
   DevArray<mfg_rve_status> d_st;
   mfg::DevBatch dev{};
+  // FP64: every RVE split over a cluster of f64_plan.cl CTAs, f64_clusters of
+  // them at once (cl 1: no clusters), and whether the six concurrent solves
+  // of the stiffness run that way too
+  mfg::F64Plan f64_plan{1, 0};
+  int f64_clusters = 0;
+  bool f64_stiffness_clusters = false;
+  DevArray<unsigned char> d_plan;
   std::unique_ptr<mfg::MixedState, mfg::MixedStateDeleter> mixed;
   int stiffness = MFG_STIFFNESS_AUTO;
   bool all_ramp = false;
@@ -350,6 +358,7 @@ struct mfg_batch {
     for (auto* a : {&d_rowptr, &d_inc, &d_bnd, &d_order, &d_queue, &d_status, &d_steps})
       a->release();
     d_st.release();
+    d_plan.release();
     for (auto* e : {&ev_run0, &ev_relax0, &ev_relax1, &ev_run1})
       if (*e) cudaEventDestroy(*e);
     if (stream) cudaStreamDestroy(stream);
@@ -392,6 +401,126 @@ mfg_status upload(DevArray<T>& d, const std::vector<T>& h, cudaStream_t s) {
   return MFG_OK;
 }
 
+// FP64: chooses the cluster size for the batch (f64_cluster_size) and, when
+// it is above 1, builds and uploads the RVEs' parts (f64_parts). `m` holds
+// the masses, 1 / m and m c, `l0` the lengths and 1 / l0, `nt` and `et` apart.
+mfg_status plan_f64_clusters(mfg_batch* b, const std::vector<double>& m,
+                             const std::vector<double>& l0, const std::vector<int2>& conn,
+                             const std::vector<int32_t>& rowptr, const std::vector<int32_t>& inc,
+                             cudaStream_t s) {
+  int clusters[5] = {b->sms, 0, 0, 0, 0};
+  for (int k = 1; k < 5; ++k)
+    clusters[k] = mfg::relax_f64_max_clusters(1 << k, mfg::kF64ClusterSmem, b->sms);
+  const int64_t nt = b->nt, et = b->et;
+  std::vector<mfg::F64Parts> parts(b->R);  // per RVE, offsets from its own start
+  int cl = 1;
+  for (;;) {
+    cl = mfg::f64_cluster_size(b->desc, clusters, 1);
+    if (cl == 1) return MFG_OK;
+    std::atomic<bool> fits{true};
+    parallel_for(b->R, [&](int r) {
+      const mfg::RveDesc& d = b->desc[r];
+      parts[r] = mfg::F64Parts();
+      mfg::f64_parts(d, cl, conn.data() + d.fiber_off, rowptr.data() + d.row_off,
+                     inc.data() + d.inc_off, parts[r]);
+      for (const mfg::F64Part& p : parts[r].part)
+        if (mfg::f64_part_bytes(p) > mfg::kF64ClusterSmem) fits = false;
+    });
+    if (fits) break;
+    for (int k = 1; k < 5; ++k)  // this size does not hold every RVE
+      if (1 << k == cl) clusters[k] = 0;
+  }
+  // first node, row, incidence and fiber of every RVE, then one allocation
+  // and one copy for all arrays
+  struct At {
+    int64_t node = 0, row = 0, inc = 0, fib = 0;
+  };
+  std::vector<At> at(b->R + 1);
+  for (int r = 0; r < b->R; ++r) {
+    const mfg::F64Parts& p = parts[r];
+    at[r + 1] = {at[r].node + static_cast<int64_t>(p.gnode.size()),
+                 at[r].row + static_cast<int64_t>(p.rows.size()),
+                 at[r].inc + static_cast<int64_t>(p.inc.size()),
+                 at[r].fib + static_cast<int64_t>(p.ends.size())};
+  }
+  const At& n = at[b->R];
+  size_t bytes = 0;
+  auto take = [&](int64_t count, size_t size) {
+    const size_t first = bytes;
+    bytes += (static_cast<size_t>(count) * size + 255) & ~static_cast<size_t>(255);
+    return first;
+  };
+  const size_t o_part = take(static_cast<int64_t>(b->R) * cl, sizeof(mfg::F64Part));
+  const size_t o_gnode = take(n.node, sizeof(int32_t));
+  const size_t o_mass = take(n.node, sizeof(mfg::F64Mass));
+  const size_t o_rows = take(n.row, sizeof(int32_t));
+  const size_t o_inc = take(n.inc, sizeof(int32_t));
+  const size_t o_ends = take(n.fib, sizeof(int2));
+  const size_t o_len = take(n.fib, sizeof(double2));
+  std::vector<unsigned char> blob(bytes);
+  parallel_for(b->R, [&](int r) {
+    mfg::F64Parts& p = parts[r];
+    const mfg::RveDesc& d = b->desc[r];
+    for (mfg::F64Part& q : p.part) {
+      q.node_off += at[r].node;
+      q.row_off += at[r].row;
+      q.inc_off += at[r].inc;
+      q.fib_off += at[r].fib;
+    }
+    auto put = [&](size_t first, int64_t index, const auto& v) {
+      if (!v.empty())
+        std::memcpy(&blob[first + static_cast<size_t>(index) * sizeof(v[0])], v.data(),
+                    v.size() * sizeof(v[0]));
+    };
+    put(o_part, static_cast<int64_t>(r) * cl, p.part);
+    put(o_gnode, at[r].node, p.gnode);
+    put(o_rows, at[r].row, p.rows);
+    put(o_inc, at[r].inc, p.inc);
+    put(o_ends, at[r].fib, p.ends);
+    mfg::F64Mass* mass = reinterpret_cast<mfg::F64Mass*>(&blob[o_mass]) + at[r].node;
+    for (size_t t = 0; t < p.gnode.size(); ++t) {
+      const int64_t i = d.node_off + p.gnode[t];
+      mass[t] = {m[i], m[nt + i], m[2 * nt + i]};
+    }
+    double2* len = reinterpret_cast<double2*>(&blob[o_len]) + at[r].fib;
+    for (size_t e = 0; e < p.slot.size(); ++e) {
+      const int64_t i = d.fiber_off + p.slot[e];
+      len[e] = make_double2(l0[i], l0[et + i]);
+    }
+  });
+  mfg_status st = upload(b->d_plan, blob, s);
+  if (st != MFG_OK) return st;
+  MFG_CUDA(cudaStreamSynchronize(s));  // the blob goes out of scope
+  mfg::F64Plan& plan = b->f64_plan;
+  plan.cl = cl;
+  plan.smem_bytes = mfg::kF64ClusterSmem;
+  const unsigned char* base = b->d_plan.p;
+  plan.part = reinterpret_cast<const mfg::F64Part*>(base + o_part);
+  plan.gnode = reinterpret_cast<const int32_t*>(base + o_gnode);
+  plan.mass = reinterpret_cast<const mfg::F64Mass*>(base + o_mass);
+  plan.rows = reinterpret_cast<const int32_t*>(base + o_rows);
+  plan.inc = reinterpret_cast<const int32_t*>(base + o_inc);
+  plan.ends = reinterpret_cast<const int2*>(base + o_ends);
+  plan.len = reinterpret_cast<const double2*>(base + o_len);
+  int k = 0;
+  while (1 << k < cl) ++k;
+  b->f64_clusters = clusters[k];
+  b->f64_stiffness_clusters =
+      mfg::f64_batch_step_us(b->desc, k, clusters[k], kStiffSlots) <
+      mfg::f64_batch_step_us(b->desc, 0, b->sms, kStiffSlots);
+  return MFG_OK;
+}
+
+// One FP64 solve of the batch view `dev` on `s`: one launch.
+cudaError_t launch_f64(const mfg_batch* b, const mfg::DevBatch& dev, const mfg::RunArgs& a,
+                       bool clusters, cudaStream_t s) {
+  if (clusters && b->f64_plan.cl > 1)
+    return mfg::launch_relax_f64_cluster(
+        dev, a, b->f64_plan, b->f64_plan.cl * std::min(b->R, b->f64_clusters), s);
+  const int grid = std::min(b->R, b->sms * mfg::relax_f64_max_blocks_per_sm(0));
+  return mfg::launch_relax_f64(dev, a, 0, grid, s);
+}
+
 mfg_status enqueue_run(mfg_batch* b, const double* F_dev, int32_t n_F, double* sigma_dev,
                        int32_t update_coords, cudaStream_t s) {
   MFG_CUDA(cudaMemsetAsync(b->d_queue.p, 0, sizeof(int32_t), s));
@@ -408,9 +537,7 @@ mfg_status enqueue_run(mfg_batch* b, const double* F_dev, int32_t n_F, double* s
   if (b->precision == MFG_PREC_MIXED) {
     e = mfg::run_mixed(*b->mixed, b->dev, a, s, &b->last_launches);
   } else {
-    int occ = mfg::relax_f64_max_blocks_per_sm(0);
-    int grid = std::min(b->R, b->sms * occ);
-    e = mfg::launch_relax_f64(b->dev, a, 0, grid, s);
+    e = launch_f64(b, b->dev, a, true, s);
     b->last_launches = 1;
   }
   if (e != cudaSuccess)
@@ -685,6 +812,10 @@ static mfg_status batch_create_impl(const mfg_network* nets, const mfg_strategy*
     // so that mfg_batch_run_device_noalloc() never reserves it mid-solve.
     void* scratch = nullptr;
     MFG_CUDA(mfg::relax_f64_static_scratch_address(&scratch));
+    // the serving kernel solves on single CTAs
+    if (opt.cluster_layout != MFG_LAYOUT_SERVING &&
+        (st = plan_f64_clusters(b.get(), m, l0, conn, rowptr, inc, s)) != MFG_OK)
+      return st;
   }
   if (b->precision == MFG_PREC_MIXED) {
     b->mixed.reset(mfg::mixed_new());
@@ -872,7 +1003,6 @@ mfg_status stiffness_concurrent(mfg_batch* b, const double Fa[kStiffSlots][9], d
   MFG_CUDA(cudaEventRecord(b->ev_relax0, s));
   MFG_CUDA(cudaEventRecord(sl.fork, s));
   int launches = 0;
-  const int grid = std::min(b->R, b->sms * mfg::relax_f64_max_blocks_per_sm(0));
   for (int k = 0; k < kStiffSlots; ++k) {
     cudaStream_t sk = sl.st[k];
     MFG_CUDA(cudaStreamWaitEvent(sk, sl.fork, 0));
@@ -898,7 +1028,7 @@ mfg_status stiffness_concurrent(mfg_batch* b, const double Fa[kStiffSlots][9], d
       launches += n;
     } else {
       e = cudaMemsetAsync(bk.queue, 0, sizeof(int32_t), sk);
-      if (e == cudaSuccess) e = mfg::launch_relax_f64(bk, ak, 0, grid, sk);
+      if (e == cudaSuccess) e = launch_f64(b, bk, ak, b->f64_stiffness_clusters, sk);
       launches += 1;
     }
     if (e != cudaSuccess)

@@ -74,6 +74,30 @@ struct DevBatch {
   int32_t* queue;        // work counter for the persistent launch
 };
 
+// One CTA's part of an RVE in the FP64 cluster solve (f64_parts), and the
+// batch's parts on the device; part[rve * cl + rank].
+struct F64Part {
+  int32_t n_free, n_bnd;   // own nodes
+  int32_t fchunk, slots;   // first boundary slot, node slots (the same in every part of an RVE)
+  int32_t n_fib, n_len;    // fibers evaluated every step; with those between boundary nodes
+  int32_t n_inc, pad;
+  int64_t node_off, row_off, inc_off, fib_off;  // into the arrays below
+};
+struct F64Mass {
+  double m, rm, mc;  // mass, 1 / mass, mass times damping
+};
+struct F64Plan {
+  int cl;  // CTAs per cluster; 1: no plan, every RVE on one CTA
+  int smem_bytes;
+  const F64Part* part;
+  const int32_t* gnode;
+  const F64Mass* mass;   // by node
+  const int32_t* rows;
+  const int32_t* inc;
+  const int2* ends;
+  const double2* len;    // by fiber: l0, 1 / l0
+};
+
 struct RunArgs {
   const double* F;  // device, n_F * 9
   int32_t n_F;
@@ -137,6 +161,14 @@ cudaError_t launch_server_f64(const DevBatch& b, const ServerArgs& sa, int grid,
 cudaError_t launch_relax_f64(const DevBatch& b, const RunArgs& a, int threads, int grid,
                              cudaStream_t s);
 int relax_f64_max_blocks_per_sm(int threads);
+// The same solve with every RVE split over a cluster of plan.cl CTAs, `grid`
+// CTAs in all (mfg_relax_f64.cu, f64_parts in mfg_f64_order.h).
+constexpr int kF64ClusterSmem = 220 * 1024;
+cudaError_t launch_relax_f64_cluster(const DevBatch& b, const RunArgs& a, const F64Plan& plan,
+                                     int grid, cudaStream_t s);
+// Clusters of cl CTAs with smem_bytes of shared memory each that the device
+// holds at once (0 when it cannot run them).
+int relax_f64_max_clusters(int cl, int smem_bytes, int sms);
 
 // Fixed-scratch variant of the FP64 launch (mfg_relax_f64.cu): scratch comes
 // from a file-scope device array of MFG_NOALLOC_SCRATCH_BYTES bytes; no

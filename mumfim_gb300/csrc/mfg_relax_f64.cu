@@ -34,14 +34,23 @@
 // 84 FP64 instructions a fiber and step; the forms of mfg_exact.cuh and one
 // quotient for both kicks leave 52, the same bits. 256 RVEs of 4,500 nodes:
 // 4.3e9 -> 7.8e9 fiber-steps/s.
+//
+// A batch that leaves SMs idle runs with every RVE split over a cluster of
+// 2 to 16 CTAs instead (relax_f64_cluster_kernel below).
+#include <algorithm>
 #include <cfloat>
 #include <climits>
+#include <type_traits>
+
+#include <cooperative_groups.h>
 
 #include "mumfim_gpu.h"
 
 #include "mfg_common.cuh"
 #include "mfg_exact.cuh"
 #include "mfg_internal.h"
+
+namespace cg = cooperative_groups;
 
 namespace mfg {
 namespace {
@@ -236,7 +245,57 @@ __device__ __forceinline__ void kick(double a, double m, double rm, double mc, d
   w += q;
 }
 
-__device__ void solve_rve(const DevBatch& b, const RunArgs& a, int rve, double* red) {
+// computeCauchyStress (BatchedFiberRVEAnalysisExplicitBase.h:58-126) and the
+// status record, by one CTA. The sum over the boundary follows the
+// reference's order, one thread per Voigt component; its terms are formed by
+// the whole CTA, kTerms nodes at a time, in shared memory (6 kTerms doubles):
+// six threads that load them one by one take about 0.3 us a boundary node.
+// Reads x and f_int past the L1 cache: other CTAs of a cluster wrote them.
+constexpr int kTerms = 128;
+
+__device__ void cauchy_stress(const DevBatch& b, const RunArgs& a, const RveDesc& d, int rve,
+                              int status, int step, double residual, double* terms) {
+  const int tid = threadIdx.x;
+  const int64_t no = d.node_off, nt = b.nt;
+  const int32_t* bo = b.bnd + d.bnd_off;
+  const int nb = d.n_nodes - d.n_free;
+  double s = 0.0;
+  for (int q0 = 0; q0 < nb; q0 += kTerms) {
+    const int n = min(kTerms, nb - q0);
+    for (int t = tid; t < 6 * n; t += kThreadsF64) {
+      const int k = t / n, q = t - k * n;
+      const int64_t i = no + bo[q0 + q];
+      // component k: (i, j) index pair of the symmetric part x_i f_j
+      const int ci = k < 3 ? k : (k == 3 ? 1 : 0);
+      const int cj = k < 3 ? k : (k == 5 ? 1 : 2);
+      const double xi = __ldcg(b.x + ci * nt + i), fj = __ldcg(b.fint + cj * nt + i);
+      double v = xi * fj;
+      if (k >= 3) v = 0.5 * (v + __ldcg(b.x + cj * nt + i) * __ldcg(b.fint + ci * nt + i));
+      terms[k * kTerms + q] = v;
+    }
+    __syncthreads();
+    if (tid < 6)
+      for (int q = 0; q < n; ++q) s += terms[tid * kTerms + q];
+    __syncthreads();
+  }
+  if (tid < 6) {
+    s *= d.scale / b.vol[rve];
+    a.sigma[6 * rve + tid] = s;
+    if (a.update_coords) b.cur_stress[6 * rve + tid] = s;
+    if (!isfinite(s)) status = 4;
+  }
+  // status word: any thread of the first warp that saw a non-finite stress
+  const unsigned bad = __ballot_sync(0xffffffffu, tid < 32 && status == 4);
+  if (tid == 0) {
+    a.st_status[rve] = bad ? 4 : status;
+    a.st_steps[rve] = step;
+    a.st_residual[rve] = residual;
+  }
+  __syncthreads();
+}
+
+__device__ void solve_rve(const DevBatch& b, const RunArgs& a, int rve, double* red,
+                          double* terms) {
   const RveDesc d = b.desc[rve];
   const RveView r = make_view(b, d);
   const LawF64 L = make_law_f64(d);
@@ -279,7 +338,10 @@ __device__ void solve_rve(const DevBatch& b, const RunArgs& a, int rve, double* 
   const int cap = d.max_steps;  // host resolves the default cap for RELAX
   int step = 0;
   double residual = 10.0;
-  double h_prev = 0.0;
+  double h = d.crit * dt_crit * 0.5;  // TeamOuterLoop.h:345
+  double h2 = 2 * h, h_prev = 0.0;
+  double done = 0.0;  // (double)step, and the RAMP fraction's divisor
+  const double cap_d = static_cast<double>(cap), cap_rd = 1.0 / cap_d;
   int status = 0;
   for (;;) {
     // `step` steps are complete. Every UPDATE_FREQ steps the residual of the
@@ -302,8 +364,6 @@ __device__ void solve_rve(const DevBatch& b, const RunArgs& a, int rve, double* 
     }
     if (!ramp && res_step && !(residual > d.tol)) break;
     if (step >= cap) break;  // RAMP: exactly max_steps steps; RELAX: cap reached
-    const double h = d.crit * dt_crit * 0.5;  // TeamOuterLoop.h:345
-    const double h2 = 2 * h;
     const bool same = h == h_prev;
     // node pass: trailing kick of step-1, leading kick + drift of step
     for (int i = tid; i < NF; i += kThreadsF64) {
@@ -320,7 +380,7 @@ __device__ void solve_rve(const DevBatch& b, const RunArgs& a, int rve, double* 
       r.x2[i] = r.x2[i] + h2 * w2;
     }
     if (ramp) {
-      const double alpha = static_cast<double>(step + 1) / static_cast<double>(d.max_steps);
+      const double alpha = div_known(done + 1.0, cap_d, cap_rd);
       for (int i = NF + tid; i < N; i += kThreadsF64) {
         const double* rb = r.ramp + 6 * (i - NF);
         r.x0[i] = rb[0] + alpha * rb[3];
@@ -329,13 +389,16 @@ __device__ void solve_rve(const DevBatch& b, const RunArgs& a, int rve, double* 
       }
     }
     __syncthreads();
+    h_prev = h;
     if (step % kUpdateFreq == 0) {
       dt_crit = block_min<kThreadsF64>(fiber_pass<true>(r, d, L), red) / d.sound_speed;
+      h = d.crit * dt_crit * 0.5;
+      h2 = 2 * h;
     } else {
       fiber_pass<false>(r, d, L);
       __syncthreads();
     }
-    h_prev = h;
+    done += 1.0;
     ++step;
   }
   if (status == 0 && !ramp && residual > d.tol) status = 3;  // MFG_E_NOT_CONVERGED
@@ -354,43 +417,12 @@ __device__ void solve_rve(const DevBatch& b, const RunArgs& a, int rve, double* 
     }
   }
   __syncthreads();
-  // ---- computeCauchyStress: one thread per Voigt component, serial order --
-  if (tid < 6) {
-    double s = 0.0;
-    const int k = tid;
-    const int32_t* bo = b.bnd + d.bnd_off;
-    for (int q = 0; q < N - NF; ++q) {
-      const int i = bo[q];
-      const double f1 = r.fi0[i], f2 = r.fi1[i], f3 = r.fi2[i];
-      const double crd1 = r.x0[i], crd2 = r.x1[i], crd3 = r.x2[i];
-      double t;
-      switch (k) {
-        case 0: t = crd1 * f1; break;
-        case 1: t = crd2 * f2; break;
-        case 2: t = crd3 * f3; break;
-        case 3: t = 0.5 * (crd2 * f3 + crd3 * f2); break;
-        case 4: t = 0.5 * (crd1 * f3 + crd3 * f1); break;
-        default: t = 0.5 * (crd1 * f2 + crd2 * f1); break;
-      }
-      s += t;
-    }
-    s *= d.scale / b.vol[rve];
-    a.sigma[6 * rve + k] = s;
-    if (a.update_coords) b.cur_stress[6 * rve + k] = s;
-    if (!isfinite(s)) status = 4;
-  }
-  // status word: any thread of the first warp that saw a non-finite stress
-  const unsigned bad = __ballot_sync(0xffffffffu, tid < 32 && status == 4);
-  if (tid == 0) {
-    a.st_status[rve] = bad ? 4 : status;
-    a.st_steps[rve] = step;
-    a.st_residual[rve] = residual;
-  }
-  __syncthreads();
+  cauchy_stress(b, a, d, rve, status, step, residual, terms);
 }
 
 __global__ void __launch_bounds__(kThreadsF64) relax_f64_kernel(const DevBatch b, const RunArgs a) {
   __shared__ double red[kThreadsF64 / 32 + 1];
+  __shared__ double terms[6 * kTerms];
   __shared__ int s_rve;
   for (;;) {
     if (threadIdx.x == 0) {
@@ -401,17 +433,404 @@ __global__ void __launch_bounds__(kThreadsF64) relax_f64_kernel(const DevBatch b
     const int rve = s_rve;
     __syncthreads();
     if (rve < 0) break;
-    solve_rve(b, a, rve, red);
+    solve_rve(b, a, rve, red, terms);
   }
 }
 
 __global__ void __launch_bounds__(kThreadsF64) server_f64_kernel(const DevBatch b,
                                                                  const ServerArgs sa) {
   __shared__ double red[kThreadsF64 / 32 + 1];
-  server_loop(sa, [&](const RunArgs& a, int rve) { solve_rve(b, a, rve, red); });
+  __shared__ double terms[6 * kTerms];
+  server_loop(sa, [&](const RunArgs& a, int rve) { solve_rve(b, a, rve, red, terms); });
+}
+
+
+// ---- one RVE over a cluster of CTAs ------------------------------------------
+//
+// For batches that leave SMs idle. One CTA solves an RVE at the FP64 rate of
+// one SM: 42 us a step at 1,000 nodes with 151 SMs doing nothing. Here CL CTAs
+// on CL SMs share it (f64_parts): each keeps two copies of its nodes'
+// positions, their velocities and the force vectors of the fibers it
+// evaluates in shared memory and reads other CTAs' positions through
+// distributed shared memory. A fiber between two CTAs is evaluated by both,
+// so force vectors stay local and a step has one cluster barrier (positions
+// moved) and one block barrier (forces formed); the two position copies swap
+// roles every step, so that no CTA writes what a slower one still reads.
+// Every number is formed by the expressions and in the order of the single
+// CTA: the same bits.
+//
+// The read-only data of the step (fiber ends and lengths, masses, rows) is
+// copied into shared memory as far as it fits: the barrier's acquire drops
+// the L1 cache, and a step of a small part is a chain of loads.
+
+template <int CL>
+struct ClusterX {
+  uint32_t base;     // shared address of the copy being read, in this CTA
+  uint32_t stride;   // bytes from one component to the next
+  __device__ __forceinline__ void load(int code, double x[3]) const {
+    uint32_t p;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;"
+                 : "=r"(p)
+                 : "r"(base + 8u * (static_cast<uint32_t>(code) & 0xFFFFFFu)),
+                   "r"(static_cast<uint32_t>(code) >> 24));
+    asm volatile("ld.shared::cluster.f64 %0, [%1];" : "=d"(x[0]) : "r"(p));
+    asm volatile("ld.shared::cluster.f64 %0, [%1];" : "=d"(x[1]) : "r"(p + stride));
+    asm volatile("ld.shared::cluster.f64 %0, [%1];" : "=d"(x[2]) : "r"(p + 2 * stride));
+  }
+};
+
+// Minimum over the cluster of a block-reduced value.
+template <int CL>
+__device__ double cluster_min(double part, double* slot) {
+  cg::cluster_group cl = cg::this_cluster();
+  if (threadIdx.x == 0) *slot = part;
+  cl.sync();
+  double t = DBL_MAX;
+#pragma unroll
+  for (int o = 0; o < CL; ++o) t = fmin(t, *cl.map_shared_rank(slot, o));
+  cl.sync();
+  return t;
+}
+
+// Copies n items to the shared memory at `at` when they fit below `end`, and
+// returns where to read them.
+template <typename T>
+__device__ __forceinline__ const T* stage(const T* src, int n, unsigned char*& at,
+                                          const unsigned char* end) {
+  const size_t bytes = (static_cast<size_t>(n) * sizeof(T) + 15) & ~static_cast<size_t>(15);
+  if (at + bytes > end) return src;
+  T* dst = reinterpret_cast<T*>(at);
+  for (int k = threadIdx.x; k < n; k += kThreadsF64) dst[k] = src[k];
+  at += bytes;
+  return dst;
+}
+
+template <int CL>
+__device__ void solve_rve_cluster(const DevBatch& b, const RunArgs& a, const F64Plan& plan,
+                                  int rve, double* red, double* cred, double* alpha_s,
+                                  double* terms,
+                                  unsigned char* smem, int smem_bytes) {
+  cg::cluster_group cluster = cg::this_cluster();
+  const int rank = static_cast<int>(cluster.block_rank());
+  const int tid = threadIdx.x;
+  const RveDesc d = b.desc[rve];
+  const F64Part part = plan.part[static_cast<int64_t>(rve) * CL + rank];
+  const LawF64 L = make_law_f64(d);
+  const int64_t no = d.node_off, nt = b.nt;
+  const int NF = d.n_free, nfo = part.n_free, nbo = part.n_bnd, S = part.slots;
+  const int n_own = nfo + nbo;
+  const bool ramp = d.mode == 1;
+  // shared memory: two copies of the positions, force vectors, velocities,
+  // then the read-only data
+  const unsigned char* end = smem + smem_bytes;
+  double* xs = reinterpret_cast<double*>(smem);
+  double* nrm = xs + 6 * S;
+  unsigned char* at = reinterpret_cast<unsigned char*>(nrm + 3 * part.n_fib);
+  at = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(at) + 15) & ~uintptr_t(15));
+  double* vel = b.v + 3 * (no + rank * part.fchunk);  // 3 per own free node
+  if (at + 24 * nfo + 16 <= end) {
+    vel = reinterpret_cast<double*>(at);
+    at += (24 * nfo + 15) & ~15;
+  }
+  double* rbs = b.ramp + 6 * (d.bnd_off + rank * (part.slots - part.fchunk));
+  if (ramp && at + 48 * nbo <= end) {
+    rbs = reinterpret_cast<double*>(at);
+    at += 48 * nbo;
+  }
+  const int2* ends = stage(plan.ends + part.fib_off, part.n_len, at, end);
+  const double2* len = stage(plan.len + part.fib_off, part.n_len, at, end);
+  const int32_t* rows = stage(plan.rows + part.row_off, nfo + 1, at, end);
+  const int32_t* inc = stage(plan.inc + part.inc_off, part.n_inc, at, end);
+  const F64Mass* mass = stage(plan.mass + part.node_off, nfo, at, end);
+  const int32_t* gnode = plan.gnode + part.node_off;
+
+  const double* F = a.F + 9 * (a.n_F > 1 ? rve : 0);
+  double Fm[9];
+#pragma unroll
+  for (int k = 0; k < 9; ++k) Fm[k] = F[k];
+  if (a.update_coords && rank == 0 && tid == 0) b.vol[rve] = jacobian(Fm) * b.vol[rve];
+
+  // ---- prologue, as solve_rve -------------------------------------------------
+  for (int t = tid; t < n_own; t += kThreadsF64) {
+    const int64_t gi = no + gnode[t];
+    const int li = t < nfo ? t : part.fchunk + (t - nfo);
+    const double xo0 = b.x[gi], xo1 = b.x[nt + gi], xo2 = b.x[2 * nt + gi];
+    double up0 = b.u[gi], up1 = b.u[nt + gi], up2 = b.u[2 * nt + gi];
+    if (!ramp) {
+      up0 = (Fm[0] - 1) * xo0 + (Fm[1] - 0) * xo1 + (Fm[2] - 0) * xo2 + up0;
+      up1 = (Fm[3] - 0) * xo0 + (Fm[4] - 1) * xo1 + (Fm[5] - 0) * xo2 + up1;
+      up2 = (Fm[6] - 0) * xo0 + (Fm[7] - 0) * xo1 + (Fm[8] - 1) * xo2 + up2;
+    }
+    const double xn0 = b.X[gi] + up0, xn1 = b.X[nt + gi] + up1, xn2 = b.X[2 * nt + gi] + up2;
+    xs[li] = xn0; xs[S + li] = xn1; xs[2 * S + li] = xn2;
+    if (t < nfo) {
+      vel[t] = 0.0; vel[nfo + t] = 0.0; vel[2 * nfo + t] = 0.0;
+    } else {
+      // the boundary does not move in RELAX mode: both copies hold it
+      xs[3 * S + li] = xn0; xs[4 * S + li] = xn1; xs[5 * S + li] = xn2;
+      if (ramp) {
+        double* rb = rbs + 6 * (t - nfo);
+        rb[0] = xn0; rb[1] = xn1; rb[2] = xn2;
+        rb[3] = (Fm[0] - 1) * xn0 + (Fm[1] - 0) * xn1 + (Fm[2] - 0) * xn2;
+        rb[4] = (Fm[3] - 0) * xn0 + (Fm[4] - 1) * xn1 + (Fm[5] - 0) * xn2;
+        rb[5] = (Fm[6] - 0) * xn0 + (Fm[7] - 0) * xn1 + (Fm[8] - 1) * xn2;
+      }
+    }
+  }
+  const uint32_t xs_addr = static_cast<uint32_t>(__cvta_generic_to_shared(xs));
+  int cur = 0;  // the copy that holds the current positions
+  ClusterX<CL> x{xs_addr, 8u * static_cast<uint32_t>(S)};
+
+  // fiber pass over the part's fibers; with kLen also the shortest length,
+  // for which the fibers between boundary nodes count too
+  auto fiber_pass = [&](auto want_len) {
+    constexpr bool kLen = decltype(want_len)::value;
+    double lmin = DBL_MAX;
+    const int n = kLen ? part.n_len : part.n_fib;
+    for (int e = tid; e < n; e += kThreadsF64) {
+      const int2 c = ends[e];
+      const double2 q = len[e];
+      double xa[3], xb[3], nv[3];
+      x.load(c.x, xa);
+      x.load(c.y, xb);
+      const double dv[3] = {xb[0] - xa[0], xb[1] - xa[1], xb[2] - xa[2]};
+      const double l = fiber_vector(L, dv, q.x, q.y, nv);
+      if (kLen) {
+        lmin = fmin(lmin, l);
+        if (e >= part.n_fib) continue;
+      }
+      nrm[e] = nv[0];
+      nrm[part.n_fib + e] = nv[1];
+      nrm[2 * part.n_fib + e] = nv[2];
+    }
+    return lmin;
+  };
+  // component k of f_int of the own free node t: its fibers in ascending
+  // original id
+  auto gather = [&](int t, int k) {
+    const int pb = rows[t], pe = rows[t + 1];
+    const double* nk = nrm + k * part.n_fib;
+    double f = 0.0;
+    for (int p = pb; p < pe; ++p) {
+      const int code = inc[p];
+      const double v = flip_sign(nk[code >> 1], !(code & 1));
+      f = p == pb ? v : f + v;
+    }
+    return f;
+  };
+  cluster.sync();
+  double dt_crit = cluster_min<CL>(
+                       block_min<kThreadsF64>(fiber_pass(std::true_type{}), red), cred) /
+                   d.sound_speed;
+
+  // ---- main loop, as solve_rve --------------------------------------------------
+  // Node pass: one thread per node and component, each component padded to
+  // whole warps, then the boundary's. A warp's FP64 instruction occupies its
+  // SM sub-partition's unit for 64 cycles, whatever it depends on, so a part
+  // of 60 nodes (2 warps of whole nodes) would leave half of the SM idle.
+  const int W = (nfo + 31) & ~31;
+  const int cap = d.max_steps;
+  int step = 0;
+  double residual = 10.0;
+  double h = d.crit * dt_crit * 0.5;  // TeamOuterLoop.h:345
+  double h2 = 2 * h, h_prev = 0.0;
+  int status = 0;
+  // RAMP fraction of the next step, kept by the last warp
+  const double cap_d = static_cast<double>(cap), cap_rd = 1.0 / cap_d;
+  double done = 1.0;
+  if (tid == kThreadsF64 - 1) *alpha_s = div_known(done, cap_d, cap_rd);
+  __syncthreads();
+  for (;;) {
+    const bool res_step = step > 0 && ((step - 1) % kUpdateFreq) == 0;
+    if (res_step) {
+      // the nodes' shares go through global memory (f_int's first component,
+      // unused at free nodes) and every CTA sums all of them in the order of
+      // solve_rve
+      for (int t = tid; t < nfo; t += kThreadsF64) {
+        const double f0 = gather(t, 0), f1 = gather(t, 1), f2 = gather(t, 2);
+        b.fint[no + gnode[t]] = f0 * f0 + f1 * f1 + f2 * f2;
+      }
+      cluster.sync();
+      double sum = 0.0;
+      for (int i = tid; i < NF; i += kThreadsF64) sum += __ldcg(b.fint + no + i);
+      residual = sqrt(block_sum<kThreadsF64>(sum, red));
+      if (!isfinite(residual)) {
+        status = 4;  // MFG_E_NONFINITE
+        break;
+      }
+    }
+    if (!ramp && res_step && !(residual > d.tol)) break;
+    if (step >= cap) break;
+    const bool same = h == h_prev;
+    const double* xc = xs + 3 * S * cur;
+    double* xn = xs + 3 * S * (1 - cur);
+    const int n_items = 3 * W + (ramp ? 3 * nbo : 0);
+    for (int item = tid; item < n_items; item += kThreadsF64) {
+      if (item < 3 * W) {
+        const int k = item < W ? 0 : (item < 2 * W ? 1 : 2);
+        const int t = item - k * W;
+        if (t < nfo) {
+          const F64Mass mm = mass[t];
+          double w = vel[k * nfo + t];
+          kick(gather(t, k), mm.m, mm.rm, mm.mc, h_prev, h, step == 0, same, w);
+          vel[k * nfo + t] = w;
+          xn[k * S + t] = xc[k * S + t] + h2 * w;
+        }
+      } else {
+        const int q = item - 3 * W;
+        const int k = q < nbo ? 0 : (q < 2 * nbo ? 1 : 2);
+        const double* rb = rbs + 6 * (q - k * nbo) + k;
+        xn[k * S + part.fchunk + (q - k * nbo)] = rb[0] + *alpha_s * rb[3];
+      }
+    }
+    cur = 1 - cur;
+    x.base = xs_addr + 24u * static_cast<uint32_t>(S) * static_cast<uint32_t>(cur);
+    cluster.sync();
+    if (ramp && tid == kThreadsF64 - 1) {
+      done += 1.0;
+      *alpha_s = div_known(done, cap_d, cap_rd);
+    }
+    h_prev = h;
+    if (step % kUpdateFreq == 0) {
+      dt_crit = cluster_min<CL>(block_min<kThreadsF64>(fiber_pass(std::true_type{}), red), cred) /
+                d.sound_speed;
+      h = d.crit * dt_crit * 0.5;
+      h2 = 2 * h;
+    } else {
+      fiber_pass(std::false_type{});
+      __syncthreads();
+    }
+    ++step;
+  }
+  if (status == 0 && !ramp && residual > d.tol) status = 3;  // MFG_E_NOT_CONVERGED
+
+  // ---- FinalizeData: positions, u = x - X, boundary f_int, stress ------------------
+  const double* xc = xs + 3 * S * cur;
+  for (int t = tid; t < n_own; t += kThreadsF64) {
+    const int64_t gi = no + gnode[t];
+    const int li = t < nfo ? t : part.fchunk + (t - nfo);
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+      const double xk = xc[k * S + li];
+      b.x[k * nt + gi] = xk;
+      if (a.update_coords) b.u[k * nt + gi] = xk - b.X[k * nt + gi];
+    }
+  }
+  cluster.sync();
+  // boundary rows from the positions just written (past the L1 cache): the
+  // vectors of their fibers may be another CTA's
+  for (int q = tid; q < nbo; q += kThreadsF64) {
+    const int i = gnode[nfo + q];
+    const int32_t* row = b.rowptr + d.row_off + i;
+    double f[3] = {0.0, 0.0, 0.0};
+    for (int p = row[0]; p < row[1]; ++p) {
+      const int code = b.inc[d.inc_off + p];
+      const int64_t e = d.fiber_off + (code >> 1);
+      const int2 c = b.conn[e];
+      double dv[3], nv[3];
+#pragma unroll
+      for (int k = 0; k < 3; ++k)
+        dv[k] = __ldcg(b.x + k * nt + no + c.y) - __ldcg(b.x + k * nt + no + c.x);
+      fiber_vector(L, dv, b.l0[e], b.rl0[e], nv);
+#pragma unroll
+      for (int k = 0; k < 3; ++k) f[k] = f[k] + flip_sign(nv[k], !(code & 1));
+    }
+#pragma unroll
+    for (int k = 0; k < 3; ++k) b.fint[k * nt + no + i] = f[k];
+  }
+  cluster.sync();
+  if (rank == 0) cauchy_stress(b, a, d, rve, status, step, residual, terms);
+}
+
+template <int CL>
+__global__ void __launch_bounds__(kThreadsF64, 1)
+relax_f64_cluster_kernel(const DevBatch b, const RunArgs a, const F64Plan plan) {
+  extern __shared__ double4 smem_f64[];
+  __shared__ double red[kThreadsF64 / 32 + 1];
+  __shared__ double terms[6 * kTerms];
+  __shared__ double cred, alpha;
+  __shared__ int s_rve;
+  cg::cluster_group cluster = cg::this_cluster();
+  for (;;) {
+    if (cluster.block_rank() == 0 && threadIdx.x == 0) {
+      const int w = atomicAdd(b.queue, 1);
+      s_rve = w < b.n_rve ? b.order[w] : -1;
+    }
+    cluster.sync();
+    const int rve = *cluster.map_shared_rank(&s_rve, 0);
+    cluster.sync();  // also: no CTA overwrites what a slower one still reads
+    if (rve < 0) break;
+    solve_rve_cluster<CL>(b, a, plan, rve, red, &cred, &alpha, terms,
+                          reinterpret_cast<unsigned char*>(smem_f64), plan.smem_bytes);
+  }
+}
+
+// Calls fn(std::integral_constant<int, CL>{}) for a cluster size of 2 to 16.
+template <class Fn>
+cudaError_t with_cluster(int cl, Fn&& fn) {
+  switch (cl) {
+    case 2: return fn(std::integral_constant<int, 2>{});
+    case 4: return fn(std::integral_constant<int, 4>{});
+    case 8: return fn(std::integral_constant<int, 8>{});
+    case 16: return fn(std::integral_constant<int, 16>{});
+    default: return cudaErrorInvalidValue;
+  }
+}
+
+template <int CL>
+cudaError_t cluster_config(int grid, int smem_bytes, cudaStream_t s, cudaLaunchConfig_t* cfg,
+                           cudaLaunchAttribute* attr) {
+  cudaError_t e = cudaFuncSetAttribute(relax_f64_cluster_kernel<CL>,
+                                       cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                       kF64ClusterSmem);
+  if (e == cudaSuccess && CL > 8)
+    e = cudaFuncSetAttribute(relax_f64_cluster_kernel<CL>,
+                             cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+  *cfg = {};
+  cfg->gridDim = dim3(static_cast<unsigned>(grid), 1, 1);
+  cfg->blockDim = dim3(kThreadsF64, 1, 1);
+  cfg->dynamicSmemBytes = static_cast<size_t>(smem_bytes);
+  cfg->stream = s;
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = CL;
+  attr[0].val.clusterDim.y = 1;
+  attr[0].val.clusterDim.z = 1;
+  cfg->attrs = attr;
+  cfg->numAttrs = 1;
+  return e;
 }
 
 }  // namespace
+
+int relax_f64_max_clusters(int cl, int smem_bytes, int sms) {
+  int n = 0;
+  const cudaError_t e = with_cluster(cl, [&](auto C) {
+    constexpr int CL = decltype(C)::value;
+    cudaLaunchAttribute attr[1];
+    cudaLaunchConfig_t cfg;
+    cudaError_t r = cluster_config<CL>(CL * sms, smem_bytes, nullptr, &cfg, attr);
+    if (r == cudaSuccess)
+      r = cudaOccupancyMaxActiveClusters(&n, relax_f64_cluster_kernel<CL>, &cfg);
+    return r;
+  });
+  if (e != cudaSuccess) {
+    cudaGetLastError();  // an unsupported size is no failure of the caller's
+    return 0;
+  }
+  return n;
+}
+
+cudaError_t launch_relax_f64_cluster(const DevBatch& b, const RunArgs& a, const F64Plan& plan,
+                                     int grid, cudaStream_t s) {
+  return with_cluster(plan.cl, [&](auto C) {
+    constexpr int CL = decltype(C)::value;
+    cudaLaunchAttribute attr[1];
+    cudaLaunchConfig_t cfg;
+    cudaError_t e = cluster_config<CL>(grid, plan.smem_bytes, s, &cfg, attr);
+    if (e != cudaSuccess) return e;
+    return cudaLaunchKernelEx(&cfg, relax_f64_cluster_kernel<CL>, b, a, plan);
+  });
+}
 
 cudaError_t launch_server_f64(const DevBatch& b, const ServerArgs& sa, int grid, cudaStream_t s) {
   server_f64_kernel<<<grid, kThreadsF64, 0, s>>>(b, sa);
