@@ -342,6 +342,9 @@ struct mfg_batch {
   bool f64_stiffness_clusters = false;
   DevArray<unsigned char> d_plan;
   std::unique_ptr<mfg::MixedState, mfg::MixedStateDeleter> mixed;
+  // the concurrent stiffness solves' own working set, when six solves at
+  // once fill the GPU where one leaves SMs idle and so takes wider clusters
+  std::unique_ptr<mfg::MixedState, mfg::MixedStateDeleter> mixed_stiff;
   int stiffness = MFG_STIFFNESS_AUTO;
   bool all_ramp = false;
   StiffSlots stiff;
@@ -350,6 +353,7 @@ struct mfg_batch {
     if (device >= 0) cudaSetDevice(device);
     stiff.release();
     mixed.reset();
+    mixed_stiff.reset();
     for (auto* a : {&d_X, &d_x, &d_u, &d_v, &d_m, &d_l0, &d_nrm, &d_fint, &d_ramp, &d_vol, &d_cur,
                     &d_F, &d_sigma, &d_res, &d_omega})
       a->release();
@@ -818,14 +822,21 @@ static mfg_status batch_create_impl(const mfg_network* nets, const mfg_strategy*
       return st;
   }
   if (b->precision == MFG_PREC_MIXED) {
-    b->mixed.reset(mfg::mixed_new());
-    cudaError_t e =
-        b->mixed ? mfg::mixed_create(*b->mixed, dv, b->desc, conn, rowptr, inc, b->sms,
-                                     opt.max_cluster_ctas > 0 ? opt.max_cluster_ctas : 8,
-                                     opt.cluster_layout == MFG_LAYOUT_SERVING,
-                                     opt.small_rve_solve,
-                                     opt.small_rves_per_cta > 0 ? opt.small_rves_per_cta : 2, s)
-                 : cudaErrorMemoryAllocation;
+    auto make = [&](std::unique_ptr<mfg::MixedState, mfg::MixedStateDeleter>& state, int copies) {
+      state.reset(mfg::mixed_new());
+      return state ? mfg::mixed_create(*state, dv, b->desc, conn, rowptr, inc, b->sms,
+                                       opt.max_cluster_ctas > 0 ? opt.max_cluster_ctas : 16,
+                                       opt.cluster_layout == MFG_LAYOUT_SERVING,
+                                       opt.small_rve_solve,
+                                       opt.small_rves_per_cta > 0 ? opt.small_rves_per_cta : 2,
+                                       copies, s)
+                   : cudaErrorMemoryAllocation;
+    };
+    cudaError_t e = make(b->mixed, 1);
+    if (e == cudaSuccess && mfg::mixed_widened(*b->mixed) &&
+        opt.stiffness != MFG_STIFFNESS_SEQUENTIAL &&
+        (b->all_ramp || opt.stiffness == MFG_STIFFNESS_CONCURRENT))
+      e = make(b->mixed_stiff, kStiffSlots);
     if (e != cudaSuccess)
       return fail(e == cudaErrorMemoryAllocation ? MFG_E_OOM : MFG_E_CUDA,
                   "mixed-precision set-up failed: %s", cudaGetErrorString(e));
@@ -973,7 +984,8 @@ mfg_status stiff_slots_ready(mfg_batch* b) {
   }
   if (e == cudaSuccess) e = cudaEventCreateWithFlags(&sl.fork, cudaEventDisableTiming);
   if (e == cudaSuccess && b->precision == MFG_PREC_MIXED)
-    e = mfg::mixed_prepare_contexts(*b->mixed, b->dev, kStiffSlots);
+    e = mfg::mixed_prepare_contexts(b->mixed_stiff ? *b->mixed_stiff : *b->mixed, b->dev,
+                                    kStiffSlots);
   if (e != cudaSuccess) {
     sl.release();
     return fail(e == cudaErrorMemoryAllocation ? MFG_E_OOM : MFG_E_CUDA,
@@ -1024,7 +1036,7 @@ mfg_status stiffness_concurrent(mfg_batch* b, const double Fa[kStiffSlots][9], d
     cudaError_t e;
     if (b->precision == MFG_PREC_MIXED) {
       int n = 0;
-      e = mfg::run_mixed(*b->mixed, bk, ak, sk, &n, k + 1);
+      e = mfg::run_mixed(b->mixed_stiff ? *b->mixed_stiff : *b->mixed, bk, ak, sk, &n, k + 1);
       launches += n;
     } else {
       e = cudaMemsetAsync(bk.queue, 0, sizeof(int32_t), sk);

@@ -26,12 +26,14 @@ constexpr int kMixedContexts = 7;
 // the cluster size; serving_layout takes clusters of 4 where the batch
 // layout would take 2. small_solve (mfg_small_rve_solve) picks the solve of
 // the RVEs whose node state fits one CTA; with the fiber-centric one, up to
-// rves_per_cta (1 or 2) small RVEs share a CTA.
+// rves_per_cta (1 or 2) small RVEs share a CTA. A batch that leaves SMs idle
+// with `copies` solves of it at once takes wider clusters (up to max_cluster,
+// 16 at most), with the same results.
 cudaError_t mixed_create(MixedState& ms, const DevBatch& b, const std::vector<RveDesc>& desc,
                          const std::vector<int2>& conn, const std::vector<int32_t>& rowptr,
                          const std::vector<int32_t>& inc, int sms, int max_cluster,
                          bool serving_layout, int small_solve, int rves_per_cta,
-                         cudaStream_t s);
+                         int copies, cudaStream_t s);
 // One run: reads the persistent FP64 state (x, u, vol), relaxes in mixed
 // precision and writes the FP64 state, stress and status back. `ctx` picks
 // the run context (0 for the batch's runs); runs on different contexts may
@@ -47,6 +49,8 @@ void mixed_destroy(MixedState* ms);
 // `small` ring CTA by CTA.
 cudaError_t launch_server_mixed(MixedState& ms, const DevBatch& b, const ServerArgs& small,
                                 const ServerArgs* big, cudaStream_t s);
+// Whether some bucket of the batch took wider clusters than its RVEs need.
+bool mixed_widened(const MixedState& ms);
 // Cluster size of an RVE's batch bucket, and whether the serving kernel
 // solves it as a cluster.
 int mixed_rve_cluster(const MixedState& ms, int rve);

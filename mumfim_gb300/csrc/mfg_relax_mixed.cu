@@ -66,6 +66,7 @@ namespace mfg {
 // the batch's runs; contexts 1-6 the concurrent perturbed solves of the
 // material stiffness, which run at the same time on the same batch.
 constexpr int kMixedBuckets = 10;
+constexpr int kMaxCluster = 16;
 struct MixedRunCtx {
   int32_t* queues = nullptr;  // one claim counter per bucket (device)
   float* u_hl = nullptr;      // run-time placement scratch; null: the batch's own
@@ -108,21 +109,27 @@ struct MixedState {
   // incidence the other end's code and the fiber's data (solve_rve_nodal).
   int2* nsell = nullptr;         // nt
   int64_t* sell_off = nullptr;   // n_rve
+  int2* sell_cta = nullptr;      // n_rve * kMaxCluster, (first, count) of the incidence records of
+                                 // each CTA's free nodes
   int32_t* ncode = nullptr;      // set-up only: SELL element codes, packed into nfc
   float4* nfc = nullptr;         // SELL elements
   int64_t n_sell = 0;
+  void* arrays = nullptr;  // the allocation that holds every array but nfc
+  void* set_up = nullptr;  // set-up only: the one that holds ncode and nfib_tmp
   int64_t* nfib_tmp = nullptr;   // set-up only: fiber of each SELL element
   int32_t* h_cl = nullptr;     // host, per RVE: cluster size of its batch bucket
   int32_t* rve_bucket = nullptr;  // device, per RVE: its batch bucket (serving kernels)
   int server_grid = 0;         // CTAs of the cluster serving kernel
   int sms = 1;
   int smem_bytes = 0;
-  // Size buckets of the batch run (kBucket[q]: cluster size and solve); the
-  // RVEs of bucket q, most fibers first, are order[bucket_off[q] ..
-  // bucket_off[q + 1]).
+  // Size buckets of the batch run; the RVEs of bucket q, most fibers first,
+  // are order[bucket_off[q] .. bucket_off[q + 1]), solved by the launch
+  // kind kKind[bucket_kind[q]] (cluster size and solve).
   int32_t* order = nullptr;
   int bucket_off[kMixedBuckets + 1] = {};
+  int bucket_kind[kMixedBuckets] = {};
   int bucket_grid[kMixedBuckets] = {};
+  int launch_order[kMixedBuckets] = {};  // buckets, largest clusters first
   // Run contexts (host memory; kernels never touch this pointer). A run is a
   // CUDA graph (queue reset, fork, one launch per bucket, join), captured
   // per context for the last run arguments and replayed while they stay
@@ -134,28 +141,41 @@ namespace {
 
 constexpr int kThreadsMixed = 1024;
 constexpr int kSmemBytesMixed = 220 * 1024;
-// Size buckets, launched in this order (largest clusters first).
+// How the RVEs of a size bucket are solved.
 struct BucketKind {
   int cl;      // CTAs per cluster
   bool all;    // fiber-centric: force vectors in shared memory too
   bool nodal;  // node-centric solve (node state in shared memory)
   int ng;      // RVEs solved side by side by one CTA (fiber-centric, all on chip)
-  bool db;     // node-centric on one CTA with two copies of the node records
+  bool db;     // node-centric with two copies of the node records
+  bool stage;  // and the read-only data of the step in shared memory too (on one CTA with
+               // two copies: for the RVEs for which it fits)
 };
 constexpr int kBuckets = kMixedBuckets;
-constexpr BucketKind kBucket[kBuckets] = {
-    {8, false, true, 1, false}, {4, false, true, 1, true},   {4, false, true, 1, false},
-    {2, false, true, 1, true},  {2, false, true, 1, false},  {1, false, true, 1, false},
-    {1, false, true, 1, true},  {1, true, false, 1, false},  {1, true, false, 2, false},
-    {1, false, false, 1, false}};
+// Launch kinds: each bucket's own (the same index), then the wider clusters a
+// bucket may take when the batch leaves SMs idle (choose_kinds).
+constexpr int kKinds = 17;
+constexpr BucketKind kKind[kKinds] = {
+    {8, false, true, 1, false, false}, {4, false, true, 1, true, false},
+    {4, false, true, 1, false, false}, {2, false, true, 1, true, false},
+    {2, false, true, 1, false, false}, {1, false, true, 1, false, false},
+    {1, false, true, 1, true, false},  {1, true, false, 1, false, false},
+    {1, true, false, 2, false, false}, {1, false, false, 1, false, false},
+    // wider
+    {8, false, true, 1, true, false},  {16, false, true, 1, true, false},
+    {16, false, true, 1, false, false}, {2, false, true, 1, true, true},
+    {4, false, true, 1, true, true},   {8, false, true, 1, true, true},
+    {16, false, true, 1, true, true}};
+constexpr const BucketKind* kBucket = kKind;
 // Placement preference (bucket_of): the first bucket whose shared memory
-// holds the RVE, else the last bucket. At each cluster size two copies of
-// the node records come first where they fit.
+// holds the RVE, else the run-time placement. At each cluster size two
+// copies of the node records come first where they fit.
 constexpr int kPref[] = {8, 7, 6, 5, 3, 4, 1, 2, 0};
 // The single-CTA buckets with an RVE order of their own, by kind.
-constexpr int kQNodal1 = 5, kQNodalDB = 6, kQFiberAll = 7, kQFiberPair = 8;
+constexpr int kQNodal1 = 5, kQNodalDB = 6, kQFiberAll = 7, kQFiberPair = 8, kQRuntime = 9;
 static_assert(kBucket[kQNodal1].cl == 1 && kBucket[kQNodal1].nodal, "bucket table");
 static_assert(kBucket[kQNodalDB].cl == 1 && kBucket[kQNodalDB].db, "bucket table");
+static_assert(!kBucket[kQRuntime].all && !kBucket[kQRuntime].nodal, "bucket table");
 static_assert(kBucket[kQFiberAll].cl == 1 && kBucket[kQFiberAll].all, "bucket table");
 static_assert(kBucket[kQFiberPair].all && kBucket[kQFiberPair].ng == 2, "bucket table");
 
@@ -408,7 +428,7 @@ struct ClusterOps {
       if (threadIdx.x == 0) *slot = part;
       cl.sync();
       double t = kMin ? DBL_MAX : 0.0;
-#pragma unroll
+#pragma unroll 1
       for (int o = 0; o < CL; ++o) {
         const double v = *cl.map_shared_rank(slot, o);
         t = kMin ? fmin(t, v) : t + v;
@@ -689,6 +709,17 @@ __host__ __device__ inline int64_t cluster_floats(int n_nodes, int n_free, int n
   const int64_t cap = even_slots((static_cast<int64_t>(n_free) + cl - 1) / cl + (nb + cl - 1) / cl);
   const int64_t echunk = (static_cast<int64_t>(n_fibers) + cl - 1) / cl;
   return (two_copies ? 15 : 9) * cap + (all ? 4 * echunk : 0);
+}
+
+// First float of the staged read-only data behind two record copies and the
+// velocities (16-byte aligned), and whether it fits: 16 bytes per incidence
+// record, 16 per node (row and mass).
+__host__ __device__ inline int64_t stage_offset(int64_t slots) {
+  return (15 * slots + 3) & ~static_cast<int64_t>(3);
+}
+__host__ __device__ inline bool stage_fits(int64_t slots, int64_t n_free, int64_t n_rec,
+                                           int64_t smem_floats) {
+  return stage_offset(slots) + 4 * n_rec + 4 * n_free <= smem_floats;
 }
 
 // Prologue of a solve in FP64 for the CTA's own nodes: the affine predictor
@@ -985,22 +1016,31 @@ __device__ void solve_rve_mixed(const DevBatch& b, const MixedState& ms, const R
 // it is the same rounding as subtracting the second-end vector, so the sums
 // are the bits the fiber-centric solve gathers.
 
+// Read-only data of the step: in global memory (read through the L1 cache),
+// or staged in the CTA's shared memory.
+template <bool kStage, typename T>
+__device__ __forceinline__ T read_only(const T* p) {
+  if constexpr (kStage)
+    return *p;
+  else
+    return __ldg(p);
+}
+
 // Internal force of one node with record `me` from its deg incidences
 // starting at p.
-template <class Nodes>
-__device__ __forceinline__ void nodal_force(const Law& L, const Nodes& u, const float4* nfc, int p,
+template <bool kStage = false, class Nodes>
+__device__ __forceinline__ void nodal_force(const Law& L, const Nodes& u, const int4* rec, int p,
                                             int deg, const NodeRec& me, float& a0, float& a1,
                                             float& a2) {
   a0 = 0.f; a1 = 0.f; a2 = 0.f;
   if (deg <= 0) return;
-  const int4* rec = reinterpret_cast<const int4*>(nfc);
-  int4 q = __ldg(rec + p);
+  int4 q = read_only<kStage>(rec + p);
   for (int k = 1;; ++k) {
     const bool more = k < deg;
     int4 qn = q;
     if (more) {
       p += 32;
-      qn = __ldg(rec + p);
+      qn = read_only<kStage>(rec + p);
     }
     const float dx = __int_as_float(q.x), dy = __int_as_float(q.y), dz = __int_as_float(q.z);
     const float4 fc = make_float4(dx, dy, dz, inv_length(dx, dy, dz));
@@ -1026,29 +1066,29 @@ __device__ __forceinline__ void nodal_force(const Law& L, const Nodes& u, const 
 // With kFuse (two copies of the node records) the same thread then drifts
 // the node at once, x += 2 h v with the new v, into the other copy `nxt`:
 // the arithmetic of pass B, without its barrier.
-template <bool kRes, bool kFuse = false, class Nodes>
+template <bool kRes, bool kFuse = false, bool kStage = false, class Nodes>
 __device__ __forceinline__ double nodal_kick(const Law& L, const Nodes& u, const LocalNodes& own,
-                                             float* vel, const float4* nfc,
+                                             float* vel, const int4* rec,
                                              const int2* srow, const float2* mass, int nfo,
                                              float hk, float c, const LocalNodes* nxt = nullptr,
                                              float h2 = 0.f) {
   double part = 0.0;
   int t = threadIdx.x;
   if (t >= nfo) return part;
-  int2 sr = __ldg(srow + t);
-  float2 mm = __ldg(mass + t);
+  int2 sr = read_only<kStage>(srow + t);
+  float2 mm = read_only<kStage>(mass + t);
   for (;;) {
     const int tn = t + kThreadsMixed;
     const bool more = tn < nfo;
     int2 srn = sr;
     float2 mmn = mm;
     if (more) {
-      srn = __ldg(srow + tn);
-      mmn = __ldg(mass + tn);
+      srn = read_only<kStage>(srow + tn);
+      mmn = read_only<kStage>(mass + tn);
     }
     float f[3];
     const NodeRec me = own.load(t);
-    nodal_force(L, u, nfc, sr.x, sr.y, me, f[0], f[1], f[2]);
+    nodal_force<kStage>(L, u, rec, sr.x, sr.y, me, f[0], f[1], f[2]);
     if constexpr (kRes)
       part += static_cast<double>(f[0]) * f[0] + static_cast<double>(f[1]) * f[1] +
               static_cast<double>(f[2]) * f[2];
@@ -1101,9 +1141,16 @@ __device__ __forceinline__ float length_pass(const Rve& r, const Nodes& u, int e
 // each own free node's force, sums the residual on those steps and applies
 // the kick (v += h f / m, both half kicks in one); pass B, after a barrier,
 // drifts the own free nodes (x += 2h v) and moves the RAMP boundary.
-template <int CL, bool kDB = false>
+//
+// kStage (two record copies only): the CTA's incidence records, rows and
+// masses are copied into shared memory first and read there. Else they come
+// from L2 every step, one incidence after the other: small parts, whose step
+// is little more than that chain, and all parts of a cluster, whose barrier
+// drops the L1 cache.
+template <int CL, bool kDB = false, bool kStage = false>
 __device__ void solve_rve_nodal(const DevBatch& b, const MixedState& ms, const RunArgs& a, int rve,
                                 double* red, double* cred, float* smem) {
+  static_assert(kDB || !kStage, "one record copy is taken when two do not fit, let alone staging");
   using Ops = ClusterOps<CL>;
   Rve r;
   r.d = b.desc[rve];
@@ -1141,9 +1188,27 @@ __device__ void solve_rve_nodal(const DevBatch& b, const MixedState& ms, const R
   r.fcon = ms.fconc + fo;
   r.ramp = reinterpret_cast<float*>(b.ramp + 6 * d.bnd_off);
   const int2* srow = ms.nsell + no;  // by node position: (first incidence, degree)
-  const int64_t so = ms.sell_off[rve];
-  const float4* nfc = ms.nfc + so;
-  const float2* mass = ms.mmass + no;
+  const int4* rec = reinterpret_cast<const int4*>(ms.nfc + ms.sell_off[rve]);
+  // the own free nodes' rows, masses and incidence records
+  const int2* own_row = srow + f_lo;
+  const float2* mass = ms.mmass + no + f_lo;
+  const int4* own_rec = rec;
+  if constexpr (kStage) {
+    const int2 part = ms.sell_cta[static_cast<int64_t>(rve) * kMaxCluster + rank];
+    const int q0 = part.x, n_rec = part.y;
+    int4* rec_s = reinterpret_cast<int4*>(smem + stage_offset(slots));
+    int2* row_s = reinterpret_cast<int2*>(rec_s + n_rec);
+    float2* mass_s = reinterpret_cast<float2*>(row_s + nfo);
+    for (int k = tid; k < n_rec; k += kThreadsMixed) rec_s[k] = __ldg(rec + q0 + k);
+    for (int t = tid; t < nfo; t += kThreadsMixed) {
+      const int2 sr = __ldg(own_row + t);
+      row_s[t] = make_int2(sr.x - q0, sr.y);
+      mass_s[t] = __ldg(mass + t);
+    }
+    own_rec = rec_s;
+    own_row = row_s;
+    mass = mass_s;
+  }
   const double* F = a.F + 9 * (a.n_F > 1 ? rve : 0);
   const bool ramp = d.mode == 1;
   double Fm[9];
@@ -1186,10 +1251,10 @@ __device__ void solve_rve_nodal(const DevBatch& b, const MixedState& ms, const R
     // residual sum costs nothing on the others); with two record copies
     // pass B is fused into it and writes the other copy
     const double part =
-        res_step ? nodal_kick<true, kDB>(r.L, u, own, vel, nfc, srow + f_lo, mass + f_lo, nfo, hk,
-                                         c, &nxt, h2)
-                 : nodal_kick<false, kDB>(r.L, u, own, vel, nfc, srow + f_lo, mass + f_lo, nfo,
-                                          hk, c, &nxt, h2);
+        res_step ? nodal_kick<true, kDB, kStage>(r.L, u, own, vel, own_rec, own_row, mass, nfo, hk,
+                                                 c, &nxt, h2)
+                 : nodal_kick<false, kDB, kStage>(r.L, u, own, vel, own_rec, own_row, mass, nfo,
+                                                  hk, c, &nxt, h2);
     if (res_step) {
       residual = sqrt(Ops::template combine<false>(block_sum<kThreadsMixed>(part, red), cred));
       // a break keeps the copy of the step's start: the drift is dropped
@@ -1246,7 +1311,7 @@ __device__ void solve_rve_nodal(const DevBatch& b, const MixedState& ms, const R
     if (i >= NF) {
       const int2 sr = __ldg(srow + i);
       float a0, a1, a2;
-      nodal_force(r.L, u, nfc, sr.x, sr.y, nr, a0, a1, a2);
+      nodal_force(r.L, u, rec, sr.x, sr.y, nr, a0, a1, a2);
       b.fint[no + i] = a0;
       b.fint[nt + no + i] = a1;
       b.fint[2 * nt + no + i] = a2;
@@ -1257,11 +1322,20 @@ __device__ void solve_rve_nodal(const DevBatch& b, const MixedState& ms, const R
   Ops::sync();
 }
 
+// Whether an RVE with two record copies on one CTA is solved with its
+// read-only data staged (up to about 1,400 nodes).
+__device__ __forceinline__ bool stages_one(const DevBatch& b, const MixedState& ms, int rve,
+                                           int smem_floats) {
+  const RveDesc& d = b.desc[rve];
+  return stage_fits(even_slots(d.n_nodes), d.n_free,
+                    ms.sell_cta[static_cast<int64_t>(rve) * kMaxCluster].y, smem_floats);
+}
+
 // Persistent relaxation over one size bucket: CTA (or cluster) after cluster
 // takes the next RVE of `order` (largest first) until the bucket is empty.
 // With NG = 2 each half of the CTA is a group that takes RVEs on its own,
 // in half of the shared memory, synchronised by its own named barrier.
-template <int CL, bool kAll, bool kNodal, int NG, bool kDB>
+template <int CL, bool kAll, bool kNodal, int NG, bool kDB, bool kStage>
 __global__ void __launch_bounds__(kThreadsMixed, 1)
 relax_mixed_kernel(const DevBatch b, const MixedState ms, const RunArgs a, int smem_floats,
                    const int32_t* order, int n_order, int32_t* queue) {
@@ -1292,8 +1366,13 @@ relax_mixed_kernel(const DevBatch b, const MixedState ms, const RunArgs a, int s
       Group<NG>::sync();
     }
     if (rve < 0) break;
-    if constexpr (kNodal)
-      solve_rve_nodal<CL, kDB>(b, ms, a, rve, red, cred, smem);
+    if constexpr (kNodal && CL == 1 && kDB && !kStage) {
+      if (stages_one(b, ms, rve, smem_floats))
+        solve_rve_nodal<1, true, true>(b, ms, a, rve, red, cred, smem);
+      else
+        solve_rve_nodal<1, true>(b, ms, a, rve, red, cred, smem);
+    } else if constexpr (kNodal)
+      solve_rve_nodal<CL, kDB, kStage>(b, ms, a, rve, red, cred, smem);
     else
       solve_rve_mixed<kAll, NG>(b, ms, a, rve, red + g * kRed, smem + g * (smem_floats / NG),
                                 smem_floats / NG);
@@ -1302,7 +1381,10 @@ relax_mixed_kernel(const DevBatch b, const MixedState ms, const RunArgs a, int s
 
 // One RVE solved by one CTA of a serving kernel: with the solve of its batch
 // bucket where that is a single CTA with an order of its own, else with the
-// run-time placement. Every solve gives the same bits.
+// run-time placement; every solve gives the same bits. The serving kernels
+// hold every solve at 64 registers: they do not stage small RVEs' data (one
+// more inlined solve spilled, 96 RVEs served 2 % slower; solves as functions,
+// 8 %).
 __device__ __forceinline__ void serve_one_cta(const DevBatch& b, const MixedState& ms,
                                               const RunArgs& a, int rve, double* red, double* cred,
                                               float* smem, int smem_floats) {
@@ -1481,6 +1563,30 @@ server_cluster_kernel(const DevBatch b, const MixedState ms, const ServerArgs bi
   }
 }
 
+// Device arrays carved out of one allocation, each on a 256-byte boundary.
+class Arena {
+ public:
+  template <typename T>
+  void add(T** p, size_t n) {
+    items_.push_back({reinterpret_cast<void**>(p), bytes_});
+    bytes_ += ((n > 0 ? n : 1) * sizeof(T) + 255) & ~static_cast<size_t>(255);
+  }
+  cudaError_t alloc(void** base) {
+    const cudaError_t e = cudaMalloc(base, bytes_);
+    if (e != cudaSuccess) return e;
+    for (const Item& i : items_) *i.p = static_cast<char*>(*base) + i.at;
+    return cudaSuccess;
+  }
+
+ private:
+  struct Item {
+    void** p;
+    size_t at;
+  };
+  std::vector<Item> items_;
+  size_t bytes_ = 0;
+};
+
 template <typename T>
 cudaError_t alloc(T** p, size_t n) {
   return cudaMalloc(reinterpret_cast<void**>(p), (n > 0 ? n : 1) * sizeof(T));
@@ -1506,10 +1612,11 @@ void ctx_release(MixedRunCtx& c) {
   c = MixedRunCtx{};
 }
 
-// Creates run context `c` (claim counters, streams, events); with
+// Creates run context `c` (claim counters; streams and events of the buckets in use); with
 // own_scratch, also its own run-time placement scratch, sized like the
 // batch's.
-cudaError_t ctx_init(MixedRunCtx& c, size_t nt, size_t et, bool own_scratch) {
+cudaError_t ctx_init(const MixedState& ms, MixedRunCtx& c, size_t nt, size_t et,
+                     bool own_scratch) {
   cudaError_t e;
   if ((e = cudaMalloc(reinterpret_cast<void**>(&c.queues), kBuckets * sizeof(int32_t))) !=
       cudaSuccess)
@@ -1524,6 +1631,7 @@ cudaError_t ctx_init(MixedRunCtx& c, size_t nt, size_t et, bool own_scratch) {
       return e;
   }
   for (int q = 0; q < kBuckets; ++q) {
+    if (ms.bucket_off[q + 1] == ms.bucket_off[q]) continue;
     if ((e = cudaStreamCreateWithFlags(&c.side[q], cudaStreamNonBlocking)) != cudaSuccess)
       return e;
     if ((e = cudaEventCreateWithFlags(&c.join[q], cudaEventDisableTiming)) != cudaSuccess)
@@ -1543,22 +1651,41 @@ void mixed_destroy(MixedState* ms) {
     for (int k = 0; k < kMixedContexts; ++k) ctx_release(ms->ctx[k]);
     delete[] ms->ctx;
   }
-  for (void* p : {static_cast<void*>(ms->u_hl), static_cast<void*>(ms->econn),
-                  static_cast<void*>(ms->icode), static_cast<void*>(ms->mslot),
-                  static_cast<void*>(ms->gnode), static_cast<void*>(ms->mrowptr),
-                  static_cast<void*>(ms->mmass), static_cast<void*>(ms->nsell),
-                  static_cast<void*>(ms->sell_off), static_cast<void*>(ms->ncode),
-                  static_cast<void*>(ms->nfc), static_cast<void*>(ms->nfib_tmp),
-                  static_cast<void*>(ms->fconc),
-                  static_cast<void*>(ms->v), static_cast<void*>(ms->mass),
-                  static_cast<void*>(ms->fcon), static_cast<void*>(ms->nrm),
-                  static_cast<void*>(ms->order), static_cast<void*>(ms->rve_bucket)})
+  for (void* p : {ms->arrays, ms->set_up, static_cast<void*>(ms->nfc)})
     if (p) cudaFree(p);
   delete[] ms->h_cl;
   delete ms;
 }
 
 namespace {
+
+// Incidence records that a CTA of a cluster of cl stages at most for its free
+// nodes: their degrees, and what slices of 32 nodes as wide as their widest
+// row add (the nodes are in falling degree within two groups, so a slice is
+// no wider than the mean row of the one before it but for each group's first
+// two).
+int64_t stage_records(const RveDesc& d, int cl, const int32_t* rowptr) {
+  const int NF = d.n_free, fchunk = (NF + cl - 1) / cl;
+  int64_t most = 0;
+  for (int lo = 0; lo < NF; lo += fchunk) {
+    const int hi = std::min(NF, lo + fchunk);
+    int widest = 0;
+    for (int j = lo; j < hi; ++j) widest = std::max(widest, rowptr[j + 1] - rowptr[j]);
+    most = std::max<int64_t>(most, rowptr[hi] - rowptr[lo] + 96LL * widest);
+  }
+  return most;
+}
+
+// Whether launch kind k holds an RVE in its CTAs' shared memory.
+bool holds(const BucketKind& k, const RveDesc& d, const int32_t* rowptr, int64_t smem_floats) {
+  if (cluster_floats(d.n_nodes, d.n_free, d.n_fibers, k.cl, k.all && !k.nodal, k.db) >
+      smem_floats / k.ng)
+    return false;
+  if (!k.stage) return true;
+  const int nb = d.n_nodes - d.n_free, fchunk = (d.n_free + k.cl - 1) / k.cl;
+  return stage_fits(even_slots(fchunk + (nb + k.cl - 1) / k.cl), fchunk,
+                    stage_records(d, k.cl, rowptr), smem_floats);
+}
 
 // Bucket of an RVE: the smallest of one CTA or a cluster of 2, 4 or 8 CTAs
 // whose shared memory holds its node state (node-centric solve; at that
@@ -1578,25 +1705,23 @@ namespace {
 // exponential the node-centric solve would evaluate at both ends of every
 // fiber, and the node-centric one for the linear law, where it runs 2 %
 // (500 - 1,300 nodes) to 37 % (1,300 - 3,300 nodes) faster.
-int bucket_of(const RveDesc& d, int smem_floats, int max_cluster, bool serving_layout,
-              int small_solve, int rves_per_cta) {
+int bucket_of(const RveDesc& d, const int32_t* rowptr, int smem_floats, int max_cluster,
+              bool serving_layout, int small_solve, int rves_per_cta) {
   const bool fiber_small =
       small_solve == MFG_SMALL_FIBER_CENTRIC ||
       (small_solve == MFG_SMALL_AUTO && d.law == MFG_LAW_NONLINEAR);
   for (int q : kPref)
     if ((fiber_small || !kBucket[q].all) && kBucket[q].cl <= max_cluster &&
         !(serving_layout && kBucket[q].cl == 2) && kBucket[q].ng <= rves_per_cta &&
-        cluster_floats(d.n_nodes, d.n_free, d.n_fibers, kBucket[q].cl,
-                       kBucket[q].all && !kBucket[q].nodal, kBucket[q].db) <=
-            smem_floats / kBucket[q].ng)
+        holds(kBucket[q], d, rowptr, smem_floats))
       return q;
-  return kBuckets - 1;
+  return kQRuntime;
 }
 
-// Calls fn(std::integral_constant<int, q>{}) for the run-time bucket index q.
+// Calls fn(std::integral_constant<int, k>{}) for the run-time launch kind k.
 template <class Fn>
-cudaError_t with_bucket(int q, Fn&& fn) {
-  switch (q) {
+cudaError_t with_kind(int k, Fn&& fn) {
+  switch (k) {
     case 0: return fn(std::integral_constant<int, 0>{});
     case 1: return fn(std::integral_constant<int, 1>{});
     case 2: return fn(std::integral_constant<int, 2>{});
@@ -1607,10 +1732,17 @@ cudaError_t with_bucket(int q, Fn&& fn) {
     case 7: return fn(std::integral_constant<int, 7>{});
     case 8: return fn(std::integral_constant<int, 8>{});
     case 9: return fn(std::integral_constant<int, 9>{});
+    case 10: return fn(std::integral_constant<int, 10>{});
+    case 11: return fn(std::integral_constant<int, 11>{});
+    case 12: return fn(std::integral_constant<int, 12>{});
+    case 13: return fn(std::integral_constant<int, 13>{});
+    case 14: return fn(std::integral_constant<int, 14>{});
+    case 15: return fn(std::integral_constant<int, 15>{});
+    case 16: return fn(std::integral_constant<int, 16>{});
     default: return cudaErrorInvalidValue;
   }
 }
-static_assert(kBuckets == 10, "with_bucket covers every bucket");
+static_assert(kKinds == 17, "with_kind covers every launch kind");
 
 template <int CL, bool kAll>
 cudaLaunchConfig_t launch_config(const MixedState& ms, unsigned grid, cudaStream_t s,
@@ -1629,41 +1761,144 @@ cudaLaunchConfig_t launch_config(const MixedState& ms, unsigned grid, cudaStream
   return cfg;
 }
 
-template <int Q>
-cudaError_t launch_bucket(const MixedState& ms, const DevBatch& b, const RunArgs& a,
+template <int K>
+cudaError_t launch_bucket(const MixedState& ms, int q, const DevBatch& b, const RunArgs& a,
                           int32_t* queue, cudaStream_t s) {
-  constexpr BucketKind k = kBucket[Q];
-  const int n = ms.bucket_off[Q + 1] - ms.bucket_off[Q];
+  constexpr BucketKind k = kKind[K];
+  const int n = ms.bucket_off[q + 1] - ms.bucket_off[q];
   cudaLaunchAttribute attr[1];
   cudaLaunchConfig_t cfg =
-      launch_config<k.cl, k.all>(ms, static_cast<unsigned>(ms.bucket_grid[Q]), s, attr);
-  return cudaLaunchKernelEx(&cfg, relax_mixed_kernel<k.cl, k.all, k.nodal, k.ng, k.db>, b, ms, a,
+      launch_config<k.cl, k.all>(ms, static_cast<unsigned>(ms.bucket_grid[q]), s, attr);
+  return cudaLaunchKernelEx(&cfg, relax_mixed_kernel<k.cl, k.all, k.nodal, k.ng, k.db, k.stage>, b, ms, a,
                             static_cast<int>(ms.smem_bytes / sizeof(float)),
-                            static_cast<const int32_t*>(ms.order + ms.bucket_off[Q]), n, queue);
+                            static_cast<const int32_t*>(ms.order + ms.bucket_off[q]), n, queue);
 }
 
-template <int Q>
-cudaError_t setup_bucket(MixedState& ms, int n) {
-  constexpr BucketKind k = kBucket[Q];
-  cudaError_t e = cudaFuncSetAttribute(relax_mixed_kernel<k.cl, k.all, k.nodal, k.ng, k.db>,
-                                       cudaFuncAttributeMaxDynamicSharedMemorySize,
+// Makes launch kind K ready and returns the clusters of it (CTAs for cl = 1)
+// the device holds at once, one CTA per SM.
+template <int K>
+cudaError_t setup_kind(const MixedState& ms, int* clusters) {
+  constexpr BucketKind k = kKind[K];
+  auto kernel = relax_mixed_kernel<k.cl, k.all, k.nodal, k.ng, k.db, k.stage>;
+  cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                        ms.smem_bytes);
+  if (e == cudaSuccess && k.cl > 8)
+    e = cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
   if (e != cudaSuccess) return e;
-  int clusters = ms.sms;
-  if (k.cl > 1 && n > 0) {
+  *clusters = ms.sms;
+  if (k.cl > 1) {
     cudaLaunchAttribute attr[1];
     cudaLaunchConfig_t cfg =
         launch_config<k.cl, k.all>(ms, static_cast<unsigned>(k.cl * ms.sms), nullptr, attr);
-    clusters = 0;
-    if ((e = cudaOccupancyMaxActiveClusters(&clusters,
-                                            relax_mixed_kernel<k.cl, k.all, k.nodal, k.ng, k.db>,
-                                            &cfg)) != cudaSuccess)
-      return e;
-    if (clusters < 1) return cudaErrorInvalidConfiguration;
+    *clusters = 0;
+    if ((e = cudaOccupancyMaxActiveClusters(clusters, kernel, &cfg)) != cudaSuccess) return e;
   }
-  // CTAs (or clusters) for n RVEs at k.ng RVEs each, at most one per SM
-  ms.bucket_grid[Q] = k.cl * std::min((n + k.ng - 1) / k.ng, clusters);
   return cudaSuccess;
+}
+
+// ---- width of the size buckets ------------------------------------------------
+
+// Time of a step of one RVE in launch kind k, in microseconds: fitted to one
+// RVE of 500 to 20,000 nodes at every cluster size. Linear law, nodes: us on
+// 1, 2, 4, 8, 16 CTAs -- 1,000: 2.4, -, 2.3, 2.3, -; 4,500: 9.8, 6.0, 3.5,
+// 2.7, 2.6; 20,000: (100 in global memory), -, 13.1, 7.4, 4.6.
+double step_us(const RveDesc& d, const BucketKind& k) {
+  const bool nl = d.law == MFG_LAW_NONLINEAR;
+  if (k.all) return k.ng == 2 ? 0.0016 * d.n_fibers + 1.45 : 0.00115 * d.n_fibers + 2.0;
+  if (!k.nodal) return 0.002 * d.n_fibers;  // (part of) the state in global memory
+  double fixed = k.cl == 1 ? 1.5 : k.cl == 2 ? 1.9 : k.cl == 4 ? 2.4 : k.cl == 8 ? 2.8 : 3.6;
+  if (k.stage || (k.cl == 1 && k.db && d.n_nodes < 1350))
+    fixed = k.cl == 1 ? 0.9 : k.cl == 2 ? 1.3 : k.cl == 4 ? 1.5 : k.cl == 8 ? 1.7 : 2.0;
+  if (!k.db) fixed += 1.2;
+  if (nl) fixed += 0.8;
+  const double per_fiber = nl ? (k.cl == 1 ? 0.0016 : 0.0022) : 0.00075;
+  return per_fiber * d.n_fibers / k.cl + fixed;
+}
+
+// Time of `copies` solves of the batch with the buckets in these kinds: RVE
+// after RVE, bucket by bucket with the largest clusters first and the longest
+// first in a bucket, each onto the SMs that are free first. clusters[k] of a
+// kind run at once, so each takes that share of the SMs.
+double batch_us(const std::vector<RveDesc>& desc, const std::vector<std::vector<int32_t>>& bucket,
+                const int* kind, const int* clusters, int sms, int copies) {
+  std::vector<int> order;
+  for (int q = 0; q < kBuckets; ++q)
+    if (!bucket[q].empty()) order.push_back(q);
+  std::stable_sort(order.begin(), order.end(),
+                   [&](int x, int y) { return kKind[kind[x]].cl > kKind[kind[y]].cl; });
+  std::vector<double> sm(sms, 0.0);  // when each SM is free, ascending
+  for (int q : order) {
+    const BucketKind& k = kKind[kind[q]];
+    const int share = k.cl == 1 ? 1 : std::min(sms, (sms + clusters[kind[q]] - 1) / clusters[kind[q]]);
+    const size_t n = bucket[q].size() * copies;
+    for (size_t i = 0; i < n; i += k.ng) {
+      const RveDesc& d = desc[bucket[q][i / copies]];
+      // two RVEs side by side on a CTA take 1.4 times as long as one there
+      const double t = step_us(d, k) * d.max_steps * (i + 1 < n && k.ng == 2 ? 1.4 : 1.0);
+      const double done = sm[share - 1] + t;
+      sm.erase(sm.begin(), sm.begin() + share);
+      sm.insert(std::upper_bound(sm.begin(), sm.end(), done), share, done);
+    }
+  }
+  return sm.back();
+}
+
+// Widens buckets while the batch's estimated time falls: a batch that leaves
+// SMs idle solves its RVEs on larger clusters than they need. Starts from
+// each bucket's own kind in `kind`; RVEs in global memory (the run-time placement)
+// go to clusters of 16 where those hold them. Bucket by bucket, so that a
+// batch keeps one launch per size bucket.
+void choose_kinds(const std::vector<RveDesc>& desc,
+                  const std::vector<std::vector<int32_t>>& bucket,
+                  const std::vector<int32_t>& rowptr, int smem_floats, int max_cluster,
+                  bool keep_fiber_centric, const int* clusters, int sms,
+                  int copies, int* kind) {
+  auto fits = [&](int q, int k) {
+    for (int32_t r : bucket[q])
+      if (!holds(kKind[k], desc[r], rowptr.data() + desc[r].row_off, smem_floats)) return false;
+    return true;
+  };
+  // the kind of cl CTAs for bucket q: staged, else two record copies, else one
+  auto wider = [&](int q, int cl) {
+    for (int level = 2; level >= 0; --level)
+      for (int k = 0; k < kKinds; ++k)
+        if (kKind[k].nodal && kKind[k].cl == cl && kKind[k].stage + kKind[k].db == level &&
+            clusters[k] > 0 && fits(q, k))
+          return k;
+    return -1;
+  };
+  // widen the bucket whose RVE takes longest, again and again; keep the best
+  // state met (a state no better than the one before it may lead to one)
+  int best[kBuckets], now[kBuckets];
+  std::copy(kind, kind + kBuckets, best);
+  std::copy(kind, kind + kBuckets, now);
+  double t_best = batch_us(desc, bucket, kind, clusters, sms, copies);
+  for (;;) {
+    int q_long = -1;
+    double longest = 0.0;
+    for (int q = 0; q < kBuckets; ++q)
+      for (int32_t r : bucket[q]) {
+        const double t = step_us(desc[r], kKind[now[q]]) * desc[r].max_steps;
+        if (t > longest) {
+          longest = t;
+          q_long = q;
+        }
+      }
+    if (q_long < 0 || (kKind[now[q_long]].all && keep_fiber_centric)) break;
+    int k = -1;
+    for (int cl = 2 * kKind[now[q_long]].cl; k < 0 && cl <= max_cluster; cl *= 2)
+      k = wider(q_long, cl);
+    if (k < 0) break;
+    now[q_long] = k;
+    const double t = batch_us(desc, bucket, now, clusters, sms, copies);
+    if (t < 0.97 * t_best) {  // a wider bucket has to pay
+      t_best = t;
+      std::copy(now, now + kBuckets, best);
+    } else if (t > 1.15 * t_best) {
+      break;
+    }
+  }
+  std::copy(best, best + kBuckets, kind);
 }
 
 }  // namespace
@@ -1672,34 +1907,20 @@ cudaError_t mixed_create(MixedState& ms, const DevBatch& b, const std::vector<Rv
                          const std::vector<int2>& conn, const std::vector<int32_t>& rowptr,
                          const std::vector<int32_t>& inc, int sms, int max_cluster,
                          bool serving_layout, int small_solve, int rves_per_cta,
-                         cudaStream_t s) {
+                         int copies, cudaStream_t s) {
   cudaError_t e;
   const size_t nt = static_cast<size_t>(b.nt), et = static_cast<size_t>(b.et);
-  if ((e = alloc(&ms.u_hl, 6 * nt)) != cudaSuccess) return e;
-  if ((e = alloc(&ms.v, 3 * nt)) != cudaSuccess) return e;
-  if ((e = alloc(&ms.mass, nt)) != cudaSuccess) return e;
-  if ((e = alloc(&ms.fcon, et)) != cudaSuccess) return e;
-  if ((e = alloc(&ms.nrm, et)) != cudaSuccess) return e;
-  if ((e = alloc(&ms.econn, et)) != cudaSuccess) return e;
-  if ((e = alloc(&ms.fconc, et)) != cudaSuccess) return e;
-  if ((e = alloc(&ms.icode, 2 * et)) != cudaSuccess) return e;
-  if ((e = alloc(&ms.mslot, et)) != cudaSuccess) return e;
-  if ((e = alloc(&ms.gnode, nt)) != cudaSuccess) return e;
-  if ((e = alloc(&ms.mrowptr, rowptr.size())) != cudaSuccess) return e;
-  if ((e = alloc(&ms.mmass, nt)) != cudaSuccess) return e;
-  if ((e = alloc(&ms.order, desc.size())) != cudaSuccess) return e;
   ms.ctx = new MixedRunCtx[kMixedContexts];
-  if ((e = ctx_init(ms.ctx[0], nt, et, false)) != cudaSuccess) return e;
   ms.sms = sms;
   ms.smem_bytes = kSmemBytesMixed;
   const int smem_floats = kSmemBytesMixed / static_cast<int>(sizeof(float));
-  if ((e = cudaFuncSetAttribute(server_mixed_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                kSmemBytesMixed)) != cudaSuccess ||
-      (e = cudaFuncSetAttribute(server_cluster_kernel,
-                                cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytesMixed)) !=
-          cudaSuccess)
-    return e;
-  {
+  if (serving_layout) {
+    if ((e = cudaFuncSetAttribute(server_mixed_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                  kSmemBytesMixed)) != cudaSuccess ||
+        (e = cudaFuncSetAttribute(server_cluster_kernel,
+                                  cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytesMixed)) !=
+            cudaSuccess)
+      return e;
     cudaLaunchAttribute attr[1];
     cudaLaunchConfig_t cfg = launch_config<kClusterServe, false>(
         ms, static_cast<unsigned>(kClusterServe * sms), nullptr, attr);
@@ -1713,15 +1934,74 @@ cudaError_t mixed_create(MixedState& ms, const DevBatch& b, const std::vector<Rv
   // size buckets, each in longest-processing-time order
   std::vector<std::vector<int32_t>> bucket(kBuckets);
   std::vector<int> rve_q(desc.size());
-  ms.h_cl = new int32_t[std::max<size_t>(desc.size(), 1)];
   for (size_t r = 0; r < desc.size(); ++r) {
-    rve_q[r] = bucket_of(desc[r], smem_floats, max_cluster, serving_layout, small_solve,
-                         rves_per_cta);
+    rve_q[r] = bucket_of(desc[r], rowptr.data() + desc[r].row_off, smem_floats,
+                         std::min(max_cluster, 8), serving_layout, small_solve, rves_per_cta);
     bucket[rve_q[r]].push_back(static_cast<int32_t>(r));
-    ms.h_cl[r] = kBucket[rve_q[r]].cl;
   }
-  if ((e = alloc(&ms.rve_bucket, desc.size())) != cudaSuccess ||
-      (!desc.empty() &&
+  int clusters[kKinds] = {};
+  for (int q = 0; q < kBuckets; ++q) {
+    std::stable_sort(bucket[q].begin(), bucket[q].end(),
+                     [&](int32_t x, int32_t y) { return desc[x].n_fibers > desc[y].n_fibers; });
+    ms.bucket_kind[q] = q;
+  }
+  // Wider clusters: not in the serving layout (its kernels solve in clusters
+  // of 4), and not worth estimating for a batch that fills the GPU many times.
+  // For several solves at once only where they leave a third of the SMs idle:
+  // their clusters wait for neighbouring SMs to fall free (six solves of 32
+  // RVEs of 1,000 - 10,000 nodes, 200 steps: 4.2 ms widened, 3.7 not; of 8 RVEs
+  // of 500 - 20,000, 84 SMs of 152: 1.7 ms, 2.8 not).
+  size_t ctas = 0;
+  for (int q = 0; q < kBuckets; ++q) ctas += bucket[q].size() * copies * kBucket[q].cl;
+  const bool widen = !serving_layout &&
+                     (!bucket[kQRuntime].empty() ||
+                      (copies == 1 ? desc.size() <= 8 * static_cast<size_t>(sms)
+                                   : 3 * ctas <= 2 * static_cast<size_t>(sms)));
+  for (int k = 0; k < kKinds; ++k) {
+    const bool used = k < kBuckets && !bucket[k].empty();
+    if (!used && !(widen && kKind[k].nodal && kKind[k].cl > 1 && kKind[k].cl <= max_cluster))
+      continue;
+    e = with_kind(k, [&](auto K) { return setup_kind<decltype(K)::value>(ms, &clusters[k]); });
+    if (e != cudaSuccess) {
+      if (used) return e;
+      cudaGetLastError();  // a wider kind this device does not run
+      clusters[k] = 0;
+    }
+    if (used && clusters[k] < 1) return cudaErrorInvalidConfiguration;
+  }
+  if (widen)
+    choose_kinds(desc, bucket, rowptr, smem_floats, max_cluster, small_solve == MFG_SMALL_FIBER_CENTRIC,
+                 clusters, sms, copies, ms.bucket_kind);
+  ms.h_cl = new int32_t[std::max<size_t>(desc.size(), 1)];
+  for (size_t r = 0; r < desc.size(); ++r) ms.h_cl[r] = kKind[ms.bucket_kind[rve_q[r]]].cl;
+  auto kind_of = [&](size_t r) -> const BucketKind& { return kKind[ms.bucket_kind[rve_q[r]]]; };
+  // The arrays whose sizes are known, in one allocation. The node records,
+  // velocities and force vectors in global memory are the run-time
+  // placement's, which the serving kernels may take for an RVE of any bucket.
+  const bool scratch = serving_layout || (!bucket[kQRuntime].empty() &&
+                                          ms.bucket_kind[kQRuntime] == kQRuntime);
+  Arena arena;
+  if (scratch) {
+    arena.add(&ms.u_hl, 6 * nt);
+    arena.add(&ms.v, 3 * nt);
+    arena.add(&ms.nrm, et);
+  }
+  arena.add(&ms.mass, nt);
+  arena.add(&ms.fcon, et);
+  arena.add(&ms.econn, et);
+  arena.add(&ms.fconc, et);
+  arena.add(&ms.icode, 2 * et);
+  arena.add(&ms.mslot, et);
+  arena.add(&ms.gnode, nt);
+  arena.add(&ms.mrowptr, rowptr.size());
+  arena.add(&ms.mmass, nt);
+  arena.add(&ms.order, desc.size());
+  arena.add(&ms.rve_bucket, desc.size());
+  arena.add(&ms.nsell, nt);
+  arena.add(&ms.sell_cta, desc.size() * kMaxCluster);
+  arena.add(&ms.sell_off, desc.size());
+  if ((e = arena.alloc(&ms.arrays)) != cudaSuccess) return e;
+  if ((!desc.empty() &&
        (e = cudaMemcpy(ms.rve_bucket, rve_q.data(), desc.size() * sizeof(int32_t),
                        cudaMemcpyHostToDevice)) != cudaSuccess))
     return e;
@@ -1730,13 +2010,13 @@ cudaError_t mixed_create(MixedState& ms, const DevBatch& b, const std::vector<Rv
     std::vector<int2> econn(et);
     std::vector<int32_t> icode(2 * et), mslot(et), gnode(nt), mrowptr(rowptr.size());
     std::vector<std::thread> pool;
-    const int nthr = std::max(1u, std::min(16u, std::thread::hardware_concurrency()));
+    const int nthr = static_cast<int>(std::max<size_t>(
+        1, std::min<size_t>({16, std::thread::hardware_concurrency(), desc.size()})));
     for (int t = 0; t < nthr; ++t)
       pool.emplace_back([&, t] {
         for (size_t r = t; r < desc.size(); r += nthr)
-          cluster_order(desc[r], kBucket[rve_q[r]].cl,
-                        kBucket[rve_q[r]].all || kBucket[rve_q[r]].nodal,
-                        kBucket[rve_q[r]].nodal, conn, rowptr, inc, econn, icode, mslot, gnode,
+          cluster_order(desc[r], kind_of(r).cl, kind_of(r).all || kind_of(r).nodal,
+                        kind_of(r).nodal, conn, rowptr, inc, econn, icode, mslot, gnode,
                         mrowptr);
       });
     for (auto& th : pool) th.join();
@@ -1759,8 +2039,8 @@ cudaError_t mixed_create(MixedState& ms, const DevBatch& b, const std::vector<Rv
       for (int t = 0; t < nthr; ++t)
         sp.emplace_back([&, t] {
           for (size_t r = t; r < desc.size(); r += nthr)
-            if (kBucket[rve_q[r]].nodal)
-              sell_off[r + 1] = sell_layout(desc[r], kBucket[rve_q[r]].cl, conn, rowptr, inc,
+            if (kind_of(r).nodal)
+              sell_off[r + 1] = sell_layout(desc[r], kind_of(r).cl, conn, rowptr, inc,
                                             gnode, 0, nullptr, nullptr, nullptr);
         });
       for (auto& th : sp) th.join();
@@ -1776,17 +2056,39 @@ cudaError_t mixed_create(MixedState& ms, const DevBatch& b, const std::vector<Rv
       for (int t = 0; t < nthr; ++t)
         sp.emplace_back([&, t] {
           for (size_t r = t; r < desc.size(); r += nthr)
-            if (kBucket[rve_q[r]].nodal)
-              sell_layout(desc[r], kBucket[rve_q[r]].cl, conn, rowptr, inc, gnode, sell_off[r],
+            if (kind_of(r).nodal)
+              sell_layout(desc[r], kind_of(r).cl, conn, rowptr, inc, gnode, sell_off[r],
                           nsell.data(), ncode.data(), nfib.data());
         });
       for (auto& th : sp) th.join();
     }
-    if ((e = alloc(&ms.nsell, nt)) != cudaSuccess ||
-        (e = alloc(&ms.sell_off, desc.size())) != cudaSuccess ||
-        (e = alloc(&ms.ncode, static_cast<size_t>(n_sell))) != cudaSuccess ||
+    // the incidence records of each CTA's free nodes
+    std::vector<int2> sell_cta(desc.size() * kMaxCluster, make_int2(0, 0));
+    for (size_t r = 0; r < desc.size(); ++r) {
+      const bool one = ms.bucket_kind[rve_q[r]] == kQNodalDB;
+      if (!kind_of(r).stage && !one) continue;
+      const RveDesc& d = desc[r];
+      const int fchunk = (d.n_free + kind_of(r).cl - 1) / kind_of(r).cl;
+      for (int P = 0; P < d.n_free; ++P) {
+        int2& part = sell_cta[r * kMaxCluster + P / fchunk];
+        const int2 row = nsell[d.node_off + P];
+        if (P % fchunk == 0) part.x = row.x;
+        part.y = std::max(part.y, row.x + 32 * (row.y - 1) + 1 - part.x);
+      }
+      const int nb = d.n_nodes - d.n_free, cl = kind_of(r).cl;
+      for (int o = 0; o < cl && !one; ++o)  // stage_records() is an upper bound
+        if (!stage_fits(even_slots(fchunk + (nb + cl - 1) / cl), fchunk,
+                        sell_cta[r * kMaxCluster + o].y, smem_floats))
+          return cudaErrorInvalidValue;
+    }
+    Arena set_up;
+    set_up.add(&ms.ncode, static_cast<size_t>(n_sell));
+    set_up.add(&ms.nfib_tmp, static_cast<size_t>(n_sell));
+    if ((!sell_cta.empty() &&
+         (e = cudaMemcpy(ms.sell_cta, sell_cta.data(), sell_cta.size() * sizeof(int2),
+                         cudaMemcpyHostToDevice)) != cudaSuccess) ||
         (e = alloc(&ms.nfc, static_cast<size_t>(n_sell))) != cudaSuccess ||
-        (e = alloc(&ms.nfib_tmp, static_cast<size_t>(n_sell))) != cudaSuccess)
+        (e = set_up.alloc(&ms.set_up)) != cudaSuccess)
       return e;
     if ((e = cudaMemcpy(ms.nsell, nsell.data(), nt * sizeof(int2), cudaMemcpyHostToDevice)) !=
             cudaSuccess ||
@@ -1803,8 +2105,6 @@ cudaError_t mixed_create(MixedState& ms, const DevBatch& b, const std::vector<Rv
   std::vector<int32_t> order;
   order.reserve(desc.size());
   for (int q = 0; q < kBuckets; ++q) {
-    std::stable_sort(bucket[q].begin(), bucket[q].end(),
-                     [&](int32_t x, int32_t y) { return desc[x].n_fibers > desc[y].n_fibers; });
     ms.bucket_off[q] = static_cast<int>(order.size());
     order.insert(order.end(), bucket[q].begin(), bucket[q].end());
   }
@@ -1815,9 +2115,15 @@ cudaError_t mixed_create(MixedState& ms, const DevBatch& b, const std::vector<Rv
     return e;
   for (int q = 0; q < kBuckets; ++q) {
     const int n = ms.bucket_off[q + 1] - ms.bucket_off[q];
-    e = with_bucket(q, [&](auto Q) { return setup_bucket<decltype(Q)::value>(ms, n); });
-    if (e != cudaSuccess) return e;
+    const BucketKind& k = kKind[ms.bucket_kind[q]];
+    // CTAs (or clusters) for n RVEs at k.ng RVEs each, at most one CTA per SM
+    ms.bucket_grid[q] = k.cl * std::min((n + k.ng - 1) / k.ng, clusters[ms.bucket_kind[q]]);
+    ms.launch_order[q] = q;
   }
+  std::stable_sort(ms.launch_order, ms.launch_order + kBuckets, [&](int x, int y) {
+    return kKind[ms.bucket_kind[x]].cl > kKind[ms.bucket_kind[y]].cl;
+  });
+  if ((e = ctx_init(ms, ms.ctx[0], nt, et, false)) != cudaSuccess) return e;
 
   const int64_t n = std::max<int64_t>(b.nt, 1);
   mixed_prepare_kernel<<<static_cast<unsigned>((n + 255) / 256), 256, 0, s>>>(b, ms);
@@ -1837,11 +2143,17 @@ cudaError_t mixed_create(MixedState& ms, const DevBatch& b, const std::vector<Rv
   }
   // the fiber ids were only needed to fill the incidences' fiber data
   if ((e = cudaStreamSynchronize(s)) != cudaSuccess) return e;
-  cudaFree(ms.nfib_tmp);
-  ms.nfib_tmp = nullptr;
-  cudaFree(ms.ncode);
-  ms.ncode = nullptr;
+  cudaFree(ms.set_up);
+  ms.set_up = nullptr;
   return cudaSuccess;
+}
+
+bool mixed_widened(const MixedState& ms) {
+  for (int q = 0; q < kBuckets; ++q)
+    if (ms.bucket_off[q + 1] > ms.bucket_off[q] && ms.bucket_kind[q] != q &&
+        kKind[ms.bucket_kind[q]].cl > kKind[q].cl)
+      return true;
+  return false;
 }
 
 int mixed_rve_cluster(const MixedState& ms, int rve) { return ms.h_cl ? ms.h_cl[rve] : 1; }
@@ -1876,13 +2188,13 @@ cudaError_t enqueue_buckets(const MixedState& ms, MixedRunCtx& c, const DevBatch
   *launches = 0;
   if ((e = cudaMemsetAsync(c.queues, 0, kBuckets * sizeof(int32_t), s)) != cudaSuccess) return e;
   if ((e = cudaEventRecord(c.fork, s)) != cudaSuccess) return e;
-  for (int q = 0; q < kBuckets; ++q) {
+  for (int q : ms.launch_order) {
     if (ms.bucket_off[q + 1] == ms.bucket_off[q]) continue;
     cudaStream_t sq = c.side[q];
     if ((e = cudaStreamWaitEvent(sq, c.fork, 0)) != cudaSuccess) return e;
     int32_t* queue = c.queues + q;
-    e = with_bucket(q, [&](auto Q) {
-      return launch_bucket<decltype(Q)::value>(ms, b, a, queue, sq);
+    e = with_kind(ms.bucket_kind[q], [&](auto K) {
+      return launch_bucket<decltype(K)::value>(ms, q, b, a, queue, sq);
     });
     if (e != cudaSuccess) return e;
     ++*launches;
@@ -1904,10 +2216,11 @@ cudaError_t mixed_prepare_contexts(MixedState& ms, const DevBatch& b, int n) {
   if (n >= kMixedContexts) return cudaErrorInvalidValue;
   // the run-time placement keeps node records, velocities and force vectors
   // in global memory: concurrent runs need their own
-  const bool runtime_bucket = ms.bucket_off[kBuckets] > ms.bucket_off[kBuckets - 1];
+  const bool runtime_bucket = ms.bucket_off[kQRuntime + 1] > ms.bucket_off[kQRuntime] &&
+                              ms.bucket_kind[kQRuntime] == kQRuntime;
   for (int k = 1; k <= n; ++k) {
     if (ms.ctx[k].ready) continue;
-    cudaError_t e = ctx_init(ms.ctx[k], static_cast<size_t>(b.nt), static_cast<size_t>(b.et),
+    cudaError_t e = ctx_init(ms, ms.ctx[k], static_cast<size_t>(b.nt), static_cast<size_t>(b.et),
                              runtime_bucket);
     if (e != cudaSuccess) {
       ctx_release(ms.ctx[k]);
