@@ -90,15 +90,17 @@ void f64_parts(const RveDesc& d, int cl, const int2* conn, const int32_t* rowptr
 
 namespace {
 
-// Time of a step of one RVE over CL = 2^k CTAs, in microseconds: the FP64
-// pipe's share (16 ns a fiber on one SM; a part also evaluates the fibers it
-// shares, a surface term), and what does not shrink with CL. Measured, one
-// RVE on 16 CTAs: 5.0 us at 1,000 nodes, 16.2 at 4,500, 52 at 20,000 (42, 165
-// and 740 us on one CTA); 36 RVEs of 4,500 nodes on 4 CTAs each 51 us.
+// Time of a step of one RVE over CL = 2^k CTAs, in microseconds: the fibers'
+// share (8 ns a fiber on one SM; a part also evaluates the fibers it shares, a
+// surface term), and what does not shrink with CL. Measured, one RVE on 16
+// CTAs: 3.7 us at 1,000 nodes, 9.7 at 4,500, 30 at 20,000; 36 RVEs of 4,500
+// nodes on 4 CTAs each 28 us; on single CTAs 120 us alone on an SM, 178 us for
+// two.
 double f64_step_us(const RveDesc& d, int k) {
   const double cl = 1 << k, fibers = d.n_fibers / cl;
-  const double shared = k == 0 ? 0.0 : std::pow(std::max(1.0, d.n_nodes / cl), -1.0 / 3.0);
-  return 0.016 * fibers * (1.0 + shared) + (k == 0 ? 2.0 : 3.0);
+  if (k == 0) return 0.0080 * fibers + 2.0;  // as one of two RVEs on an SM
+  const double shared = std::pow(std::max(1.0, d.n_nodes / cl), -1.0 / 3.0);
+  return 0.0082 * fibers * (1.0 + shared) + 3.0;
 }
 
 }  // namespace
@@ -111,7 +113,8 @@ double f64_batch_step_us(const std::vector<RveDesc>& desc, int k, int clusters, 
   std::sort(t.begin(), t.end(), std::greater<double>());
   std::priority_queue<double, std::vector<double>, std::greater<double>> free_at;
   for (int c = 0; c < std::max(1, clusters); ++c) free_at.push(0.0);
-  double end = 0.0;
+  // a single CTA alone on its SM does not fill it
+  double end = k == 0 && !t.empty() ? 1.3 * t.front() : 0.0;
   for (double x : t) {
     const double at = free_at.top() + x;
     free_at.pop();

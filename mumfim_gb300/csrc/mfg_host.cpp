@@ -337,7 +337,7 @@ struct mfg_batch {
   // FP64: every RVE split over a cluster of f64_plan.cl CTAs, f64_clusters of
   // them at once (cl 1: no clusters), and whether the six concurrent solves
   // of the stiffness run that way too
-  mfg::F64Plan f64_plan{1, 0};
+  mfg::F64Plan f64_plan{1, 0, 0};
   int f64_clusters = 0;
   bool f64_stiffness_clusters = false;
   DevArray<unsigned char> d_plan;
@@ -407,7 +407,8 @@ mfg_status upload(DevArray<T>& d, const std::vector<T>& h, cudaStream_t s) {
 
 // FP64: chooses the cluster size for the batch (f64_cluster_size) and, when
 // it is above 1, builds and uploads the RVEs' parts (f64_parts). `m` holds
-// the masses, 1 / m and m c, `l0` the lengths and 1 / l0, `nt` and `et` apart.
+// the masses, their reciprocals and m c, `l0` the lengths and their
+// reciprocals, `nt` and `et` apart.
 mfg_status plan_f64_clusters(mfg_batch* b, const std::vector<double>& m,
                              const std::vector<double>& l0, const std::vector<int2>& conn,
                              const std::vector<int32_t>& rowptr, const std::vector<int32_t>& inc,
@@ -460,7 +461,7 @@ mfg_status plan_f64_clusters(mfg_batch* b, const std::vector<double>& m,
   const size_t o_rows = take(n.row, sizeof(int32_t));
   const size_t o_inc = take(n.inc, sizeof(int32_t));
   const size_t o_ends = take(n.fib, sizeof(int2));
-  const size_t o_len = take(n.fib, sizeof(double2));
+  const size_t o_len = take(n.fib, sizeof(mfg::F64Len));
   std::vector<unsigned char> blob(bytes);
   parallel_for(b->R, [&](int r) {
     mfg::F64Parts& p = parts[r];
@@ -484,12 +485,12 @@ mfg_status plan_f64_clusters(mfg_batch* b, const std::vector<double>& m,
     mfg::F64Mass* mass = reinterpret_cast<mfg::F64Mass*>(&blob[o_mass]) + at[r].node;
     for (size_t t = 0; t < p.gnode.size(); ++t) {
       const int64_t i = d.node_off + p.gnode[t];
-      mass[t] = {m[i], m[nt + i], m[2 * nt + i]};
+      mass[t] = {m[i], mfg::bits_of(m[nt + i]), m[2 * nt + i]};
     }
-    double2* len = reinterpret_cast<double2*>(&blob[o_len]) + at[r].fib;
+    mfg::F64Len* len = reinterpret_cast<mfg::F64Len*>(&blob[o_len]) + at[r].fib;
     for (size_t e = 0; e < p.slot.size(); ++e) {
       const int64_t i = d.fiber_off + p.slot[e];
-      len[e] = make_double2(l0[i], l0[et + i]);
+      len[e] = {l0[i], mfg::bits_of(l0[et + i])};
     }
   });
   mfg_status st = upload(b->d_plan, blob, s);
@@ -498,6 +499,15 @@ mfg_status plan_f64_clusters(mfg_batch* b, const std::vector<double>& m,
   mfg::F64Plan& plan = b->f64_plan;
   plan.cl = cl;
   plan.smem_bytes = mfg::kF64ClusterSmem;
+  // the part that a fiber is in, on average over the fibers
+  double sum = 0.0, squares = 0.0;
+  for (const mfg::F64Parts& p : parts)
+    for (const mfg::F64Part& q : p.part) {
+      sum += q.n_fib;
+      squares += static_cast<double>(q.n_fib) * q.n_fib;
+    }
+  plan.threads = squares > mfg::kF64SmallParts * sum ? mfg::kF64ClusterThreads
+                                                     : mfg::kF64SmallThreads;
   const unsigned char* base = b->d_plan.p;
   plan.part = reinterpret_cast<const mfg::F64Part*>(base + o_part);
   plan.gnode = reinterpret_cast<const int32_t*>(base + o_gnode);
@@ -505,7 +515,7 @@ mfg_status plan_f64_clusters(mfg_batch* b, const std::vector<double>& m,
   plan.rows = reinterpret_cast<const int32_t*>(base + o_rows);
   plan.inc = reinterpret_cast<const int32_t*>(base + o_inc);
   plan.ends = reinterpret_cast<const int2*>(base + o_ends);
-  plan.len = reinterpret_cast<const double2*>(base + o_len);
+  plan.len = reinterpret_cast<const mfg::F64Len*>(base + o_len);
   int k = 0;
   while (1 << k < cl) ++k;
   b->f64_clusters = clusters[k];
@@ -696,6 +706,7 @@ static mfg_status batch_create_impl(const mfg_network* nets, const mfg_strategy*
     d.mode = st.mode;
     d.max_steps = st.mode == MFG_MODE_RAMP ? st.max_steps
                                            : (st.max_steps > 0 ? st.max_steps : MFG_DEFAULT_STEP_CAP);
+    d.r_steps = mfg::exact_reciprocal(d.max_steps);
     d.sound_speed = std::sqrt(rc.youngs_modulus / rc.density);  // TeamOuterLoop.h:72
     d.scale = nets[r].scale_factor;
     no += s.n_nodes;
@@ -714,7 +725,8 @@ static mfg_status batch_create_impl(const mfg_network* nets, const mfg_strategy*
   const int64_t nt = no, et = fo;
 
   // ---- pack ------------------------------------------------------------
-  // FP64 batches: 1 / m and m c follow the masses, 1 / l0 the lengths
+  // FP64 batches: the masses' reciprocals (exact_reciprocal) and m c follow
+  // the masses, the lengths' reciprocals the lengths
   const bool f64 = b->precision == MFG_PREC_F64;
   std::vector<double> X(3 * nt), m(f64 ? 3 * nt : nt), l0(f64 ? 2 * et : et);
   std::vector<int2> conn(et);
@@ -732,11 +744,11 @@ static mfg_status batch_create_impl(const mfg_network* nets, const mfg_strategy*
     std::memcpy(&inc[d.inc_off], s.inc.data(), 2 * s.n_fibers * sizeof(int32_t));
     if (f64) {
       for (int i = 0; i < N; ++i) {
-        m[nt + d.node_off + i] = mfg::exact_reciprocal(s.m[i]);
+        m[nt + d.node_off + i] = mfg::from_bits(mfg::exact_reciprocal(s.m[i]));
         m[2 * nt + d.node_off + i] = s.m[i] * d.c;
       }
       for (int e = 0; e < s.n_fibers; ++e)
-        l0[et + d.fiber_off + e] = mfg::exact_reciprocal(s.l0[e]);
+        l0[et + d.fiber_off + e] = mfg::from_bits(mfg::exact_reciprocal(s.l0[e]));
     }
     if (!s.bnd_order.empty())
       std::memcpy(&bnd[d.bnd_off], s.bnd_order.data(), s.bnd_order.size() * sizeof(int32_t));
@@ -796,11 +808,11 @@ static mfg_status batch_create_impl(const mfg_network* nets, const mfg_strategy*
   dv.u = b->d_u.p;
   dv.v = b->d_v.p;
   dv.m = b->d_m.p;
-  dv.rm = b->d_m.p + (f64 ? nt : 0);
+  dv.rm = reinterpret_cast<const uint64_t*>(b->d_m.p + (f64 ? nt : 0));
   dv.mc = b->d_m.p + (f64 ? 2 * nt : 0);
   dv.conn = b->d_conn.p;
   dv.l0 = b->d_l0.p;
-  dv.rl0 = b->d_l0.p + (f64 ? et : 0);
+  dv.rl0 = reinterpret_cast<const uint64_t*>(b->d_l0.p + (f64 ? et : 0));
   dv.nrm = b->d_nrm.p;
   dv.fint = b->d_fint.p;
   dv.rowptr = b->d_rowptr.p;

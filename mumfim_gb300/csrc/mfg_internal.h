@@ -39,7 +39,8 @@ struct RveDesc {
   int64_t row_off;    // first entry in the packed CSR row pointer array
   int64_t bnd_off;    // first boundary node in the packed boundary scratch
   int32_t n_nodes, n_free, n_fibers, law;
-  int32_t max_steps, mode, pad0, pad1;
+  int32_t max_steps, mode;
+  uint64_t r_steps;   // exact_reciprocal(max_steps), mfg_exact.cuh
   double E, A, B, lt;  // reaction 0: modulus, area, nonlinear B and transition ratio
   double c, crit, tol; // strategy
   double sound_speed;  // sqrt(E / rho)
@@ -57,11 +58,11 @@ struct DevBatch {
   double* u;         // 3 * nt displacement
   double* v;         // 3 * nt velocity
   const double* m;   // nt lumped mass
-  const double* rm;  // nt 1 / mass for div_known(), and mass times damping (FP64 batches)
+  const uint64_t* rm;  // nt exact_reciprocal(mass), and mass times damping (FP64 batches)
   const double* mc;
   const int2* conn;  // et fiber end nodes (RVE-local ids)
   const double* l0;  // et reference lengths
-  const double* rl0; // et 1 / length for div_known() (FP64 batches)
+  const uint64_t* rl0;  // et exact_reciprocal(length) (FP64 batches)
   double* nrm;       // 3 * et per-fiber force vectors (scratch)
   double* fint;      // 3 * nt internal force (boundary rows used by the stress)
   const int32_t* rowptr;  // per RVE n_nodes + 1 offsets into that RVE's incidences
@@ -84,18 +85,25 @@ struct F64Part {
   int64_t node_off, row_off, inc_off, fib_off;  // into the arrays below
 };
 struct F64Mass {
-  double m, rm, mc;  // mass, 1 / mass, mass times damping
+  double m;     // mass
+  uint64_t rm;  // exact_reciprocal(mass)
+  double mc;    // mass times damping
+};
+struct F64Len {
+  double l0;   // reference length
+  uint64_t r;  // exact_reciprocal(l0)
 };
 struct F64Plan {
   int cl;  // CTAs per cluster; 1: no plan, every RVE on one CTA
   int smem_bytes;
+  int threads;  // of a CTA: kF64ClusterThreads, or kF64SmallThreads for small parts
   const F64Part* part;
   const int32_t* gnode;
   const F64Mass* mass;   // by node
   const int32_t* rows;
   const int32_t* inc;
   const int2* ends;
-  const double2* len;    // by fiber: l0, 1 / l0
+  const F64Len* len;     // by fiber
 };
 
 struct RunArgs {
@@ -164,6 +172,8 @@ int relax_f64_max_blocks_per_sm(int threads);
 // The same solve with every RVE split over a cluster of plan.cl CTAs, `grid`
 // CTAs in all (mfg_relax_f64.cu, f64_parts in mfg_f64_order.h).
 constexpr int kF64ClusterSmem = 220 * 1024;
+constexpr int kF64ClusterThreads = 512, kF64SmallThreads = 256;
+constexpr double kF64SmallParts = 288;  // fibers of a small part, at most
 cudaError_t launch_relax_f64_cluster(const DevBatch& b, const RunArgs& a, const F64Plan& plan,
                                      int grid, cudaStream_t s);
 // Clusters of cl CTAs with smem_bytes of shared memory each that the device

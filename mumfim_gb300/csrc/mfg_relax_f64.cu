@@ -28,12 +28,14 @@
 //   fiber pass : l = |x2 - x1|; T = law(l0, l); nrm = (x2 - x1) * (T / l)
 // giving two block barriers per step.
 //
-// What bounds it: the FP64 pipe, 2 lanes per clock and SM (82 % busy over 304
-// RVEs of 4,500 nodes). The general divisions and square root, a second
-// quotient h f / m for the trailing kick and a minimum no step needed made
-// 84 FP64 instructions a fiber and step; the forms of mfg_exact.cuh and one
-// quotient for both kicks leave 52, the same bits. 256 RVEs of 4,500 nodes:
-// 4.3e9 -> 7.8e9 fiber-steps/s.
+// What bounds it: the FP64 pipe, one warp instruction in 19 cycles and SM, at
+// 84 FP64 instructions a fiber and step with the general divisions and square
+// root, a second quotient h f / m for the trailing kick and a minimum no step
+// needed. Quotients, square roots and half of a fiber's products run on the
+// integer units instead (mfg_exact.cuh), which idle otherwise: 24 FP64
+// instructions a fiber, the same bits; 512 threads at 64 registers, two CTAs
+// an SM, so that 32 warps keep both busy. 256 RVEs of 4,500 nodes: 4.4e9 ->
+// 1.6e10 fiber-steps/s.
 //
 // A batch that leaves SMs idle runs with every RVE split over a cluster of
 // 2 to 16 CTAs instead (relax_f64_cluster_kernel below).
@@ -55,7 +57,18 @@ namespace cg = cooperative_groups;
 namespace mfg {
 namespace {
 
-constexpr int kThreadsF64 = 256;
+constexpr int kThreadsF64 = 512;
+constexpr int kSumThreads = 256;  // partial sums of the residual
+// Which products run in integers: 1 the force vector's three, 2 also the
+// squares of the length, 3 also the linear law's, 4 also the nodes'. An FP64
+// product costs 19 cycles of the SM's pipe, an integer one 30 issue slots, so
+// it pays where warps are many. 304 RVEs of 4,500 nodes on single CTAs, levels
+// 0, 2, 3, 4: 1.20, 1.51, 1.54, 1.50e10 fiber-steps/s, but 1.08, 1.26, 1.20,
+// 1.18e10 for 152 (one CTA an SM); clusters of 512 threads, 36 RVEs, levels 1,
+// 2, 3, 4: 34, 28, 30, 31 us a step. A small part's warps are few, and a step
+// is a chain: 4.0 us with level 2 at 512 threads for one RVE of 1,000 nodes,
+// 3.7 with level 0 at 256.
+constexpr int kMulF64 = 2, kMulCluster = 2, kMulSmall = 0;
 
 // Reaction law of one RVE with everything that does not depend on the fiber
 // formed once, by the expressions the reference forms per fiber.
@@ -97,11 +110,23 @@ __device__ __forceinline__ LawF64 make_law_f64(const RveDesc& d) {
   return L;
 }
 
+// a b, in integers (mul_exact) when kInt.
+template <bool kInt>
+__device__ __forceinline__ double product(double a, double b) {
+  if constexpr (kInt)
+    return mul_exact(a, b);
+  else
+    return a * b;
+}
+
 // Force at length ratio lr of a fiber of reference length l0; alpha_l0 =
 // alpha / l0 (nonlinear law only).
+template <int kMul = 0>
 __device__ __forceinline__ double reaction_force(const LawF64& L, double lr, double l0,
                                                  double alpha_l0) {
-  if (!L.nonlinear) return lr * L.half_E * L.A * (lr * lr - 1);
+  if (!L.nonlinear)
+    return product<(kMul > 2)>(product<(kMul > 2)>(product<(kMul > 2)>(lr, L.half_E), L.A),
+                               product<(kMul > 2)>(lr, lr) - 1);
   if (lr > L.lt) return alpha_l0 * L.kt * (lr - L.lt) * l0 + L.bt;
   if (lr < 1.0) return alpha_l0 * L.kc * (lr - 1.0) * l0 + L.bc;
   const double gs = 1.0 / 2.0 * (lr * lr - 1);
@@ -121,32 +146,41 @@ __device__ __noinline__ double fiber_vector_general(const LawF64& L, const doubl
   return l;
 }
 
-// The same, with the square root and the three quotients of mfg_exact.cuh
-// (rl0 = RN(1 / l0), or 0 to ask for the general operations): 33 FP64
-// instructions on the linear law instead of 45, the same bits.
+// The same, with the square root and the quotients of mfg_exact.cuh (R0 =
+// exact_reciprocal(l0), 0 to ask for the general operations): 16 FP64
+// instructions on the linear law instead of 45 (10 with kMul = 2), the same
+// bits.
+template <int kMul>
 __device__ __forceinline__ double fiber_vector(const LawF64& L, const double d[3], double l0,
-                                               double rl0, double n[3]) {
-  const double s = d[0] * d[0] + d[1] * d[1] + d[2] * d[2];
-  double l, y;
-  sqrt_recip(s, rsqrt_start(s), l, y);
-  const double lr = div_known(l, l0, rl0);
-  const double T =
-      reaction_force(L, lr, l0, L.nonlinear ? div_known(L.alpha, l0, rl0) : 0.0);
-  if (L.exact && in_range(s) && hi_word(rl0) != 0 && !all_ones(l) && (in_range(T) || is_zero(T))) {
-    const double q = div_known(T, l, y);
-    n[0] = d[0] * q; n[1] = d[1] * q; n[2] = d[2] * q;
-    return l;
+                                               uint64_t R0, double n[3]) {
+  const double s = product<(kMul > 1)>(d[0], d[0]) + product<(kMul > 1)>(d[1], d[1]) +
+                   product<(kMul > 1)>(d[2], d[2]);
+  if (L.exact && in_range(s) && R0 != 0) {
+    double l;
+    uint64_t R;
+    if (sqrt_recip(s, rsqrt_start(root_operand(s)), l, R)) {
+      const double T = reaction_force<kMul>(L, div_known(l, l0, R0), l0,
+                                      L.nonlinear ? div_known(L.alpha, l0, R0) : 0.0);
+      const bool zero = is_zero(T);
+      if (zero || in_range(T)) {
+        const double q = zero ? T : div_root(T, l, R);
+#pragma unroll
+        for (int k = 0; k < 3; ++k) n[k] = product<(kMul > 0)>(d[k], q);
+        return l;
+      }
+    }
   }
   return fiber_vector_general(L, d, l0, n);
 }
 
-// x / m for a node's mass (rm = RN(1 / m), or 0): div_known() where it
-// applies. The general division is a call: inlined, the compiler runs it
-// ahead of the test on every node (12 FP64 instructions a fiber, measured).
+// x / m for a node's mass (R = exact_reciprocal(m), or 0): div_known() where
+// it applies. The general division is a call: inlined, the compiler runs it
+// ahead of the test on every node.
 __device__ __noinline__ double general_quotient(double x, double m) { return x / m; }
 
-__device__ __forceinline__ double over_mass(double x, double m, double rm) {
-  if ((in_range(x) && hi_word(rm) != 0) || is_zero(x)) return div_known(x, m, rm);
+__device__ __forceinline__ double over_mass(double x, double m, uint64_t R) {
+  if (is_zero(x)) return x;
+  if (in_range(x) && R != 0) return div_known(x, m, R);
   return general_quotient(x, m);
 }
 
@@ -158,9 +192,11 @@ __device__ __forceinline__ double flip_sign(double x, bool flip) {
 struct RveView {
   const double *X0, *X1, *X2;
   double *x0, *x1, *x2, *u0, *u1, *u2, *v0, *v1, *v2;
-  const double *m, *rm, *mc;
+  const double *m, *mc;
+  const uint64_t* rm;
   const int2* conn;
-  const double *l0, *rl0;
+  const double* l0;
+  const uint64_t* rl0;
   double *n0, *n1, *n2;
   double *fi0, *fi1, *fi2;
   const int32_t* rowptr;
@@ -222,7 +258,7 @@ __device__ __forceinline__ double fiber_pass(const RveView& r, const RveDesc& d,
     const int2 c = __ldg(r.conn + e);
     const double dv[3] = {r.x0[c.y] - r.x0[c.x], r.x1[c.y] - r.x1[c.x], r.x2[c.y] - r.x2[c.x]};
     double n[3];
-    const double l = fiber_vector(L, dv, __ldg(r.l0 + e), __ldg(r.rl0 + e), n);
+    const double l = fiber_vector<kMulF64>(L, dv, __ldg(r.l0 + e), __ldg(r.rl0 + e), n);
     if (kLen) lmin = fmin(lmin, l);
     r.n0[e] = n[0];
     r.n1[e] = n[1];
@@ -237,10 +273,11 @@ __device__ __forceinline__ double fiber_pass(const RveView& r, const RveDesc& d,
 // Between refreshes of the time step both half kicks add the same quotient
 // h f / m, formed once
 // (`same`).
-__device__ __forceinline__ void kick(double a, double m, double rm, double mc, double h_prev,
+template <int kMul>
+__device__ __forceinline__ void kick(double a, double m, uint64_t rm, double mc, double h_prev,
                                      double h, bool first, bool same, double& w) {
-  const double f = -(a + mc * w);  // f = -f_int - c m v
-  const double q = over_mass(h * f, m, rm);
+  const double f = -(a + product<(kMul > 3)>(mc, w));  // f = -f_int - c m v
+  const double q = over_mass(product<(kMul > 3)>(h, f), m, rm);
   if (!first) w += same ? q : over_mass(h_prev * f, m, rm);
   w += q;
 }
@@ -253,6 +290,7 @@ __device__ __forceinline__ void kick(double a, double m, double rm, double mc, d
 // Reads x and f_int past the L1 cache: other CTAs of a cluster wrote them.
 constexpr int kTerms = 128;
 
+template <int NT>
 __device__ void cauchy_stress(const DevBatch& b, const RunArgs& a, const RveDesc& d, int rve,
                               int status, int step, double residual, double* terms) {
   const int tid = threadIdx.x;
@@ -262,7 +300,7 @@ __device__ void cauchy_stress(const DevBatch& b, const RunArgs& a, const RveDesc
   double s = 0.0;
   for (int q0 = 0; q0 < nb; q0 += kTerms) {
     const int n = min(kTerms, nb - q0);
-    for (int t = tid; t < 6 * n; t += kThreadsF64) {
+    for (int t = tid; t < 6 * n; t += NT) {
       const int k = t / n, q = t - k * n;
       const int64_t i = no + bo[q0 + q];
       // component k: (i, j) index pair of the symmetric part x_i f_j
@@ -341,7 +379,7 @@ __device__ void solve_rve(const DevBatch& b, const RunArgs& a, int rve, double* 
   double h = d.crit * dt_crit * 0.5;  // TeamOuterLoop.h:345
   double h2 = 2 * h, h_prev = 0.0;
   double done = 0.0;  // (double)step, and the RAMP fraction's divisor
-  const double cap_d = static_cast<double>(cap), cap_rd = 1.0 / cap_d;
+  const double cap_d = static_cast<double>(cap);
   int status = 0;
   for (;;) {
     // `step` steps are complete. Every UPDATE_FREQ steps the residual of the
@@ -349,13 +387,17 @@ __device__ void solve_rve(const DevBatch& b, const RunArgs& a, int rve, double* 
     // condition is the reference's (TeamOuterLoop.h:371) plus the step cap.
     const bool res_step = step > 0 && ((step - 1) % kUpdateFreq) == 0;
     if (res_step) {
-      double part = 0.0;
+      // shares through global memory (f_int's first component, unused at free
+      // nodes), summed in the order of kSumThreads strided partial sums
       for (int i = tid; i < NF; i += kThreadsF64) {
         double a0, a1, a2;
         gather_fint(r, i, a0, a1, a2);
-        const double l0r = -a0, l1r = -a1, l2r = -a2;
-        part += l0r * l0r + l1r * l1r + l2r * l2r;
+        r.fi0[i] = a0 * a0 + a1 * a1 + a2 * a2;
       }
+      __syncthreads();
+      double part = 0.0;
+      if (tid < kSumThreads)
+        for (int i = tid; i < NF; i += kSumThreads) part += r.fi0[i];
       residual = sqrt(block_sum<kThreadsF64>(part, red));
       if (!isfinite(residual)) {
         status = 4;  // MFG_E_NONFINITE
@@ -369,18 +411,19 @@ __device__ void solve_rve(const DevBatch& b, const RunArgs& a, int rve, double* 
     for (int i = tid; i < NF; i += kThreadsF64) {
       double a0, a1, a2;
       gather_fint(r, i, a0, a1, a2);
-      const double mass = __ldg(r.m + i), rm = __ldg(r.rm + i), mc = __ldg(r.mc + i);
+      const double mass = __ldg(r.m + i), mc = __ldg(r.mc + i);
+      const uint64_t rm = __ldg(r.rm + i);
       double w0 = r.v0[i], w1 = r.v1[i], w2 = r.v2[i];
-      kick(a0, mass, rm, mc, h_prev, h, step == 0, same, w0);
-      kick(a1, mass, rm, mc, h_prev, h, step == 0, same, w1);
-      kick(a2, mass, rm, mc, h_prev, h, step == 0, same, w2);
+      kick<kMulF64>(a0, mass, rm, mc, h_prev, h, step == 0, same, w0);
+      kick<kMulF64>(a1, mass, rm, mc, h_prev, h, step == 0, same, w1);
+      kick<kMulF64>(a2, mass, rm, mc, h_prev, h, step == 0, same, w2);
       r.v0[i] = w0; r.v1[i] = w1; r.v2[i] = w2;
-      r.x0[i] = r.x0[i] + h2 * w0;
-      r.x1[i] = r.x1[i] + h2 * w1;
-      r.x2[i] = r.x2[i] + h2 * w2;
+      r.x0[i] = r.x0[i] + product<(kMulF64 > 3)>(h2, w0);
+      r.x1[i] = r.x1[i] + product<(kMulF64 > 3)>(h2, w1);
+      r.x2[i] = r.x2[i] + product<(kMulF64 > 3)>(h2, w2);
     }
     if (ramp) {
-      const double alpha = div_known(done + 1.0, cap_d, cap_rd);
+      const double alpha = div_known(done + 1.0, cap_d, d.r_steps);
       for (int i = NF + tid; i < N; i += kThreadsF64) {
         const double* rb = r.ramp + 6 * (i - NF);
         r.x0[i] = rb[0] + alpha * rb[3];
@@ -417,10 +460,10 @@ __device__ void solve_rve(const DevBatch& b, const RunArgs& a, int rve, double* 
     }
   }
   __syncthreads();
-  cauchy_stress(b, a, d, rve, status, step, residual, terms);
+  cauchy_stress<kThreadsF64>(b, a, d, rve, status, step, residual, terms);
 }
 
-__global__ void __launch_bounds__(kThreadsF64) relax_f64_kernel(const DevBatch b, const RunArgs a) {
+__global__ void __launch_bounds__(kThreadsF64, 2) relax_f64_kernel(const DevBatch b, const RunArgs a) {
   __shared__ double red[kThreadsF64 / 32 + 1];
   __shared__ double terms[6 * kTerms];
   __shared__ int s_rve;
@@ -437,7 +480,7 @@ __global__ void __launch_bounds__(kThreadsF64) relax_f64_kernel(const DevBatch b
   }
 }
 
-__global__ void __launch_bounds__(kThreadsF64) server_f64_kernel(const DevBatch b,
+__global__ void __launch_bounds__(kThreadsF64, 2) server_f64_kernel(const DevBatch b,
                                                                  const ServerArgs sa) {
   __shared__ double red[kThreadsF64 / 32 + 1];
   __shared__ double terms[6 * kTerms];
@@ -448,7 +491,8 @@ __global__ void __launch_bounds__(kThreadsF64) server_f64_kernel(const DevBatch 
 // ---- one RVE over a cluster of CTAs ------------------------------------------
 //
 // For batches that leave SMs idle. One CTA solves an RVE at the FP64 rate of
-// one SM: 42 us a step at 1,000 nodes with 151 SMs doing nothing. Here CL CTAs
+// one SM: 64 us a step at 1,000 nodes, as the kernel was, with 151 SMs doing
+// nothing; 3.7 us on 16. Here CL CTAs
 // on CL SMs share it (f64_parts): each keeps two copies of its nodes'
 // positions, their velocities and the force vectors of the fibers it
 // evaluates in shared memory and reads other CTAs' positions through
@@ -494,18 +538,18 @@ __device__ double cluster_min(double part, double* slot) {
 
 // Copies n items to the shared memory at `at` when they fit below `end`, and
 // returns where to read them.
-template <typename T>
+template <int NT, typename T>
 __device__ __forceinline__ const T* stage(const T* src, int n, unsigned char*& at,
                                           const unsigned char* end) {
   const size_t bytes = (static_cast<size_t>(n) * sizeof(T) + 15) & ~static_cast<size_t>(15);
   if (at + bytes > end) return src;
   T* dst = reinterpret_cast<T*>(at);
-  for (int k = threadIdx.x; k < n; k += kThreadsF64) dst[k] = src[k];
+  for (int k = threadIdx.x; k < n; k += NT) dst[k] = src[k];
   at += bytes;
   return dst;
 }
 
-template <int CL>
+template <int CL, int NT, int kMul>
 __device__ void solve_rve_cluster(const DevBatch& b, const RunArgs& a, const F64Plan& plan,
                                   int rve, double* red, double* cred, double* alpha_s,
                                   double* terms,
@@ -537,11 +581,11 @@ __device__ void solve_rve_cluster(const DevBatch& b, const RunArgs& a, const F64
     rbs = reinterpret_cast<double*>(at);
     at += 48 * nbo;
   }
-  const int2* ends = stage(plan.ends + part.fib_off, part.n_len, at, end);
-  const double2* len = stage(plan.len + part.fib_off, part.n_len, at, end);
-  const int32_t* rows = stage(plan.rows + part.row_off, nfo + 1, at, end);
-  const int32_t* inc = stage(plan.inc + part.inc_off, part.n_inc, at, end);
-  const F64Mass* mass = stage(plan.mass + part.node_off, nfo, at, end);
+  const int2* ends = stage<NT>(plan.ends + part.fib_off, part.n_len, at, end);
+  const F64Len* len = stage<NT>(plan.len + part.fib_off, part.n_len, at, end);
+  const int32_t* rows = stage<NT>(plan.rows + part.row_off, nfo + 1, at, end);
+  const int32_t* inc = stage<NT>(plan.inc + part.inc_off, part.n_inc, at, end);
+  const F64Mass* mass = stage<NT>(plan.mass + part.node_off, nfo, at, end);
   const int32_t* gnode = plan.gnode + part.node_off;
 
   const double* F = a.F + 9 * (a.n_F > 1 ? rve : 0);
@@ -551,7 +595,7 @@ __device__ void solve_rve_cluster(const DevBatch& b, const RunArgs& a, const F64
   if (a.update_coords && rank == 0 && tid == 0) b.vol[rve] = jacobian(Fm) * b.vol[rve];
 
   // ---- prologue, as solve_rve -------------------------------------------------
-  for (int t = tid; t < n_own; t += kThreadsF64) {
+  for (int t = tid; t < n_own; t += NT) {
     const int64_t gi = no + gnode[t];
     const int li = t < nfo ? t : part.fchunk + (t - nfo);
     const double xo0 = b.x[gi], xo1 = b.x[nt + gi], xo2 = b.x[2 * nt + gi];
@@ -587,14 +631,14 @@ __device__ void solve_rve_cluster(const DevBatch& b, const RunArgs& a, const F64
     constexpr bool kLen = decltype(want_len)::value;
     double lmin = DBL_MAX;
     const int n = kLen ? part.n_len : part.n_fib;
-    for (int e = tid; e < n; e += kThreadsF64) {
+    for (int e = tid; e < n; e += NT) {
       const int2 c = ends[e];
-      const double2 q = len[e];
+      const F64Len q = len[e];
       double xa[3], xb[3], nv[3];
       x.load(c.x, xa);
       x.load(c.y, xb);
       const double dv[3] = {xb[0] - xa[0], xb[1] - xa[1], xb[2] - xa[2]};
-      const double l = fiber_vector(L, dv, q.x, q.y, nv);
+      const double l = fiber_vector<kMul>(L, dv, q.l0, q.r, nv);
       if (kLen) {
         lmin = fmin(lmin, l);
         if (e >= part.n_fib) continue;
@@ -620,7 +664,7 @@ __device__ void solve_rve_cluster(const DevBatch& b, const RunArgs& a, const F64
   };
   cluster.sync();
   double dt_crit = cluster_min<CL>(
-                       block_min<kThreadsF64>(fiber_pass(std::true_type{}), red), cred) /
+                       block_min<NT>(fiber_pass(std::true_type{}), red), cred) /
                    d.sound_speed;
 
   // ---- main loop, as solve_rve --------------------------------------------------
@@ -636,9 +680,9 @@ __device__ void solve_rve_cluster(const DevBatch& b, const RunArgs& a, const F64
   double h2 = 2 * h, h_prev = 0.0;
   int status = 0;
   // RAMP fraction of the next step, kept by the last warp
-  const double cap_d = static_cast<double>(cap), cap_rd = 1.0 / cap_d;
+  const double cap_d = static_cast<double>(cap);
   double done = 1.0;
-  if (tid == kThreadsF64 - 1) *alpha_s = div_known(done, cap_d, cap_rd);
+  if (tid == NT - 1) *alpha_s = div_known(done, cap_d, d.r_steps);
   __syncthreads();
   for (;;) {
     const bool res_step = step > 0 && ((step - 1) % kUpdateFreq) == 0;
@@ -646,14 +690,15 @@ __device__ void solve_rve_cluster(const DevBatch& b, const RunArgs& a, const F64
       // the nodes' shares go through global memory (f_int's first component,
       // unused at free nodes) and every CTA sums all of them in the order of
       // solve_rve
-      for (int t = tid; t < nfo; t += kThreadsF64) {
+      for (int t = tid; t < nfo; t += NT) {
         const double f0 = gather(t, 0), f1 = gather(t, 1), f2 = gather(t, 2);
         b.fint[no + gnode[t]] = f0 * f0 + f1 * f1 + f2 * f2;
       }
       cluster.sync();
       double sum = 0.0;
-      for (int i = tid; i < NF; i += kThreadsF64) sum += __ldcg(b.fint + no + i);
-      residual = sqrt(block_sum<kThreadsF64>(sum, red));
+      if (tid < kSumThreads)
+        for (int i = tid; i < NF; i += kSumThreads) sum += __ldcg(b.fint + no + i);
+      residual = sqrt(block_sum<NT>(sum, red));
       if (!isfinite(residual)) {
         status = 4;  // MFG_E_NONFINITE
         break;
@@ -665,16 +710,16 @@ __device__ void solve_rve_cluster(const DevBatch& b, const RunArgs& a, const F64
     const double* xc = xs + 3 * S * cur;
     double* xn = xs + 3 * S * (1 - cur);
     const int n_items = 3 * W + (ramp ? 3 * nbo : 0);
-    for (int item = tid; item < n_items; item += kThreadsF64) {
+    for (int item = tid; item < n_items; item += NT) {
       if (item < 3 * W) {
         const int k = item < W ? 0 : (item < 2 * W ? 1 : 2);
         const int t = item - k * W;
         if (t < nfo) {
           const F64Mass mm = mass[t];
           double w = vel[k * nfo + t];
-          kick(gather(t, k), mm.m, mm.rm, mm.mc, h_prev, h, step == 0, same, w);
+          kick<kMul>(gather(t, k), mm.m, mm.rm, mm.mc, h_prev, h, step == 0, same, w);
           vel[k * nfo + t] = w;
-          xn[k * S + t] = xc[k * S + t] + h2 * w;
+          xn[k * S + t] = xc[k * S + t] + product<(kMul > 3)>(h2, w);
         }
       } else {
         const int q = item - 3 * W;
@@ -686,13 +731,13 @@ __device__ void solve_rve_cluster(const DevBatch& b, const RunArgs& a, const F64
     cur = 1 - cur;
     x.base = xs_addr + 24u * static_cast<uint32_t>(S) * static_cast<uint32_t>(cur);
     cluster.sync();
-    if (ramp && tid == kThreadsF64 - 1) {
+    if (ramp && tid == NT - 1) {
       done += 1.0;
-      *alpha_s = div_known(done, cap_d, cap_rd);
+      *alpha_s = div_known(done, cap_d, d.r_steps);
     }
     h_prev = h;
     if (step % kUpdateFreq == 0) {
-      dt_crit = cluster_min<CL>(block_min<kThreadsF64>(fiber_pass(std::true_type{}), red), cred) /
+      dt_crit = cluster_min<CL>(block_min<NT>(fiber_pass(std::true_type{}), red), cred) /
                 d.sound_speed;
       h = d.crit * dt_crit * 0.5;
       h2 = 2 * h;
@@ -706,7 +751,7 @@ __device__ void solve_rve_cluster(const DevBatch& b, const RunArgs& a, const F64
 
   // ---- FinalizeData: positions, u = x - X, boundary f_int, stress ------------------
   const double* xc = xs + 3 * S * cur;
-  for (int t = tid; t < n_own; t += kThreadsF64) {
+  for (int t = tid; t < n_own; t += NT) {
     const int64_t gi = no + gnode[t];
     const int li = t < nfo ? t : part.fchunk + (t - nfo);
 #pragma unroll
@@ -719,7 +764,7 @@ __device__ void solve_rve_cluster(const DevBatch& b, const RunArgs& a, const F64
   cluster.sync();
   // boundary rows from the positions just written (past the L1 cache): the
   // vectors of their fibers may be another CTA's
-  for (int q = tid; q < nbo; q += kThreadsF64) {
+  for (int q = tid; q < nbo; q += NT) {
     const int i = gnode[nfo + q];
     const int32_t* row = b.rowptr + d.row_off + i;
     double f[3] = {0.0, 0.0, 0.0};
@@ -731,7 +776,7 @@ __device__ void solve_rve_cluster(const DevBatch& b, const RunArgs& a, const F64
 #pragma unroll
       for (int k = 0; k < 3; ++k)
         dv[k] = __ldcg(b.x + k * nt + no + c.y) - __ldcg(b.x + k * nt + no + c.x);
-      fiber_vector(L, dv, b.l0[e], b.rl0[e], nv);
+      fiber_vector<0>(L, dv, b.l0[e], b.rl0[e], nv);
 #pragma unroll
       for (int k = 0; k < 3; ++k) f[k] = f[k] + flip_sign(nv[k], !(code & 1));
     }
@@ -739,14 +784,14 @@ __device__ void solve_rve_cluster(const DevBatch& b, const RunArgs& a, const F64
     for (int k = 0; k < 3; ++k) b.fint[k * nt + no + i] = f[k];
   }
   cluster.sync();
-  if (rank == 0) cauchy_stress(b, a, d, rve, status, step, residual, terms);
+  if (rank == 0) cauchy_stress<NT>(b, a, d, rve, status, step, residual, terms);
 }
 
-template <int CL>
-__global__ void __launch_bounds__(kThreadsF64, 1)
+template <int CL, int NT, int kMul>
+__global__ void __launch_bounds__(NT, 1)
 relax_f64_cluster_kernel(const DevBatch b, const RunArgs a, const F64Plan plan) {
   extern __shared__ double4 smem_f64[];
-  __shared__ double red[kThreadsF64 / 32 + 1];
+  __shared__ double red[NT / 32 + 1];
   __shared__ double terms[6 * kTerms];
   __shared__ double cred, alpha;
   __shared__ int s_rve;
@@ -760,39 +805,41 @@ relax_f64_cluster_kernel(const DevBatch b, const RunArgs a, const F64Plan plan) 
     const int rve = *cluster.map_shared_rank(&s_rve, 0);
     cluster.sync();  // also: no CTA overwrites what a slower one still reads
     if (rve < 0) break;
-    solve_rve_cluster<CL>(b, a, plan, rve, red, &cred, &alpha, terms,
+    solve_rve_cluster<CL, NT, kMul>(b, a, plan, rve, red, &cred, &alpha, terms,
                           reinterpret_cast<unsigned char*>(smem_f64), plan.smem_bytes);
   }
 }
 
-// Calls fn(std::integral_constant<int, CL>{}) for a cluster size of 2 to 16.
-template <class Fn>
-cudaError_t with_cluster(int cl, Fn&& fn) {
+using ClusterKernel = void (*)(DevBatch, RunArgs, F64Plan);
+
+template <int NT, int kMul>
+ClusterKernel cluster_kernel_of(int cl) {
   switch (cl) {
-    case 2: return fn(std::integral_constant<int, 2>{});
-    case 4: return fn(std::integral_constant<int, 4>{});
-    case 8: return fn(std::integral_constant<int, 8>{});
-    case 16: return fn(std::integral_constant<int, 16>{});
-    default: return cudaErrorInvalidValue;
+    case 2: return relax_f64_cluster_kernel<2, NT, kMul>;
+    case 4: return relax_f64_cluster_kernel<4, NT, kMul>;
+    case 8: return relax_f64_cluster_kernel<8, NT, kMul>;
+    case 16: return relax_f64_cluster_kernel<16, NT, kMul>;
+    default: return nullptr;
   }
 }
 
-template <int CL>
-cudaError_t cluster_config(int grid, int smem_bytes, cudaStream_t s, cudaLaunchConfig_t* cfg,
+cudaError_t cluster_config(int cl, int threads, int grid, int smem_bytes, cudaStream_t s,
+                           ClusterKernel* kernel, cudaLaunchConfig_t* cfg,
                            cudaLaunchAttribute* attr) {
-  cudaError_t e = cudaFuncSetAttribute(relax_f64_cluster_kernel<CL>,
-                                       cudaFuncAttributeMaxDynamicSharedMemorySize,
+  *kernel = threads == kF64ClusterThreads ? cluster_kernel_of<kF64ClusterThreads, kMulCluster>(cl)
+                                          : cluster_kernel_of<kF64SmallThreads, kMulSmall>(cl);
+  if (!*kernel) return cudaErrorInvalidValue;
+  cudaError_t e = cudaFuncSetAttribute(*kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                        kF64ClusterSmem);
-  if (e == cudaSuccess && CL > 8)
-    e = cudaFuncSetAttribute(relax_f64_cluster_kernel<CL>,
-                             cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+  if (e == cudaSuccess && cl > 8)
+    e = cudaFuncSetAttribute(*kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
   *cfg = {};
   cfg->gridDim = dim3(static_cast<unsigned>(grid), 1, 1);
-  cfg->blockDim = dim3(kThreadsF64, 1, 1);
+  cfg->blockDim = dim3(static_cast<unsigned>(threads), 1, 1);
   cfg->dynamicSmemBytes = static_cast<size_t>(smem_bytes);
   cfg->stream = s;
   attr[0].id = cudaLaunchAttributeClusterDimension;
-  attr[0].val.clusterDim.x = CL;
+  attr[0].val.clusterDim.x = static_cast<unsigned>(cl);
   attr[0].val.clusterDim.y = 1;
   attr[0].val.clusterDim.z = 1;
   cfg->attrs = attr;
@@ -804,15 +851,12 @@ cudaError_t cluster_config(int grid, int smem_bytes, cudaStream_t s, cudaLaunchC
 
 int relax_f64_max_clusters(int cl, int smem_bytes, int sms) {
   int n = 0;
-  const cudaError_t e = with_cluster(cl, [&](auto C) {
-    constexpr int CL = decltype(C)::value;
-    cudaLaunchAttribute attr[1];
-    cudaLaunchConfig_t cfg;
-    cudaError_t r = cluster_config<CL>(CL * sms, smem_bytes, nullptr, &cfg, attr);
-    if (r == cudaSuccess)
-      r = cudaOccupancyMaxActiveClusters(&n, relax_f64_cluster_kernel<CL>, &cfg);
-    return r;
-  });
+  ClusterKernel kernel = nullptr;
+  cudaLaunchAttribute attr[1];
+  cudaLaunchConfig_t cfg;
+  cudaError_t e =
+      cluster_config(cl, kF64ClusterThreads, cl * sms, smem_bytes, nullptr, &kernel, &cfg, attr);
+  if (e == cudaSuccess) e = cudaOccupancyMaxActiveClusters(&n, kernel, &cfg);
   if (e != cudaSuccess) {
     cudaGetLastError();  // an unsupported size is no failure of the caller's
     return 0;
@@ -822,14 +866,13 @@ int relax_f64_max_clusters(int cl, int smem_bytes, int sms) {
 
 cudaError_t launch_relax_f64_cluster(const DevBatch& b, const RunArgs& a, const F64Plan& plan,
                                      int grid, cudaStream_t s) {
-  return with_cluster(plan.cl, [&](auto C) {
-    constexpr int CL = decltype(C)::value;
-    cudaLaunchAttribute attr[1];
-    cudaLaunchConfig_t cfg;
-    cudaError_t e = cluster_config<CL>(grid, plan.smem_bytes, s, &cfg, attr);
-    if (e != cudaSuccess) return e;
-    return cudaLaunchKernelEx(&cfg, relax_f64_cluster_kernel<CL>, b, a, plan);
-  });
+  ClusterKernel kernel = nullptr;
+  cudaLaunchAttribute attr[1];
+  cudaLaunchConfig_t cfg;
+  const cudaError_t e =
+      cluster_config(plan.cl, plan.threads, grid, plan.smem_bytes, s, &kernel, &cfg, attr);
+  if (e != cudaSuccess) return e;
+  return cudaLaunchKernelEx(&cfg, kernel, b, a, plan);
 }
 
 cudaError_t launch_server_f64(const DevBatch& b, const ServerArgs& sa, int grid, cudaStream_t s) {
