@@ -54,6 +54,7 @@
 #include "mfg_internal.h"
 #include "mumfim_gpu.h"
 #include "mfg_mixed.h"
+#include "mfg_mixed_law.cuh"
 #include "mfg_mixed_order.h"
 
 namespace cg = cooperative_groups;
@@ -242,57 +243,6 @@ __global__ void mixed_prepare_sell_kernel(const MixedState ms, const int32_t* nc
     reinterpret_cast<int4*>(ms.nfc)[i] =
         make_int4(__float_as_int(fc.x), __float_as_int(fc.y), __float_as_int(fc.z), code >> 1);
   }
-}
-
-// Per-RVE constants of the fiber law in the T/l form used here.
-struct Law {
-  int nonlinear;
-  float ea;      // E A
-  float ea_b;    // alpha = E A / B (toe: T/l = alpha expm1(B g) / l0)
-  float B;
-  float lt;      // transition stretch
-  float Mt, bt;  // linear continuation T = Mt (lambda - lt) + bt above lt
-};
-
-__device__ __forceinline__ Law make_law(const RveDesc& d) {
-  Law L;
-  L.nonlinear = d.law == 1;
-  L.ea = static_cast<float>(d.E * d.A);
-  L.B = static_cast<float>(d.B);
-  L.lt = static_cast<float>(d.lt);
-  L.ea_b = 0.f;
-  L.Mt = 0.f;
-  L.bt = 0.f;
-  if (L.nonlinear) {
-    // FiberReactions.cc:16-71 with alpha = E A / B, g_t = (lt^2 - 1)/2:
-    //   m l0 = alpha ((1 + lt^2 B) e^{B g_t} - 1),  b = alpha lt (e^{B g_t} - 1)
-    const double alpha = d.E * d.A / d.B;
-    const double gt = 0.5 * (d.lt * d.lt - 1.0);
-    const double eg = exp(d.B * gt);
-    L.ea_b = static_cast<float>(alpha);
-    L.Mt = static_cast<float>(alpha * ((1.0 + d.lt * d.lt * d.B) * eg - 1.0));
-    L.bt = static_cast<float>(alpha * d.lt * (eg - 1.0));
-  }
-  return L;
-}
-
-// T / l of one fiber from its Green strain g and 1/l0.
-__device__ __forceinline__ float tension_over_length(const Law& L, float g, float rl0) {
-  if (!L.nonlinear) return L.ea * g * rl0;
-  const float lam2 = fmaf(2.f, g, 1.f);
-  if (g < 0.f) {
-    // below the compressive transition (ratio 1): T = E A (lambda - 1)
-    const float lam = sqrtf(fmaxf(lam2, 0.f));
-    const float lm1 = 2.f * g / (lam + 1.f);
-    return L.ea * lm1 * rl0 / lam;
-  }
-  const float lam = sqrtf(lam2);
-  if (lam > L.lt) {
-    const float T = fmaf(L.Mt, lam - L.lt, L.bt);
-    return T * rl0 / lam;
-  }
-  // toe: T = alpha lambda (e^{B g} - 1), so T / l = alpha (e^{B g} - 1) / l0
-  return L.ea_b * expm1f(L.B * g) * rl0;
 }
 
 // TwoSum accumulation of an increment into (hi, lo).
@@ -1801,17 +1751,19 @@ cudaError_t setup_kind(const MixedState& ms, int* clusters) {
 // Time of a step of one RVE in launch kind k, in microseconds: fitted to one
 // RVE of 500 to 20,000 nodes at every cluster size. Linear law, nodes: us on
 // 1, 2, 4, 8, 16 CTAs -- 1,000: 2.4, -, 2.3, 2.3, -; 4,500: 9.8, 6.0, 3.5,
-// 2.7, 2.6; 20,000: (100 in global memory), -, 13.1, 7.4, 4.6.
+// 2.7, 2.6; 20,000: (100 in global memory), -, 13.1, 7.4, 4.6. Nonlinear --
+// 1,000: 4.9, 4.3, 3.9, 3.7, -; 4,500: 16.9, 10.4, 6.3, 4.7, 4.7; 20,000: -, -,
+// 22, 12.8, 8.0.
 double step_us(const RveDesc& d, const BucketKind& k) {
   const bool nl = d.law == MFG_LAW_NONLINEAR;
-  if (k.all) return k.ng == 2 ? 0.0016 * d.n_fibers + 1.45 : 0.00115 * d.n_fibers + 2.0;
+  if (k.all) return k.ng == 2 ? 0.0014 * d.n_fibers + 1.5 : 0.0011 * d.n_fibers + 2.0;
   if (!k.nodal) return 0.002 * d.n_fibers;  // (part of) the state in global memory
   double fixed = k.cl == 1 ? 1.5 : k.cl == 2 ? 1.9 : k.cl == 4 ? 2.4 : k.cl == 8 ? 2.8 : 3.6;
   if (k.stage || (k.cl == 1 && k.db && d.n_nodes < 1350))
     fixed = k.cl == 1 ? 0.9 : k.cl == 2 ? 1.3 : k.cl == 4 ? 1.5 : k.cl == 8 ? 1.7 : 2.0;
   if (!k.db) fixed += 1.2;
   if (nl) fixed += 0.8;
-  const double per_fiber = nl ? (k.cl == 1 ? 0.0016 : 0.0022) : 0.00075;
+  const double per_fiber = nl ? (k.cl == 1 ? 0.0012 : 0.0015) : 0.00075;
   return per_fiber * d.n_fibers / k.cl + fixed;
 }
 
