@@ -7,6 +7,83 @@
 
 namespace mfg {
 
+namespace {
+
+// Order of the nodes inside each group of 8 consecutive positions of one
+// CTA's free nodes (`order`: storage ids by local position) that lessens the
+// shared-memory bank conflicts of the node-centric solve.
+//
+// A warp's 16-byte reads of the other ends' records are served 8 lanes at a
+// time, one pass for each record of a bank group (slot mod 8) beyond the
+// first. The 8 nodes of a group read their k-th other ends together; which
+// slot mod 8 a node has within its own group is free. Each set of records
+// read together counts its members by slot mod 8; group after group, the
+// nodes take the free place whose members are fewest over the sets they are
+// in. One sweep: 7.7 passes for a warp's 16-byte reads instead of 9.4 (4 without
+// conflicts), 4.8 for its 8-byte ones instead of 5.3 (2), at 0.1 us a node; a
+// second sweep gains 0.1 more.
+struct BankScratch {
+  std::vector<int32_t> place, first, fill, set;  // by node, by node, by node, by incidence
+  std::vector<uint64_t> count;
+};
+
+void spread_banks(int32_t* order, int n, int owner_lo, int owner_hi, const int2* conn,
+                  const int32_t* row, const int32_t* inc, BankScratch& w) {
+  if (n < 16) return;
+  int widest = 0, total = 0;
+  for (int t = 0; t < n; ++t) {
+    const int deg = row[order[t] + 1] - row[order[t]];
+    w.place[order[t] - owner_lo] = t;
+    widest = std::max(widest, deg);
+    total += deg;
+  }
+  // the sets that each node's record is in: the k-th other ends of the group
+  // of a neighbour of whose row it is the k-th; groups never change
+  w.first.assign(n + 1, 0);
+  w.set.resize(total);
+  for (int j = owner_lo; j < owner_hi; ++j)
+    w.first[j - owner_lo + 1] = w.first[j - owner_lo] + row[j + 1] - row[j];
+  std::vector<int32_t>& end = w.fill;
+  end.assign(w.first.begin(), w.first.end() - 1);
+  for (int i = owner_lo; i < owner_hi; ++i) {
+    const int base = (w.place[i - owner_lo] >> 3) * widest;
+    for (int p = row[i], k = 0; p < row[i + 1]; ++p, ++k) {
+      const int2 c = conn[inc[p] >> 1];
+      const int j = (inc[p] & 1) ? c.x : c.y;
+      if (j >= owner_lo && j < owner_hi) w.set[end[j - owner_lo]++] = base + k;
+    }
+  }
+  // count[set]: its members by slot mod 8, one byte each (at most 8)
+  w.count.assign(static_cast<size_t>((n + 7) / 8) * widest, 0);
+  auto add = [&](int j, uint64_t member) {
+    for (int q = w.first[j - owner_lo]; q < end[j - owner_lo]; ++q) w.count[w.set[q]] += member;
+  };
+  for (int t = 0; t < n; ++t) add(order[t], 1ull << (8 * (t & 7)));
+  for (int g = 0; g + 8 <= n; g += 8) {
+    int32_t node[8];
+    std::copy(order + g, order + g + 8, node);
+    for (int c = 0; c < 8; ++c) add(node[c], 0 - (1ull << (8 * c)));
+    unsigned taken = 0;
+    for (int m = 0; m < 8; ++m) {
+      // byte sums: a node in more than 31 sets may wrap, which only costs the
+      // quality of its place
+      uint64_t cost = 0;
+      const int j = node[m] - owner_lo;
+      for (int q = w.first[j]; q < end[j]; ++q) cost += w.count[w.set[q]];
+      int best = -1;
+      for (int c = 0; c < 8; ++c)
+        if (!(taken >> c & 1) &&
+            (best < 0 || (cost >> (8 * c) & 255) < (cost >> (8 * best) & 255)))
+          best = c;
+      taken |= 1u << best;
+      order[g + best] = node[m];
+      add(node[m], 1ull << (8 * best));
+    }
+  }
+}
+
+}  // namespace
+
 void cluster_order(const RveDesc& d, int cl, bool own_order, bool heavy_first,
                    const std::vector<int2>& conn,
                    const std::vector<int32_t>& rowptr, const std::vector<int32_t>& inc,
@@ -40,6 +117,9 @@ void cluster_order(const RveDesc& d, int cl, bool own_order, bool heavy_first,
   // nodes: position of each node (identity but for the free blocks)
   std::vector<int> pos(N);
   for (int j = 0; j < N; ++j) pos[j] = j;
+  std::vector<int32_t> ids(fchunk);
+  BankScratch banks;
+  banks.place.resize(fchunk);
   for (int o = 0; o < cl; ++o) {
     const int f_lo = std::min(NF, o * fchunk), f_hi = std::min(NF, f_lo + fchunk);
     std::vector<std::pair<int, int>> order;  // (group * 1024 + degree rank, node)
@@ -58,6 +138,13 @@ void cluster_order(const RveDesc& d, int cl, bool own_order, bool heavy_first,
                      [](const std::pair<int, int>& x, const std::pair<int, int>& y) {
                        return x.first < y.first;
                      });
+    if (heavy_first) {
+      for (size_t k = 0; k < order.size(); ++k) ids[k] = order[k].second;
+      spread_banks(ids.data(), f_hi - f_lo, f_lo, f_hi, conn.data() + fo, rowptr.data() + ro,
+                   inc.data() + io, banks);
+      for (size_t k = 0; k < order.size(); ++k) pos[ids[k]] = f_lo + static_cast<int>(k);
+      continue;
+    }
     int q = f_lo;
     for (const auto& kv : order) pos[kv.second] = q++;
   }
