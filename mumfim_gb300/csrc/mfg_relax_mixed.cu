@@ -66,7 +66,7 @@ namespace mfg {
 // arguments, and the run-time placement's global scratch. Context 0 serves
 // the batch's runs; contexts 1-6 the concurrent perturbed solves of the
 // material stiffness, which run at the same time on the same batch.
-constexpr int kMixedBuckets = 10;
+constexpr int kMixedBuckets = 11;
 constexpr int kMaxCluster = 16;
 struct MixedRunCtx {
   int32_t* queues = nullptr;  // one claim counter per bucket (device)
@@ -149,19 +149,19 @@ struct BucketKind {
   bool nodal;  // node-centric solve (node state in shared memory)
   int ng;      // RVEs solved side by side by one CTA (fiber-centric, all on chip)
   bool db;     // node-centric with two copies of the node records
-  bool stage;  // and the read-only data of the step in shared memory too (on one CTA with
-               // two copies: for the RVEs for which it fits)
+  bool stage;  // and the read-only data of the step in shared memory too
 };
 constexpr int kBuckets = kMixedBuckets;
 // Launch kinds: each bucket's own (the same index), then the wider clusters a
 // bucket may take when the batch leaves SMs idle (choose_kinds).
-constexpr int kKinds = 17;
+constexpr int kKinds = 18;
 constexpr BucketKind kKind[kKinds] = {
     {8, false, true, 1, false, false}, {4, false, true, 1, true, false},
     {4, false, true, 1, false, false}, {2, false, true, 1, true, false},
     {2, false, true, 1, false, false}, {1, false, true, 1, false, false},
     {1, false, true, 1, true, false},  {1, true, false, 1, false, false},
     {1, true, false, 2, false, false}, {1, false, false, 1, false, false},
+    {1, false, true, 1, true, true},
     // wider
     {8, false, true, 1, true, false},  {16, false, true, 1, true, false},
     {16, false, true, 1, false, false}, {2, false, true, 1, true, true},
@@ -170,12 +170,15 @@ constexpr BucketKind kKind[kKinds] = {
 constexpr const BucketKind* kBucket = kKind;
 // Placement preference (bucket_of): the first bucket whose shared memory
 // holds the RVE, else the run-time placement. At each cluster size two
-// copies of the node records come first where they fit.
-constexpr int kPref[] = {8, 7, 6, 5, 3, 4, 1, 2, 0};
+// copies of the node records come first where they fit, on one CTA with the
+// step's read-only data before without.
+constexpr int kPref[] = {8, 7, 10, 6, 5, 3, 4, 1, 2, 0};
 // The single-CTA buckets with an RVE order of their own, by kind.
-constexpr int kQNodal1 = 5, kQNodalDB = 6, kQFiberAll = 7, kQFiberPair = 8, kQRuntime = 9;
+constexpr int kQNodal1 = 5, kQNodalDB = 6, kQFiberAll = 7, kQFiberPair = 8, kQRuntime = 9,
+              kQNodalStage = 10;
 static_assert(kBucket[kQNodal1].cl == 1 && kBucket[kQNodal1].nodal, "bucket table");
 static_assert(kBucket[kQNodalDB].cl == 1 && kBucket[kQNodalDB].db, "bucket table");
+static_assert(kBucket[kQNodalStage].cl == 1 && kBucket[kQNodalStage].stage, "bucket table");
 static_assert(!kBucket[kQRuntime].all && !kBucket[kQRuntime].nodal, "bucket table");
 static_assert(kBucket[kQFiberAll].cl == 1 && kBucket[kQFiberAll].all, "bucket table");
 static_assert(kBucket[kQFiberPair].all && kBucket[kQFiberPair].ng == 2, "bucket table");
@@ -626,10 +629,13 @@ __device__ __forceinline__ void mixed_stress(const DevBatch& b, const RunArgs& a
     for (int j = 0; j < NG; ++j) acc[j] = 0.0;
     for (int q = tid, j = 0; q < nb; q += Group<NG>::kSize, j = (j + 1 == NG ? 0 : j + 1)) {
       const int i = bo[q];
-      const double t = k < 3 ? xi[i] * fi[i] : 0.5 * (xi[i] * fj[i] + xj[i] * fi[i]);
+      // every rounding written out: the kernels that compile this sum would
+      // each contract it in a way of their own
+      const double t = k < 3 ? __dmul_rn(xi[i], fi[i])
+                             : 0.5 * __fma_rn(xj[i], fi[i], __dmul_rn(xi[i], fj[i]));
 #pragma unroll
       for (int jj = 0; jj < NG; ++jj)
-        if (jj == j) acc[jj] += t;
+        if (jj == j) acc[jj] = __dadd_rn(acc[jj], t);
     }
     const double sk = group_sum<NG>(acc, red) * sc;
     bad = bad || !isfinite(sk);
@@ -664,13 +670,13 @@ __host__ __device__ inline int64_t cluster_floats(int n_nodes, int n_free, int n
 
 // First float of the staged read-only data behind two record copies and the
 // velocities (16-byte aligned), and whether it fits: 16 bytes per incidence
-// record, 16 per node (row and mass).
+// record, 16 per free node (row and mass), 24 per boundary node (RAMP).
 __host__ __device__ inline int64_t stage_offset(int64_t slots) {
   return (15 * slots + 3) & ~static_cast<int64_t>(3);
 }
-__host__ __device__ inline bool stage_fits(int64_t slots, int64_t n_free, int64_t n_rec,
-                                           int64_t smem_floats) {
-  return stage_offset(slots) + 4 * n_rec + 4 * n_free <= smem_floats;
+__host__ __device__ inline bool stage_fits(int64_t slots, int64_t n_free, int64_t n_bnd,
+                                           int64_t n_rec, int64_t smem_floats) {
+  return stage_offset(slots) + 4 * n_rec + 4 * n_free + 6 * n_bnd <= smem_floats;
 }
 
 // Prologue of a solve in FP64 for the CTA's own nodes: the affine predictor
@@ -731,14 +737,15 @@ __device__ __forceinline__ void mixed_prologue(const DevBatch& b, const MixedSta
   }
 }
 
-// RAMP mode: the own boundary nodes move by their exact (hi, lo) increment.
-template <int NG = 1>
-__device__ __forceinline__ void ramp_boundary(const Rve& r, const LocalNodes& own, int g_lo,
-                                              int g_hi, int fchunk, const LocalNodes* dst = nullptr) {
-  const int NF = r.d.n_free;
-  for (int i = g_lo + Group<NG>::tid(); i < g_hi; i += Group<NG>::kSize) {
-    const float* rb = r.ramp + 12 * (i - NF);
-    const int li = fchunk + (i - g_lo);
+// RAMP mode: the own boundary nodes move by their exact (hi, lo) increment,
+// kStride floats apart from `ramp` on. The last threads take them: the first
+// ones have the most free nodes.
+template <int NG = 1, int kStride = 12>
+__device__ __forceinline__ void ramp_boundary(const float* ramp, const LocalNodes& own, int n,
+                                              int fchunk, const LocalNodes* dst = nullptr) {
+  for (int q = Group<NG>::kSize - 1 - Group<NG>::tid(); q < n; q += Group<NG>::kSize) {
+    const float* rb = ramp + kStride * q;
+    const int li = fchunk + q;
     NodeRec nr = own.load(li);
 #pragma unroll
     for (int k = 0; k < 3; ++k) {
@@ -894,7 +901,7 @@ __device__ void solve_rve_mixed(const DevBatch& b, const MixedState& ms, const R
         i = in;
       }
     }
-    if (ramp) ramp_boundary<NG>(r, own, g_lo, g_hi, fchunk);
+    if (ramp) ramp_boundary<NG>(r.ramp + 12 * (g_lo - NF), own, g_hi - g_lo, fchunk);
     G::sync();
     const bool dt_step = (step % kUpdateFreq) == 0;
     if (dt_step) {
@@ -1151,6 +1158,7 @@ __device__ void solve_rve_nodal(const DevBatch& b, const MixedState& ms, const R
   const int2* own_row = srow + f_lo;
   const float2* mass = ms.mmass + no + f_lo;
   const int4* own_rec = rec;
+  float* ramp_s = nullptr;  // staged: the own boundary nodes' increments
   if constexpr (kStage) {
     const int2 part = ms.sell_cta[static_cast<int64_t>(rve) * kMaxCluster + rank];
     const int q0 = part.x, n_rec = part.y;
@@ -1166,6 +1174,7 @@ __device__ void solve_rve_nodal(const DevBatch& b, const MixedState& ms, const R
     own_rec = rec_s;
     own_row = row_s;
     mass = mass_s;
+    ramp_s = reinterpret_cast<float*>(mass_s + nfo);
   }
   const double* F = a.F + 9 * (a.n_F > 1 ? rve : 0);
   const bool ramp = d.mode == 1;
@@ -1174,6 +1183,13 @@ __device__ void solve_rve_nodal(const DevBatch& b, const MixedState& ms, const R
   for (int k = 0; k < 9; ++k) Fm[k] = F[k];
   if (a.update_coords && rank == 0 && tid == 0) b.vol[rve] = jacobian(Fm) * b.vol[rve];
   mixed_prologue<true>(b, ms, r, Fm, ramp, f_lo, g_lo, nfo, n_own, fchunk, own, vel);
+  if constexpr (kStage) {
+    if (ramp) {  // written by this CTA in the prologue
+      __syncthreads();
+      for (int q = tid; q < 6 * (g_hi - g_lo); q += kThreadsMixed)
+        ramp_s[q] = r.ramp[12 * (g_lo - NF + q / 6) + q % 6];
+    }
+  }
   Ops::sync();
   if constexpr (kDB) {
     // boundary records in the second copy too (RAMP moves them into it every
@@ -1242,7 +1258,12 @@ __device__ void solve_rve_nodal(const DevBatch& b, const MixedState& ms, const R
         own.put(t, nr);
       }
     }
-    if (ramp) ramp_boundary(r, own, g_lo, g_hi, fchunk, kDB ? &nxt : nullptr);
+    if (ramp) {
+      if constexpr (kStage)
+        ramp_boundary<1, 6>(ramp_s, own, g_hi - g_lo, fchunk, &nxt);
+      else
+        ramp_boundary(r.ramp + 12 * (g_lo - NF), own, g_hi - g_lo, fchunk, kDB ? &nxt : nullptr);
+    }
     Ops::sync();
     if constexpr (kDB) {
       const LocalNodes t = own;
@@ -1285,14 +1306,7 @@ __device__ void solve_rve_nodal(const DevBatch& b, const MixedState& ms, const R
   Ops::sync();
 }
 
-// Whether an RVE with two record copies on one CTA is solved with its
-// read-only data staged (up to about 1,400 nodes).
-__device__ __forceinline__ bool stages_one(const DevBatch& b, const MixedState& ms, int rve,
-                                           int smem_floats) {
-  const RveDesc& d = b.desc[rve];
-  return stage_fits(even_slots(d.n_nodes), d.n_free,
-                    ms.sell_cta[static_cast<int64_t>(rve) * kMaxCluster].y, smem_floats);
-}
+extern __shared__ float4 mixed_smem[];
 
 // Persistent relaxation over one size bucket: CTA (or cluster) after cluster
 // takes the next RVE of `order` (largest first) until the bucket is empty.
@@ -1300,14 +1314,14 @@ __device__ __forceinline__ bool stages_one(const DevBatch& b, const MixedState& 
 // in half of the shared memory, synchronised by its own named barrier.
 template <int CL, bool kAll, bool kNodal, int NG, bool kDB, bool kStage>
 __global__ void __launch_bounds__(kThreadsMixed, 1)
-relax_mixed_kernel(const DevBatch b, const MixedState ms, const RunArgs a, int smem_floats,
-                   const int32_t* order, int n_order, int32_t* queue) {
+relax_mixed_kernel(const __grid_constant__ DevBatch b, const __grid_constant__ MixedState ms,
+                   const __grid_constant__ RunArgs a, int smem_floats, const int32_t* order,
+                   int n_order, int32_t* queue) {
   static_assert(kNodal || CL == 1, "the fiber-centric solve runs on one CTA");
   static_assert(NG == 1 || (CL == 1 && kAll && !kNodal), "only small fiber-centric RVEs pair up");
   static_assert(!kDB || kNodal, "two record copies: node-centric solve");
   constexpr int kRed = kThreadsMixed / 32 + 1;
-  extern __shared__ float4 smem4[];
-  float* smem = reinterpret_cast<float*>(smem4);
+  float* smem = reinterpret_cast<float*>(mixed_smem);
   __shared__ double red[NG * kRed];
   __shared__ double cred[1];
   __shared__ int s_rve[NG];
@@ -1329,12 +1343,7 @@ relax_mixed_kernel(const DevBatch b, const MixedState ms, const RunArgs a, int s
       Group<NG>::sync();
     }
     if (rve < 0) break;
-    if constexpr (kNodal && CL == 1 && kDB && !kStage) {
-      if (stages_one(b, ms, rve, smem_floats))
-        solve_rve_nodal<1, true, true>(b, ms, a, rve, red, cred, smem);
-      else
-        solve_rve_nodal<1, true>(b, ms, a, rve, red, cred, smem);
-    } else if constexpr (kNodal)
+    if constexpr (kNodal)
       solve_rve_nodal<CL, kDB, kStage>(b, ms, a, rve, red, cred, smem);
     else
       solve_rve_mixed<kAll, NG>(b, ms, a, rve, red + g * kRed, smem + g * (smem_floats / NG),
@@ -1354,7 +1363,7 @@ __device__ __forceinline__ void serve_one_cta(const DevBatch& b, const MixedStat
   const int q = __ldg(ms.rve_bucket + rve);
   if (q == kQNodal1)
     solve_rve_nodal<1>(b, ms, a, rve, red, cred, smem);
-  else if (q == kQNodalDB)
+  else if (q == kQNodalDB || q == kQNodalStage)
     solve_rve_nodal<1, true>(b, ms, a, rve, red, cred, smem);
   else if (q == kQFiberAll || q == kQFiberPair)
     solve_rve_mixed<true>(b, ms, a, rve, red, smem, smem_floats);
@@ -1646,7 +1655,7 @@ bool holds(const BucketKind& k, const RveDesc& d, const int32_t* rowptr, int64_t
     return false;
   if (!k.stage) return true;
   const int nb = d.n_nodes - d.n_free, fchunk = (d.n_free + k.cl - 1) / k.cl;
-  return stage_fits(even_slots(fchunk + (nb + k.cl - 1) / k.cl), fchunk,
+  return stage_fits(even_slots(fchunk + (nb + k.cl - 1) / k.cl), fchunk, (nb + k.cl - 1) / k.cl,
                     stage_records(d, k.cl, rowptr), smem_floats);
 }
 
@@ -1702,10 +1711,11 @@ cudaError_t with_kind(int k, Fn&& fn) {
     case 14: return fn(std::integral_constant<int, 14>{});
     case 15: return fn(std::integral_constant<int, 15>{});
     case 16: return fn(std::integral_constant<int, 16>{});
+    case 17: return fn(std::integral_constant<int, 17>{});
     default: return cudaErrorInvalidValue;
   }
 }
-static_assert(kKinds == 17, "with_kind covers every launch kind");
+static_assert(kKinds == 18, "with_kind covers every launch kind");
 
 template <int CL, bool kAll>
 cudaLaunchConfig_t launch_config(const MixedState& ms, unsigned grid, cudaStream_t s,
@@ -1772,7 +1782,7 @@ double step_us(const RveDesc& d, const BucketKind& k) {
   if (k.all) return k.ng == 2 ? 0.0014 * d.n_fibers + 1.5 : 0.0011 * d.n_fibers + 2.0;
   if (!k.nodal) return 0.002 * d.n_fibers;  // (part of) the state in global memory
   double fixed = k.cl == 1 ? 1.5 : k.cl == 2 ? 1.9 : k.cl == 4 ? 2.4 : k.cl == 8 ? 2.8 : 3.6;
-  if (k.stage || (k.cl == 1 && k.db && d.n_nodes < 1350))
+  if (k.stage)
     fixed = k.cl == 1 ? 0.9 : k.cl == 2 ? 1.3 : k.cl == 4 ? 1.5 : k.cl == 8 ? 1.7 : 2.0;
   if (!k.db) fixed += 1.2;
   if (nl) fixed += 0.8;
@@ -2030,8 +2040,7 @@ cudaError_t mixed_create(MixedState& ms, const DevBatch& b, const std::vector<Rv
     // the incidence records of each CTA's free nodes
     std::vector<int2> sell_cta(desc.size() * kMaxCluster, make_int2(0, 0));
     for (size_t r = 0; r < desc.size(); ++r) {
-      const bool one = ms.bucket_kind[rve_q[r]] == kQNodalDB;
-      if (!kind_of(r).stage && !one) continue;
+      if (!kind_of(r).stage) continue;
       const RveDesc& d = desc[r];
       const int fchunk = (d.n_free + kind_of(r).cl - 1) / kind_of(r).cl;
       for (int P = 0; P < d.n_free; ++P) {
@@ -2041,8 +2050,8 @@ cudaError_t mixed_create(MixedState& ms, const DevBatch& b, const std::vector<Rv
         part.y = std::max(part.y, row.x + 32 * (row.y - 1) + 1 - part.x);
       }
       const int nb = d.n_nodes - d.n_free, cl = kind_of(r).cl;
-      for (int o = 0; o < cl && !one; ++o)  // stage_records() is an upper bound
-        if (!stage_fits(even_slots(fchunk + (nb + cl - 1) / cl), fchunk,
+      for (int o = 0; o < cl; ++o)  // stage_records() is an upper bound
+        if (!stage_fits(even_slots(fchunk + (nb + cl - 1) / cl), fchunk, (nb + cl - 1) / cl,
                         sell_cta[r * kMaxCluster + o].y, smem_floats))
           return cudaErrorInvalidValue;
     }
