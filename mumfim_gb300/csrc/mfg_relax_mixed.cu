@@ -44,6 +44,8 @@
 #include <algorithm>
 #include <cfloat>
 #include <cmath>
+#include <functional>
+#include <queue>
 #include <thread>
 #include <type_traits>
 #include <vector>
@@ -1771,29 +1773,34 @@ cudaError_t setup_kind(const MixedState& ms, int* clusters) {
 
 // ---- width of the size buckets ------------------------------------------------
 
-// Time of a step of one RVE in launch kind k, in microseconds: fitted to one
-// RVE of 500 to 20,000 nodes at every cluster size. Linear law, nodes: us on
-// 1, 2, 4, 8, 16 CTAs -- 1,000: 2.4, -, 2.3, 2.3, -; 4,500: 9.8, 6.0, 3.5,
-// 2.7, 2.6; 20,000: (100 in global memory), -, 13.1, 7.4, 4.6. Nonlinear --
-// 1,000: 4.9, 4.3, 3.9, 3.7, -; 4,500: 16.9, 10.4, 6.3, 4.7, 4.7; 20,000: -, -,
-// 22, 12.8, 8.0.
+// Time of a step of one RVE in launch kind k, in microseconds: fitted to
+// batches of 1 to 304 RVEs of one size at every cluster size, as they run side
+// by side. Linear law, nodes: us on 1, 2, 4, 8, 16 CTAs -- 1,000: 2.3, -, 2.4,
+// 2.4, -; 2,500: 6.3, 3.9, 2.8, 2.4, -; 4,500: 9.9, 5.9, 3.3, 2.6, 2.5; 9,000:
+// -, 11.5, 6.3, -, -; 20,000: (100 in global memory), -, 13, 7.0, 4.0.
+// Nonlinear -- 1,000: 4.9, 3.8, 3.9, 3.6, -; 4,500: 16, 9.5, 5.8, 4.5, 4.6;
+// 20,000: -, -, 21, 12, 7.4.
 double step_us(const RveDesc& d, const BucketKind& k) {
   const bool nl = d.law == MFG_LAW_NONLINEAR;
   if (k.all) return k.ng == 2 ? 0.0014 * d.n_fibers + 1.5 : 0.0011 * d.n_fibers + 2.0;
   if (!k.nodal) return 0.002 * d.n_fibers;  // (part of) the state in global memory
-  double fixed = k.cl == 1 ? 1.5 : k.cl == 2 ? 1.9 : k.cl == 4 ? 2.4 : k.cl == 8 ? 2.8 : 3.6;
-  if (k.stage)
-    fixed = k.cl == 1 ? 0.9 : k.cl == 2 ? 1.3 : k.cl == 4 ? 1.5 : k.cl == 8 ? 1.7 : 2.0;
-  if (!k.db) fixed += 1.2;
-  if (nl) fixed += 0.8;
-  const double per_fiber = nl ? (k.cl == 1 ? 0.0012 : 0.0015) : 0.00075;
-  return per_fiber * d.n_fibers / k.cl + fixed;
+  // barriers and the tail of a part, by cluster size (1, 2, 4, 8, 16): one
+  // copy of the node records, two, and two with the read-only data staged
+  constexpr double fixed[3][5] = {
+      {1.2, 2.8, 3.5, 3.5, 4.5}, {1.2, 2.4, 2.3, 2.3, 1.8}, {0.6, 1.4, 1.2, 1.45, 1.6}};
+  int log2_cl = 0;
+  while (1 << log2_cl < k.cl) ++log2_cl;
+  const double per_fiber = nl ? (k.cl == 1 ? 0.0013 : 0.0015) : 0.0008;
+  return per_fiber * d.n_fibers / k.cl + fixed[k.db + k.stage][log2_cl] + (nl ? 0.9 : 0.0);
 }
 
 // Time of `copies` solves of the batch with the buckets in these kinds: RVE
 // after RVE, bucket by bucket with the largest clusters first and the longest
-// first in a bucket, each onto the SMs that are free first. clusters[k] of a
-// kind run at once, so each takes that share of the SMs.
+// first in a bucket, each onto the SMs that are free first. No more than
+// clusters[k] of a kind run at once, whatever SMs are left beside them: 36 of
+// 4 CTAs and 15 of 8 on 152 SMs, which a share of whole SMs a cluster (5 and
+// 11) would take for 30 and 13 (36 RVEs of 19,500 nodes, then put on clusters
+// of 8 in three waves: 22.0 us a step, on 4 in one wave: 13.0).
 double batch_us(const std::vector<RveDesc>& desc, const std::vector<std::vector<int32_t>>& bucket,
                 const int* kind, const int* clusters, int sms, int copies) {
   std::vector<int> order;
@@ -1804,15 +1811,24 @@ double batch_us(const std::vector<RveDesc>& desc, const std::vector<std::vector<
   std::vector<double> sm(sms, 0.0);  // when each SM is free, ascending
   for (int q : order) {
     const BucketKind& k = kKind[kind[q]];
-    const int share = k.cl == 1 ? 1 : std::min(sms, (sms + clusters[kind[q]] - 1) / clusters[kind[q]]);
+    const int share = std::min(k.cl, sms);
+    const size_t most = static_cast<size_t>(std::max(clusters[kind[q]], 1));
+    std::priority_queue<double, std::vector<double>, std::greater<double>> ends;
     const size_t n = bucket[q].size() * copies;
     for (size_t i = 0; i < n; i += k.ng) {
       const RveDesc& d = desc[bucket[q][i / copies]];
       // two RVEs side by side on a CTA take 1.4 times as long as one there
       const double t = step_us(d, k) * d.max_steps * (i + 1 < n && k.ng == 2 ? 1.4 : 1.0);
-      const double done = sm[share - 1] + t;
-      sm.erase(sm.begin(), sm.begin() + share);
-      sm.insert(std::upper_bound(sm.begin(), sm.end(), done), share, done);
+      double start = sm[share - 1];
+      if (ends.size() == most) {  // one of the kind has to end first
+        start = std::max(start, ends.top());
+        ends.pop();
+      }
+      ends.push(start + t);
+      // the SMs that come free last before then, so that the others stay free
+      const auto hi = std::upper_bound(sm.begin(), sm.end(), start);
+      sm.erase(hi - share, hi);
+      sm.insert(std::upper_bound(sm.begin(), sm.end(), start + t), share, start + t);
     }
   }
   return sm.back();
