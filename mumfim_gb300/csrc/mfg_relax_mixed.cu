@@ -1892,6 +1892,78 @@ void choose_kinds(const std::vector<RveDesc>& desc,
   std::copy(best, best + kBuckets, kind);
 }
 
+// Serving layout: which of the RVEs that one CTA holds go to clusters of 4 all
+// the same. A wave of requests, one per RVE, ends with its longest chain, and
+// a single CTA takes two to three times as long for its RVE as a cluster, at
+// up to twice the SM time. Requests are taken in order, large ones first: the
+// wave's time is estimated so (clusters for the large, then CTA by CTA) for the
+// longest 0, 1, 2, 3, 4, 6, ... single-CTA RVEs moved, and the best is taken
+// where it saves a tenth. Two waves of 96 RVEs of 500 - 20,000 nodes, both laws,
+// 200 steps: 14.2 ms with every RVE on one CTA that fits one, 11.3 so; of 13
+// RVEs of 1,800 - 5,100 nodes, 344 steps: 10.5, 5.3; of 53 RVEs up to 2,200 nodes,
+// where nothing moves: 2.9, 2.9. Returns the bucket per RVE in rve_q.
+void serve_on_clusters(const std::vector<RveDesc>& desc, const std::vector<int32_t>& rowptr,
+                       int smem_floats, int clusters, std::vector<int>& rve_q) {
+  constexpr int kQCluster = 2, kQClusterDB = 1;
+  static_assert(kKind[kQCluster].cl == kClusterServe && kKind[kQClusterDB].cl == kClusterServe,
+                "bucket table");
+  const size_t n = rve_q.size();
+  // a wave that fills the CTAs several times over is better off on single ones
+  if (clusters < 1 || n > 4 * static_cast<size_t>(clusters) * kClusterServe) return;
+  std::vector<double> one(n), four(n);  // a request's time on one CTA and on a cluster
+  std::vector<int> movable;
+  for (size_t r = 0; r < n; ++r) {
+    int q = rve_q[r] == kQNodalStage ? kQNodalDB : rve_q[r];  // not staged there
+    one[r] = step_us(desc[r], kKind[q]) * desc[r].max_steps * (kKind[q].ng == 2 ? 1.3 : 1.0);
+    four[r] = step_us(desc[r], kKind[kQCluster]) * desc[r].max_steps;
+    if (kKind[q].cl == 1 && q != kQRuntime && four[r] < 0.8 * one[r] &&
+        holds(kKind[kQCluster], desc[r], rowptr.data() + desc[r].row_off, smem_floats))
+      movable.push_back(static_cast<int>(r));
+  }
+  std::stable_sort(movable.begin(), movable.end(), [&](int x, int y) { return one[x] > one[y]; });
+  using Heap = std::priority_queue<double, std::vector<double>, std::greater<double>>;
+  std::vector<char> moved(n, 0);
+  auto wave = [&] {
+    Heap by_cluster, by_cta;
+    for (int c = 0; c < clusters; ++c) by_cluster.push(0.0);
+    double end = 0.0;
+    for (size_t r = 0; r < n; ++r)
+      if (moved[r] || kKind[rve_q[r]].cl == kClusterServe) {
+        const double t = by_cluster.top() + four[r];
+        by_cluster.pop();
+        by_cluster.push(t);
+        end = std::max(end, t);
+      }
+    for (; !by_cluster.empty(); by_cluster.pop())
+      for (int k = 0; k < kClusterServe; ++k) by_cta.push(by_cluster.top());
+    for (size_t r = 0; r < n; ++r)
+      if (!moved[r] && kKind[rve_q[r]].cl != kClusterServe) {
+        const double t = by_cta.top() + one[r];
+        by_cta.pop();
+        by_cta.push(t);
+        end = std::max(end, t);
+      }
+    return end;
+  };
+  double best = 0.9 * wave();
+  size_t take = 0, m = 0;
+  while (m < movable.size()) {
+    const size_t next = std::min(movable.size(), m + 1 + m / 3);
+    for (; m < next; ++m) moved[movable[m]] = 1;
+    const double t = wave();
+    if (t < best) {
+      best = t;
+      take = m;
+    }
+  }
+  for (size_t k = 0; k < take; ++k) {
+    const int r = movable[k];
+    rve_q[r] = holds(kKind[kQClusterDB], desc[r], rowptr.data() + desc[r].row_off, smem_floats)
+                   ? kQClusterDB
+                   : kQCluster;
+  }
+}
+
 }  // namespace
 
 cudaError_t mixed_create(MixedState& ms, const DevBatch& b, const std::vector<RveDesc>& desc,
@@ -1925,11 +1997,12 @@ cudaError_t mixed_create(MixedState& ms, const DevBatch& b, const std::vector<Rv
   // size buckets, each in longest-processing-time order
   std::vector<std::vector<int32_t>> bucket(kBuckets);
   std::vector<int> rve_q(desc.size());
-  for (size_t r = 0; r < desc.size(); ++r) {
+  for (size_t r = 0; r < desc.size(); ++r)
     rve_q[r] = bucket_of(desc[r], rowptr.data() + desc[r].row_off, smem_floats,
                          std::min(max_cluster, 8), serving_layout, small_solve, rves_per_cta);
-    bucket[rve_q[r]].push_back(static_cast<int32_t>(r));
-  }
+  if (serving_layout && max_cluster >= kClusterServe && small_solve != MFG_SMALL_FIBER_CENTRIC)
+    serve_on_clusters(desc, rowptr, smem_floats, ms.server_grid / kClusterServe, rve_q);
+  for (size_t r = 0; r < desc.size(); ++r) bucket[rve_q[r]].push_back(static_cast<int32_t>(r));
   int clusters[kKinds] = {};
   for (int q = 0; q < kBuckets; ++q) {
     std::stable_sort(bucket[q].begin(), bucket[q].end(),
