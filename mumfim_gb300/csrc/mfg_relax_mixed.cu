@@ -152,11 +152,12 @@ struct BucketKind {
   int ng;      // RVEs solved side by side by one CTA (fiber-centric, all on chip)
   bool db;     // node-centric with two copies of the node records
   bool stage;  // and the read-only data of the step in shared memory too
+  bool split = false;  // and four lanes to a node of a nonlinear RVE (nodal_kick_split)
 };
 constexpr int kBuckets = kMixedBuckets;
 // Launch kinds: each bucket's own (the same index), then the wider clusters a
 // bucket may take when the batch leaves SMs idle (choose_kinds).
-constexpr int kKinds = 18;
+constexpr int kKinds = 21;
 constexpr BucketKind kKind[kKinds] = {
     {8, false, true, 1, false, false}, {4, false, true, 1, true, false},
     {4, false, true, 1, false, false}, {2, false, true, 1, true, false},
@@ -168,7 +169,8 @@ constexpr BucketKind kKind[kKinds] = {
     {8, false, true, 1, true, false},  {16, false, true, 1, true, false},
     {16, false, true, 1, false, false}, {2, false, true, 1, true, true},
     {4, false, true, 1, true, true},   {8, false, true, 1, true, true},
-    {16, false, true, 1, true, true}};
+    {16, false, true, 1, true, true}, {4, false, true, 1, true, true, true},
+    {8, false, true, 1, true, true, true}, {16, false, true, 1, true, true, true}};
 constexpr const BucketKind* kBucket = kKind;
 // Placement preference (bucket_of): the first bucket whose shared memory
 // holds the RVE, else the run-time placement. At each cluster size two
@@ -1083,6 +1085,72 @@ __device__ __forceinline__ double nodal_kick(const Law& L, const Nodes& u, const
   return part;
 }
 
+// Pass A with the drift on the nonlinear law for a CTA of at most kThreadsMixed
+// / 4 nodes, 4 lanes to a node: lane l of a warp computes the incidences sub,
+// sub + 4, ... of node l mod 8, sub = l / 8, and the node's lanes add a turn's
+// vectors one after the other in the row's order, so the sum is the same bits.
+// A small part's step is the chain of its longest row's incidences, each a read
+// of a record, then of the node it names (in another CTA's shared memory), then
+// the law (one nonlinear RVE on 16 CTAs, a step: 4,500 nodes 4.6 -> 3.5 us, 1,000
+// on 8 CTAs 3.6 -> 2.5). On the linear law, whose chain is short, the exchange
+// costs what it saves (4,500 nodes: 2.5 -> 2.9 us), and so it does with 2 lanes
+// to a node for up to kThreadsMixed / 2 nodes (nonlinear, 4,500 on 8: 4.5 -> 4.9).
+constexpr int kLanes = 4;
+constexpr int kSplitNodes = kThreadsMixed / kLanes;
+template <class Nodes>
+__device__ __forceinline__ void nodal_kick_split(const Law& law, const Nodes& u,
+                                                 const LocalNodes& own, float* vel,
+                                                 const int4* rec, const int2* srow,
+                                                 const float2* mass, int nfo, float hk, float c,
+                                                 const LocalNodes& nxt, float h2) {
+  constexpr int kNodes = 32 / kLanes;  // of a warp
+  const int lane = threadIdx.x & 31, node = lane & (kNodes - 1), sub = lane / kNodes;
+  const int t = (static_cast<int>(threadIdx.x) >> 5) * kNodes + node;
+  if (t - node >= nfo) return;  // the whole warp
+  const bool mine = t < nfo;
+  const int2 sr = mine ? srow[t] : make_int2(0, 0);
+  const NodeRec me = own.load(mine ? t : 0);
+  const int most = __reduce_max_sync(0xffffffffu, sr.y);
+  float a[3] = {0.f, 0.f, 0.f};
+  for (int k = 0; k < most; k += kLanes) {
+    float4 f = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (k + sub < sr.y) {
+      const int4 q = rec[sr.x + 32 * (k + sub)];
+      const float dx = __int_as_float(q.x), dy = __int_as_float(q.y), dz = __int_as_float(q.z);
+      const float4 fc = make_float4(dx, dy, dz, inv_length(dx, dy, dz));
+      float du[3];
+      disp_diff(u.load(q.w), me, du);
+      f = force_vec<1>(law, du, fc, green(du, fc));
+    }
+    __syncwarp();
+#pragma unroll
+    for (int j = 0; j < kLanes; ++j) {
+      const int from = j * kNodes + node;
+      const float x = __shfl_sync(0xffffffffu, f.x, from);
+      const float y = __shfl_sync(0xffffffffu, f.y, from);
+      const float z = __shfl_sync(0xffffffffu, f.z, from);
+      if (k + j < sr.y) {
+        a[0] = __fadd_rn(a[0], x);
+        a[1] = __fadd_rn(a[1], y);
+        a[2] = __fadd_rn(a[2], z);
+      }
+    }
+  }
+  if (!mine || sub != 0) return;
+  const float2 mm = mass[t];
+  const float mc = mm.y * c;
+  const float km = hk * mm.x;
+  NodeRec nr = me;
+#pragma unroll
+  for (int q = 0; q < 3; ++q) {
+    float w = vel[3 * t + q];
+    w = fmaf(km, -a[q] - mc * w, w);
+    vel[3 * t + q] = w;
+    comp_add(nr.hi[q], nr.lo[q], h2 * w);
+  }
+  nxt.put(t, nr);
+}
+
 // Shortest current length among fiber slots e_lo + tid, + kThreadsMixed, ...
 // < e_hi (the critical time step's input, every 100 steps).
 template <class Nodes>
@@ -1114,7 +1182,7 @@ __device__ __forceinline__ float length_pass(const Rve& r, const Nodes& u, int e
 // from L2 every step, one incidence after the other: small parts, whose step
 // is little more than that chain, and all parts of a cluster, whose barrier
 // drops the L1 cache.
-template <int CL, bool kDB = false, bool kStage = false>
+template <int CL, bool kDB = false, bool kStage = false, bool kSplit = false>
 __device__ void solve_rve_nodal(const DevBatch& b, const MixedState& ms, const RunArgs& a, int rve,
                                 double* red, double* cred, float* smem) {
   static_assert(kDB || !kStage, "one record copy is taken when two do not fit, let alone staging");
@@ -1228,14 +1296,19 @@ __device__ void solve_rve_nodal(const DevBatch& b, const MixedState& ms, const R
     // pass B is fused into it and writes the other copy; and compiled per law,
     // so that the choice is made once a step and not at every fiber (512 RVEs
     // of 500 - 20,000 nodes, 1,000 steps: 44.7 -> 43.5 ms)
-    const double part =
-        res_step ? nodal_kick<true, kDB, kStage>(r.L, u, own, vel, own_rec, own_row, mass, nfo, hk,
-                                                 c, &nxt, h2)
-        : r.L.nonlinear
-            ? nodal_kick<false, kDB, kStage, 1>(r.L, u, own, vel, own_rec, own_row, mass, nfo, hk,
-                                                c, &nxt, h2)
-            : nodal_kick<false, kDB, kStage, 0>(r.L, u, own, vel, own_rec, own_row, mass, nfo, hk,
-                                                c, &nxt, h2);
+    double part = 0.0;
+    if (res_step) {
+      part = nodal_kick<true, kDB, kStage>(r.L, u, own, vel, own_rec, own_row, mass, nfo, hk, c,
+                                           &nxt, h2);
+    } else if (kSplit && r.L.nonlinear && nfo <= kSplitNodes) {
+      nodal_kick_split(r.L, u, own, vel, own_rec, own_row, mass, nfo, hk, c, nxt, h2);
+    } else if (r.L.nonlinear) {
+      nodal_kick<false, kDB, kStage, 1>(r.L, u, own, vel, own_rec, own_row, mass, nfo, hk, c,
+                                        &nxt, h2);
+    } else {
+      nodal_kick<false, kDB, kStage, 0>(r.L, u, own, vel, own_rec, own_row, mass, nfo, hk, c,
+                                        &nxt, h2);
+    }
     if (res_step) {
       residual = sqrt(Ops::template combine<false>(block_sum<kThreadsMixed>(part, red), cred));
       // a break keeps the copy of the step's start: the drift is dropped
@@ -1314,7 +1387,7 @@ extern __shared__ float4 mixed_smem[];
 // takes the next RVE of `order` (largest first) until the bucket is empty.
 // With NG = 2 each half of the CTA is a group that takes RVEs on its own,
 // in half of the shared memory, synchronised by its own named barrier.
-template <int CL, bool kAll, bool kNodal, int NG, bool kDB, bool kStage>
+template <int CL, bool kAll, bool kNodal, int NG, bool kDB, bool kStage, bool kSplit>
 __global__ void __launch_bounds__(kThreadsMixed, 1)
 relax_mixed_kernel(const __grid_constant__ DevBatch b, const __grid_constant__ MixedState ms,
                    const __grid_constant__ RunArgs a, int smem_floats, const int32_t* order,
@@ -1346,7 +1419,7 @@ relax_mixed_kernel(const __grid_constant__ DevBatch b, const __grid_constant__ M
     }
     if (rve < 0) break;
     if constexpr (kNodal)
-      solve_rve_nodal<CL, kDB, kStage>(b, ms, a, rve, red, cred, smem);
+      solve_rve_nodal<CL, kDB, kStage, kSplit>(b, ms, a, rve, red, cred, smem);
     else
       solve_rve_mixed<kAll, NG>(b, ms, a, rve, red + g * kRed, smem + g * (smem_floats / NG),
                                 smem_floats / NG);
@@ -1714,10 +1787,13 @@ cudaError_t with_kind(int k, Fn&& fn) {
     case 15: return fn(std::integral_constant<int, 15>{});
     case 16: return fn(std::integral_constant<int, 16>{});
     case 17: return fn(std::integral_constant<int, 17>{});
+    case 18: return fn(std::integral_constant<int, 18>{});
+    case 19: return fn(std::integral_constant<int, 19>{});
+    case 20: return fn(std::integral_constant<int, 20>{});
     default: return cudaErrorInvalidValue;
   }
 }
-static_assert(kKinds == 18, "with_kind covers every launch kind");
+static_assert(kKinds == 21, "with_kind covers every launch kind");
 
 template <int CL, bool kAll>
 cudaLaunchConfig_t launch_config(const MixedState& ms, unsigned grid, cudaStream_t s,
@@ -1744,7 +1820,7 @@ cudaError_t launch_bucket(const MixedState& ms, int q, const DevBatch& b, const 
   cudaLaunchAttribute attr[1];
   cudaLaunchConfig_t cfg =
       launch_config<k.cl, k.all>(ms, static_cast<unsigned>(ms.bucket_grid[q]), s, attr);
-  return cudaLaunchKernelEx(&cfg, relax_mixed_kernel<k.cl, k.all, k.nodal, k.ng, k.db, k.stage>, b, ms, a,
+  return cudaLaunchKernelEx(&cfg, relax_mixed_kernel<k.cl, k.all, k.nodal, k.ng, k.db, k.stage, k.split>, b, ms, a,
                             static_cast<int>(ms.smem_bytes / sizeof(float)),
                             static_cast<const int32_t*>(ms.order + ms.bucket_off[q]), n, queue);
 }
@@ -1754,7 +1830,7 @@ cudaError_t launch_bucket(const MixedState& ms, int q, const DevBatch& b, const 
 template <int K>
 cudaError_t setup_kind(const MixedState& ms, int* clusters) {
   constexpr BucketKind k = kKind[K];
-  auto kernel = relax_mixed_kernel<k.cl, k.all, k.nodal, k.ng, k.db, k.stage>;
+  auto kernel = relax_mixed_kernel<k.cl, k.all, k.nodal, k.ng, k.db, k.stage, k.split>;
   cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                        ms.smem_bytes);
   if (e == cudaSuccess && k.cl > 8)
@@ -1778,7 +1854,7 @@ cudaError_t setup_kind(const MixedState& ms, int* clusters) {
 // by side. Linear law, nodes: us on 1, 2, 4, 8, 16 CTAs -- 1,000: 2.3, -, 2.4,
 // 2.4, -; 2,500: 6.3, 3.9, 2.8, 2.4, -; 4,500: 9.9, 5.9, 3.3, 2.6, 2.5; 9,000:
 // -, 11.5, 6.3, -, -; 20,000: (100 in global memory), -, 13, 7.0, 4.0.
-// Nonlinear -- 1,000: 4.9, 3.8, 3.9, 3.6, -; 4,500: 16, 9.5, 5.8, 4.5, 4.6;
+// Nonlinear -- 1,000: 4.9, 3.8, 2.9, 2.6, -; 4,500: 16, 9.6, 5.7, 4.5, 3.6;
 // 20,000: -, -, 21, 12, 7.4.
 double step_us(const RveDesc& d, const BucketKind& k) {
   const bool nl = d.law == MFG_LAW_NONLINEAR;
@@ -1790,6 +1866,8 @@ double step_us(const RveDesc& d, const BucketKind& k) {
       {1.2, 2.8, 3.5, 3.5, 4.5}, {1.2, 2.4, 2.3, 2.3, 1.8}, {0.6, 1.4, 1.2, 1.45, 1.6}};
   int log2_cl = 0;
   while (1 << log2_cl < k.cl) ++log2_cl;
+  const bool split = k.split && nl && d.n_free <= k.cl * kSplitNodes;
+  if (split) return 0.0019 * d.n_fibers / k.cl + 1.9;
   const double per_fiber = nl ? (k.cl == 1 ? 0.0013 : 0.0015) : 0.0008;
   return per_fiber * d.n_fibers / k.cl + fixed[k.db + k.stage][log2_cl] + (nl ? 0.9 : 0.0);
 }
@@ -1849,12 +1927,20 @@ void choose_kinds(const std::vector<RveDesc>& desc,
       if (!holds(kKind[k], desc[r], rowptr.data() + desc[r].row_off, smem_floats)) return false;
     return true;
   };
+  // four lanes to a node where the bucket has a nonlinear RVE whose parts are
+  // small enough: the kernel's linear steps are a tenth slower for it
+  auto splits = [&](int q, int cl) {
+    for (int32_t r : bucket[q])
+      if (desc[r].law == MFG_LAW_NONLINEAR && desc[r].n_free <= cl * kSplitNodes) return true;
+    return false;
+  };
   // the kind of cl CTAs for bucket q: staged, else two record copies, else one
   auto wider = [&](int q, int cl) {
-    for (int level = 2; level >= 0; --level)
+    for (int level = 3; level >= 0; --level)
       for (int k = 0; k < kKinds; ++k)
-        if (kKind[k].nodal && kKind[k].cl == cl && kKind[k].stage + kKind[k].db == level &&
-            clusters[k] > 0 && fits(q, k))
+        if (kKind[k].nodal && kKind[k].cl == cl &&
+            kKind[k].split + kKind[k].stage + kKind[k].db == level && clusters[k] > 0 &&
+            fits(q, k) && (!kKind[k].split || splits(q, cl)))
           return k;
     return -1;
   };
