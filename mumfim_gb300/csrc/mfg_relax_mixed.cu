@@ -1036,7 +1036,7 @@ __device__ __forceinline__ void nodal_force(const Law& L, const Nodes& u, const 
 // the node at once, x += 2 h v with the new v, into the other copy `nxt`:
 // the arithmetic of pass B, without its barrier.
 template <bool kRes, bool kFuse = false, bool kStage = false, int kLaw = -1, class Nodes>
-__device__ __forceinline__ double nodal_kick(const Law& L, const Nodes& u, const LocalNodes& own,
+__device__ __forceinline__ double nodal_kick(const Law& law, const Nodes& u, const LocalNodes& own,
                                              float* vel, const int4* rec,
                                              const int2* srow, const float2* mass, int nfo,
                                              float hk, float c, const LocalNodes* nxt = nullptr,
@@ -1044,6 +1044,7 @@ __device__ __forceinline__ double nodal_kick(const Law& L, const Nodes& u, const
   double part = 0.0;
   int t = threadIdx.x;
   if (t >= nfo) return part;
+  const Law L = law;  // in registers for the pass
   int2 sr = read_only<kStage>(srow + t);
   float2 mm = read_only<kStage>(mass + t);
   for (;;) {
@@ -1165,6 +1166,15 @@ __device__ __forceinline__ float length_pass(const Rve& r, const Nodes& u, int e
   return lmin;
 }
 
+// a where kFirst, else b.
+template <bool kFirst, class T>
+__device__ __forceinline__ const T& pick(const T& a, const T& b) {
+  if constexpr (kFirst)
+    return a;
+  else
+    return b;
+}
+
 // One RVE by one CTA or the CL CTAs of a cluster, node-centric; every CTA
 // keeps its own nodes' records and velocities in shared memory (the caller
 // guarantees 9 floats per node slot fit). Node ranges per CTA, the node
@@ -1190,7 +1200,17 @@ __device__ void solve_rve_nodal(const DevBatch& b, const MixedState& ms, const R
   Rve r;
   r.d = b.desc[rve];
   const RveDesc& d = r.d;
-  r.L = make_law(d);
+  // Staged, the law's constants and those of the residual steps stay in
+  // registers (read from shared memory, the kernels with split nodes spill: 1,000
+  // nonlinear nodes 2.6 -> 3.2 us a step); else they are read where they are
+  // needed, since the step itself fills the registers (192 nonlinear RVEs of
+  // 2,000 - 8,000 nodes 23.1 -> 22.6 ms, 512 RVEs of 500 - 20,000 43.0 -> 42.6).
+  __shared__ Law s_law;
+  if constexpr (kStage)
+    r.L = make_law(d);
+  else if (threadIdx.x == 0)
+    s_law = make_law(d);
+  const Law& law = pick<kStage>(r.L, s_law);
   const int N = d.n_nodes, NF = d.n_free, E = d.n_fibers;
   const int tid = threadIdx.x;
   const int64_t no = d.node_off, fo = d.fiber_off, nt = b.nt;
@@ -1267,13 +1287,21 @@ __device__ void solve_rve_nodal(const DevBatch& b, const MixedState& ms, const R
     for (int t = tid; t < g_hi - g_lo; t += kThreadsMixed)
       nxt.put(fchunk + t, own.load(fchunk + t));
   }
-  double dt_crit = Ops::template combine<true>(
-                       block_min<kThreadsMixed>(length_pass(r, u, e_lo, e_hi), red), cred) /
-                   d.sound_speed;
+  auto half_step = [&] {
+    const RveDesc& dr = pick<kStage>(d, b.desc[rve]);
+    Rve fibers;
+    fibers.conn = kStage ? r.conn : ms.econn + dr.fiber_off;
+    fibers.fcon = kStage ? r.fcon : ms.fconc + dr.fiber_off;
+    const double dt_crit = Ops::template combine<true>(
+                               block_min<kThreadsMixed>(length_pass(fibers, u, e_lo, e_hi), red),
+                               cred) /
+                           dr.sound_speed;
+    return static_cast<float>(dr.crit * dt_crit * 0.5);
+  };
 
   const int step_cap = d.max_steps;
   const float c = static_cast<float>(d.c);
-  float h_cur = static_cast<float>(d.crit * dt_crit * 0.5);
+  float h_cur = half_step();
   int step = 0;
   double residual = 10.0;
   float h_prev = 0.f;
@@ -1281,13 +1309,7 @@ __device__ void solve_rve_nodal(const DevBatch& b, const MixedState& ms, const R
   for (;;) {
     const bool res_step = step > 0 && ((step - 1) % kUpdateFreq) == 0;
     if (!res_step && step >= step_cap) break;
-    if (res_step) {
-      // the time step from the positions after the last drift
-      dt_crit = Ops::template combine<true>(
-                    block_min<kThreadsMixed>(length_pass(r, u, e_lo, e_hi), red), cred) /
-                d.sound_speed;
-      h_cur = static_cast<float>(d.crit * dt_crit * 0.5);
-    }
+    if (res_step) h_cur = half_step();  // from the positions after the last drift
     const float h = h_cur;
     const float hk = h_prev + h;  // trailing kick of step-1 + leading kick of step
     const float h2 = h + h;
@@ -1298,15 +1320,15 @@ __device__ void solve_rve_nodal(const DevBatch& b, const MixedState& ms, const R
     // of 500 - 20,000 nodes, 1,000 steps: 44.7 -> 43.5 ms)
     double part = 0.0;
     if (res_step) {
-      part = nodal_kick<true, kDB, kStage>(r.L, u, own, vel, own_rec, own_row, mass, nfo, hk, c,
+      part = nodal_kick<true, kDB, kStage>(law, u, own, vel, own_rec, own_row, mass, nfo, hk, c,
                                            &nxt, h2);
-    } else if (kSplit && r.L.nonlinear && nfo <= kSplitNodes) {
-      nodal_kick_split(r.L, u, own, vel, own_rec, own_row, mass, nfo, hk, c, nxt, h2);
-    } else if (r.L.nonlinear) {
-      nodal_kick<false, kDB, kStage, 1>(r.L, u, own, vel, own_rec, own_row, mass, nfo, hk, c,
+    } else if (kSplit && law.nonlinear && nfo <= kSplitNodes) {
+      nodal_kick_split(law, u, own, vel, own_rec, own_row, mass, nfo, hk, c, nxt, h2);
+    } else if (law.nonlinear) {
+      nodal_kick<false, kDB, kStage, 1>(law, u, own, vel, own_rec, own_row, mass, nfo, hk, c,
                                         &nxt, h2);
     } else {
-      nodal_kick<false, kDB, kStage, 0>(r.L, u, own, vel, own_rec, own_row, mass, nfo, hk, c,
+      nodal_kick<false, kDB, kStage, 0>(law, u, own, vel, own_rec, own_row, mass, nfo, hk, c,
                                         &nxt, h2);
     }
     if (res_step) {
@@ -1316,7 +1338,7 @@ __device__ void solve_rve_nodal(const DevBatch& b, const MixedState& ms, const R
         status = 4;
         break;
       }
-      if (!ramp && !(residual > d.tol)) break;
+      if (!ramp && !(residual > pick<kStage>(d, b.desc[rve]).tol)) break;
       if (step >= step_cap) break;
     } else if constexpr (!kDB) {
       Ops::sync();
@@ -1352,13 +1374,16 @@ __device__ void solve_rve_nodal(const DevBatch& b, const MixedState& ms, const R
     h_prev = h;
     ++step;
   }
-  if (status == 0 && !ramp && residual > d.tol) status = 3;
+  if (status == 0 && !ramp && residual > pick<kStage>(d, b.desc[rve]).tol) status = 3;
 
   // ---- finalize: FP64 positions, boundary f_int, stress ---------------------
+  const int64_t node_off = pick<kStage>(d, b.desc[rve]).node_off;
+  const int2* rows = ms.nsell + node_off;
+  const int4* recs = reinterpret_cast<const int4*>(ms.nfc + ms.sell_off[rve]);
   for (int t = tid; t < n_own; t += kThreadsMixed) {
     const int i = t < nfo ? f_lo + t : g_lo + (t - nfo);
     const int li = t < nfo ? t : fchunk + (t - nfo);
-    const int64_t gi = __ldg(ms.gnode + no + i);  // batch node index
+    const int64_t gi = __ldg(ms.gnode + node_off + i);  // batch node index
     const NodeRec nr = own.load(li);
 #pragma unroll
     for (int k = 0; k < 3; ++k) {
@@ -1368,12 +1393,12 @@ __device__ void solve_rve_nodal(const DevBatch& b, const MixedState& ms, const R
       if (a.update_coords) b.u[k * nt + gi] = xk - Xk;
     }
     if (i >= NF) {
-      const int2 sr = __ldg(srow + i);
+      const int2 sr = __ldg(rows + i);
       float a0, a1, a2;
-      nodal_force(r.L, u, rec, sr.x, sr.y, nr, a0, a1, a2);
-      b.fint[no + i] = a0;
-      b.fint[nt + no + i] = a1;
-      b.fint[2 * nt + no + i] = a2;
+      nodal_force(law, u, recs, sr.x, sr.y, nr, a0, a1, a2);
+      b.fint[node_off + i] = a0;
+      b.fint[nt + node_off + i] = a1;
+      b.fint[2 * nt + node_off + i] = a2;
     }
   }
   Ops::sync();
