@@ -105,9 +105,10 @@ typedef struct mfg_strategy {
   int32_t mode;                  /* mfg_mode */
 } mfg_strategy;
 
-/* Arithmetic of the solve. F64 is the plain kernel: IEEE FP64 with the
+/* Arithmetic of the solve. F64 is IEEE FP64 with the
  * reference's operation order and no contraction, bit-identical to a serial
- * CPU run of the same algorithm. MIXED runs fiber forces and the integrator in
+ * CPU run of the same algorithm (on one CTA per RVE, or on clusters of 2 to 16
+ * where the batch leaves SMs idle). MIXED runs fiber forces and the integrator in
  * FP32 on top of FP64 reference coordinates plus Kahan-compensated FP32
  * displacements, and keeps FP64 for the stress, the residual and dt. */
 typedef enum mfg_precision { MFG_PREC_F64 = 0, MFG_PREC_MIXED = 1 } mfg_precision;
@@ -117,12 +118,15 @@ typedef struct mfg_options {
   int32_t device;           /* CUDA device ordinal */
   int32_t threads_per_rve;  /* ignored: the CTA size is fixed per precision */
   int32_t max_cluster_ctas; /* mixed precision: largest thread-block cluster an RVE
-                               may be split over (1, 2, 4 or 8; 0 = 8). 1 solves
-                               every RVE on one CTA, with the same results. */
-  int32_t cluster_layout;   /* mixed precision: mfg_cluster_layout. MFG_LAYOUT_SERVING
-                               places RVEs that need a cluster on clusters of 4
-                               (never 2), the size the serving kernel solves in
-                               clusters; the results are the same either way. */
+                               may be split over (1, 2, 4 or 8; 0 = as many as pay,
+                               up to 16). 1 solves every RVE on one CTA, with the
+                               same results. */
+  int32_t cluster_layout;   /* mfg_cluster_layout. Mixed precision: MFG_LAYOUT_SERVING
+                               places RVEs that need a cluster, and those that end a
+                               wave of requests sooner there, on clusters of 4 (never
+                               2), the size the serving kernel solves in clusters.
+                               FP64: MFG_LAYOUT_SERVING keeps every RVE on one CTA.
+                               The results are the same either way. */
   int32_t stiffness;        /* mfg_stiffness_solves: how mfg_batch_material_stiffness()
                                runs its six perturbed solves */
   int32_t small_rves_per_cta; /* mixed precision, MFG_SMALL_FIBER_CENTRIC only: how many

@@ -118,11 +118,13 @@ class BatchedFiberRVEAnalysisExplicit:
 
     networks    sequence of network_io.FiberNetwork (reaction 0 drives the solve)
     strategies  one strategy.SolutionStrategy per network
-    precision   "f64" (plain kernel, bit-identical to a serial CPU run) or "mixed"
+    precision   "f64" (bit-identical to a serial CPU run) or "mixed"
     max_cluster_ctas  mixed precision: largest thread-block cluster an RVE may be
-                split over (1, 2, 4 or 8; 0 = 8); results do not depend on it
-    serving_layout  mixed precision: RVEs that need a cluster get clusters of 4
-                (never 2), the layout the serving kernel uses; same results
+                split over (1, 2, 4 or 8; 0 = as many as pay, up to 16); results do
+                not depend on it
+    serving_layout  the layout the serving kernel uses. Mixed precision: RVEs that
+                need a cluster, or end a wave of requests sooner on one, get clusters
+                of 4 (never 2). FP64: one CTA per RVE. Same results
     stiffness   "auto", "sequential" or "concurrent": how computeMaterialStiffness
                 runs its six perturbed solves (mfg_stiffness_solves in
                 include/mumfim_gpu.h)

@@ -30,17 +30,19 @@
 //
 // Placement: one CTA of 1024 threads per SM with 220 KB of dynamic shared
 // memory, in size buckets launched concurrently. RVEs run node-centric on
-// one CTA or on the 2, 4 or 8 CTAs of a thread-block cluster, each CTA
+// one CTA or on the 2 to 16 CTAs of a thread-block cluster, each CTA
 // keeping its nodes' records (hi, lo) and velocities in shared memory and
 // reading other CTAs' through distributed shared memory; where a second copy
 // of the records fits at that size, the drift fuses into the kick and a
-// step has one barrier instead of two. On the nonlinear law, or on request,
+// step has one barrier instead of two. A batch that leaves SMs idle takes
+// wider clusters than its RVEs need, whose small parts keep the step's
+// read-only data in shared memory too. On the nonlinear law, or on request,
 // RVEs whose whole state fits one CTA's shared memory (or half of it, two
 // per CTA) run fiber-centric instead.
 // Those RVEs get their own fiber and node order (cluster_order) that keeps
-// most loads local and the warps' work even. RVEs too large for a cluster of
-// 8 run fiber-centric on one CTA, placed by size at run time down to global
-// memory.
+// most loads local and the warps' work even. RVEs too large for the largest
+// cluster run fiber-centric on one CTA, placed by size at run time down to
+// global memory.
 #include <algorithm>
 #include <cfloat>
 #include <cmath>
