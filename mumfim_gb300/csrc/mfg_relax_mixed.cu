@@ -146,6 +146,9 @@ namespace {
 
 constexpr int kThreadsMixed = 1024;
 constexpr int kSmemBytesMixed = 220 * 1024;
+// Four lanes to a node: of the nonlinear RVEs of a bucket, or of every RVE of
+// a bucket that is all linear and all in small parts.
+enum { kSplitNone, kSplitNonlinear, kSplitLinear };
 // How the RVEs of a size bucket are solved.
 struct BucketKind {
   int cl;      // CTAs per cluster
@@ -154,12 +157,12 @@ struct BucketKind {
   int ng;      // RVEs solved side by side by one CTA (fiber-centric, all on chip)
   bool db;     // node-centric with two copies of the node records
   bool stage;  // and the read-only data of the step in shared memory too
-  bool split = false;  // and four lanes to a node of a nonlinear RVE (nodal_kick_split)
+  int split = kSplitNone;  // and four lanes to a node (nodal_kick_split)
 };
 constexpr int kBuckets = kMixedBuckets;
 // Launch kinds: each bucket's own (the same index), then the wider clusters a
 // bucket may take when the batch leaves SMs idle (choose_kinds).
-constexpr int kKinds = 21;
+constexpr int kKinds = 24;
 constexpr BucketKind kKind[kKinds] = {
     {8, false, true, 1, false, false}, {4, false, true, 1, true, false},
     {4, false, true, 1, false, false}, {2, false, true, 1, true, false},
@@ -171,8 +174,13 @@ constexpr BucketKind kKind[kKinds] = {
     {8, false, true, 1, true, false},  {16, false, true, 1, true, false},
     {16, false, true, 1, false, false}, {2, false, true, 1, true, true},
     {4, false, true, 1, true, true},   {8, false, true, 1, true, true},
-    {16, false, true, 1, true, true}, {4, false, true, 1, true, true, true},
-    {8, false, true, 1, true, true, true}, {16, false, true, 1, true, true, true}};
+    {16, false, true, 1, true, true},
+    {4, false, true, 1, true, true, kSplitNonlinear},
+    {8, false, true, 1, true, true, kSplitNonlinear},
+    {16, false, true, 1, true, true, kSplitNonlinear},
+    {4, false, true, 1, true, true, kSplitLinear},
+    {8, false, true, 1, true, true, kSplitLinear},
+    {16, false, true, 1, true, true, kSplitLinear}};
 constexpr const BucketKind* kBucket = kKind;
 // Placement preference (bucket_of): the first bucket whose shared memory
 // holds the RVE, else the run-time placement. At each cluster size two
@@ -1088,19 +1096,21 @@ __device__ __forceinline__ double nodal_kick(const Law& law, const Nodes& u, con
   return part;
 }
 
-// Pass A with the drift on the nonlinear law for a CTA of at most kThreadsMixed
-// / 4 nodes, 4 lanes to a node: lane l of a warp computes the incidences sub,
-// sub + 4, ... of node l mod 8, sub = l / 8, and the node's lanes add a turn's
-// vectors one after the other in the row's order, so the sum is the same bits.
-// A small part's step is the chain of its longest row's incidences, each a read
-// of a record, then of the node it names (in another CTA's shared memory), then
-// the law (one nonlinear RVE on 16 CTAs, a step: 4,500 nodes 4.6 -> 3.5 us, 1,000
-// on 8 CTAs 3.6 -> 2.5). On the linear law, whose chain is short, the exchange
-// costs what it saves (4,500 nodes: 2.5 -> 2.9 us), and so it does with 2 lanes
-// to a node for up to kThreadsMixed / 2 nodes (nonlinear, 4,500 on 8: 4.5 -> 4.9).
+// Pass A with the drift for a CTA of at most kThreadsMixed / 4 nodes, 4 lanes to
+// a node: lane l of a warp computes the incidences sub, sub + 4, ... of node l
+// mod 8, sub = l / 8, and the node's lanes add a turn's vectors one after the
+// other in the row's order, so the sum is the same bits. A small part's step is
+// the chain of its longest row's incidences, each a read of a record, then of
+// the node it names (in another CTA's shared memory), then the law. One RVE, a
+// step: nonlinear, 4,500 nodes on 16 CTAs 4.6 -> 3.5 us, 1,000 on 8 3.6 -> 2.6;
+// linear, 4,500 on 16 2.5 -> 2.3, 2,500 on 16 2.4 -> 2.0, 1,000 on 4 2.3 -> 2.0. The
+// linear ones only in a kernel without the other passes: spills are read from
+// L2 after each cluster barrier, and beside them cost more than is gained
+// (2.5 -> 2.9). Two lanes to a node for up to kThreadsMixed / 2 nodes lose
+// (nonlinear, 4,500 on 8: 4.5 -> 4.9).
 constexpr int kLanes = 4;
 constexpr int kSplitNodes = kThreadsMixed / kLanes;
-template <class Nodes>
+template <int kLaw, class Nodes>
 __device__ __forceinline__ void nodal_kick_split(const Law& law, const Nodes& u,
                                                  const LocalNodes& own, float* vel,
                                                  const int4* rec, const int2* srow,
@@ -1123,7 +1133,7 @@ __device__ __forceinline__ void nodal_kick_split(const Law& law, const Nodes& u,
       const float4 fc = make_float4(dx, dy, dz, inv_length(dx, dy, dz));
       float du[3];
       disp_diff(u.load(q.w), me, du);
-      f = force_vec<1>(law, du, fc, green(du, fc));
+      f = force_vec<kLaw>(law, du, fc, green(du, fc));
     }
     __syncwarp();
 #pragma unroll
@@ -1194,7 +1204,7 @@ __device__ __forceinline__ const T& pick(const T& a, const T& b) {
 // from L2 every step, one incidence after the other: small parts, whose step
 // is little more than that chain, and all parts of a cluster, whose barrier
 // drops the L1 cache.
-template <int CL, bool kDB = false, bool kStage = false, bool kSplit = false>
+template <int CL, bool kDB = false, bool kStage = false, int kSplit = kSplitNone>
 __device__ void solve_rve_nodal(const DevBatch& b, const MixedState& ms, const RunArgs& a, int rve,
                                 double* red, double* cred, float* smem) {
   static_assert(kDB || !kStage, "one record copy is taken when two do not fit, let alone staging");
@@ -1322,10 +1332,12 @@ __device__ void solve_rve_nodal(const DevBatch& b, const MixedState& ms, const R
     // of 500 - 20,000 nodes, 1,000 steps: 44.7 -> 43.5 ms)
     double part = 0.0;
     if (res_step) {
-      part = nodal_kick<true, kDB, kStage>(law, u, own, vel, own_rec, own_row, mass, nfo, hk, c,
-                                           &nxt, h2);
-    } else if (kSplit && law.nonlinear && nfo <= kSplitNodes) {
-      nodal_kick_split(law, u, own, vel, own_rec, own_row, mass, nfo, hk, c, nxt, h2);
+      part = nodal_kick<true, kDB, kStage, kSplit == kSplitLinear ? 0 : -1>(
+          law, u, own, vel, own_rec, own_row, mass, nfo, hk, c, &nxt, h2);
+    } else if constexpr (kSplit == kSplitLinear) {
+      nodal_kick_split<0>(law, u, own, vel, own_rec, own_row, mass, nfo, hk, c, nxt, h2);
+    } else if (kSplit == kSplitNonlinear && law.nonlinear && nfo <= kSplitNodes) {
+      nodal_kick_split<1>(law, u, own, vel, own_rec, own_row, mass, nfo, hk, c, nxt, h2);
     } else if (law.nonlinear) {
       nodal_kick<false, kDB, kStage, 1>(law, u, own, vel, own_rec, own_row, mass, nfo, hk, c,
                                         &nxt, h2);
@@ -1397,7 +1409,7 @@ __device__ void solve_rve_nodal(const DevBatch& b, const MixedState& ms, const R
     if (i >= NF) {
       const int2 sr = __ldg(rows + i);
       float a0, a1, a2;
-      nodal_force(law, u, recs, sr.x, sr.y, nr, a0, a1, a2);
+      nodal_force<false, kSplit == kSplitLinear ? 0 : -1>(law, u, recs, sr.x, sr.y, nr, a0, a1, a2);
       b.fint[node_off + i] = a0;
       b.fint[nt + node_off + i] = a1;
       b.fint[2 * nt + node_off + i] = a2;
@@ -1414,7 +1426,7 @@ extern __shared__ float4 mixed_smem[];
 // takes the next RVE of `order` (largest first) until the bucket is empty.
 // With NG = 2 each half of the CTA is a group that takes RVEs on its own,
 // in half of the shared memory, synchronised by its own named barrier.
-template <int CL, bool kAll, bool kNodal, int NG, bool kDB, bool kStage, bool kSplit>
+template <int CL, bool kAll, bool kNodal, int NG, bool kDB, bool kStage, int kSplit>
 __global__ void __launch_bounds__(kThreadsMixed, 1)
 relax_mixed_kernel(const __grid_constant__ DevBatch b, const __grid_constant__ MixedState ms,
                    const __grid_constant__ RunArgs a, int smem_floats, const int32_t* order,
@@ -1817,10 +1829,13 @@ cudaError_t with_kind(int k, Fn&& fn) {
     case 18: return fn(std::integral_constant<int, 18>{});
     case 19: return fn(std::integral_constant<int, 19>{});
     case 20: return fn(std::integral_constant<int, 20>{});
+    case 21: return fn(std::integral_constant<int, 21>{});
+    case 22: return fn(std::integral_constant<int, 22>{});
+    case 23: return fn(std::integral_constant<int, 23>{});
     default: return cudaErrorInvalidValue;
   }
 }
-static_assert(kKinds == 21, "with_kind covers every launch kind");
+static_assert(kKinds == 24, "with_kind covers every launch kind");
 
 template <int CL, bool kAll>
 cudaLaunchConfig_t launch_config(const MixedState& ms, unsigned grid, cudaStream_t s,
@@ -1878,8 +1893,8 @@ cudaError_t setup_kind(const MixedState& ms, int* clusters) {
 
 // Time of a step of one RVE in launch kind k, in microseconds: fitted to
 // batches of 1 to 304 RVEs of one size at every cluster size, as they run side
-// by side. Linear law, nodes: us on 1, 2, 4, 8, 16 CTAs -- 1,000: 2.3, -, 2.4,
-// 2.4, -; 2,500: 6.3, 3.9, 2.8, 2.4, -; 4,500: 9.9, 5.9, 3.3, 2.6, 2.5; 9,000:
+// by side. Linear law, nodes: us on 1, 2, 4, 8, 16 CTAs -- 1,000: 2.3, 2.3, 2.0,
+// 2.0, -; 2,500: 6.3, 3.8, 2.6, 2.4, 2.0; 4,500: 9.9, 5.8, 3.2, 2.6, 2.3; 9,000:
 // -, 11.5, 6.3, -, -; 20,000: (100 in global memory), -, 13, 7.0, 4.0.
 // Nonlinear -- 1,000: 4.9, 3.8, 2.9, 2.6, -; 4,500: 16, 9.6, 5.7, 4.5, 3.6;
 // 20,000: -, -, 21, 12, 7.4.
@@ -1893,7 +1908,7 @@ double step_us(const RveDesc& d, const BucketKind& k) {
       {1.2, 2.8, 3.5, 3.5, 4.5}, {1.2, 2.4, 2.3, 2.3, 1.8}, {0.6, 1.4, 1.2, 1.45, 1.6}};
   int log2_cl = 0;
   while (1 << log2_cl < k.cl) ++log2_cl;
-  const bool split = k.split && nl && d.n_free <= k.cl * kSplitNodes;
+  const bool split = k.split == kSplitNonlinear && nl && d.n_free <= k.cl * kSplitNodes;
   if (split) return 0.0019 * d.n_fibers / k.cl + 1.9;
   const double per_fiber = nl ? (k.cl == 1 ? 0.0013 : 0.0015) : 0.0008;
   return per_fiber * d.n_fibers / k.cl + fixed[k.db + k.stage][log2_cl] + (nl ? 0.9 : 0.0);
@@ -1954,20 +1969,26 @@ void choose_kinds(const std::vector<RveDesc>& desc,
       if (!holds(kKind[k], desc[r], rowptr.data() + desc[r].row_off, smem_floats)) return false;
     return true;
   };
-  // four lanes to a node where the bucket has a nonlinear RVE whose parts are
-  // small enough: the kernel's linear steps are a tenth slower for it
-  auto splits = [&](int q, int cl) {
-    for (int32_t r : bucket[q])
-      if (desc[r].law == MFG_LAW_NONLINEAR && desc[r].n_free <= cl * kSplitNodes) return true;
-    return false;
+  // Four lanes to a node where the bucket has a nonlinear RVE whose parts are
+  // small enough (the kernel's linear steps are a tenth slower for it), or
+  // where every RVE is linear in such parts (a kernel without the other passes).
+  auto splits = [&](int q, int cl, int split) {
+    bool some = false, all = true;
+    for (int32_t r : bucket[q]) {
+      const bool small = desc[r].n_free <= cl * kSplitNodes;
+      some = some || (small && desc[r].law == MFG_LAW_NONLINEAR);
+      all = all && small && desc[r].law != MFG_LAW_NONLINEAR;
+    }
+    return split == kSplitNonlinear ? some : all;
   };
   // the kind of cl CTAs for bucket q: staged, else two record copies, else one
   auto wider = [&](int q, int cl) {
     for (int level = 3; level >= 0; --level)
       for (int k = 0; k < kKinds; ++k)
         if (kKind[k].nodal && kKind[k].cl == cl &&
-            kKind[k].split + kKind[k].stage + kKind[k].db == level && clusters[k] > 0 &&
-            fits(q, k) && (!kKind[k].split || splits(q, cl)))
+            (kKind[k].split != kSplitNone) + kKind[k].stage + kKind[k].db == level &&
+            clusters[k] > 0 && fits(q, k) &&
+            (kKind[k].split == kSplitNone || splits(q, cl, kKind[k].split)))
           return k;
     return -1;
   };

@@ -1,6 +1,6 @@
-"""Nonlinear RVEs in parts of a few nodes, four lanes to a node: the same bits
-as one CTA per RVE, at part sizes around the limit, with parts that fill no
-warp, and beside RVEs on the linear law."""
+"""RVEs in parts of a few nodes, four lanes to a node: the same bits as one CTA
+per RVE, at part sizes around the limit, with parts that fill no warp, for
+batches all on the linear law and for nonlinear RVEs beside linear ones."""
 import numpy as np
 import pytest
 
@@ -14,14 +14,16 @@ pytestmark = pytest.mark.gpu
     (350, 900, 1_400, 2_000, 2_800, 3_600),
 ])
 @pytest.mark.parametrize("relax", [False, True])
-def test_split_nodes_match_one_cta(lib_path, sizes, relax):
+@pytest.mark.parametrize("linear", [False, True])
+def test_split_nodes_match_one_cta(lib_path, sizes, relax, linear):
     import mumfim_gb300 as m
     from mumfim_gb300 import synthetic as S
     from mumfim_gb300.network_io import Reaction
     nets, F = [], []
     for i, n in enumerate(sizes):
         coords, conn = S.knn_network(n, 3 + i % 3, S.geometry_seed(47, i))
-        rc = Reaction(1, 1e-3, 1.0, 1.0, 4.0, 1.02) if i % 3 != 2 else S._linear_params(47, i)
+        rc = Reaction(1, 1e-3, 1.0, 1.0, 4.0, 1.02) \
+            if i % 3 != 2 and not linear else S._linear_params(47, i)
         nets.append(m.FiberNetwork(coords, conn, [rc]))
         F.append(np.eye(3) + (S.uniform(S.param_seed(47, i), 9) * 0.2 - 0.1).reshape(3, 3))
     F = np.stack(F)
