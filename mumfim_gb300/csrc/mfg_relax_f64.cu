@@ -179,8 +179,11 @@ __device__ __forceinline__ double fiber_vector(const LawF64& L, const double d[3
 __device__ __noinline__ double general_quotient(double x, double m) { return x / m; }
 
 __device__ __forceinline__ double over_mass(double x, double m, uint64_t R) {
-  if (is_zero(x)) return x;
-  if (in_range(x) && R != 0) return div_known(x, m, R);
+  if (is_zero(x)) {
+    if (R != 0) return x;  // else the mass may be zero: 0 / 0
+  } else if (in_range(x) && R != 0) {
+    return div_known(x, m, R);
+  }
   return general_quotient(x, m);
 }
 
