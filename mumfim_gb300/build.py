@@ -37,6 +37,7 @@ SOURCES = [
     ("mfg_metrics.cpp", "cxx", []),
     ("mfg_coupling.cpp", "cxx", []),
     ("mfg_mixed_order.cpp", "cxx", []),
+    ("mfg_mixed_place.cpp", "cxx", []),
     ("mfg_f64_order.cpp", "cxx", []),
     ("mfg_relax_f64.cu", "cuda", ["--fmad=false"]),
     ("mfg_aux.cu", "cuda", ["--fmad=false"]),

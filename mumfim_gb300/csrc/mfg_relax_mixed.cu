@@ -60,6 +60,7 @@
 #include "mfg_mixed.h"
 #include "mfg_mixed_law.cuh"
 #include "mfg_mixed_order.h"
+#include "mfg_mixed_place.h"
 
 namespace cg = cooperative_groups;
 
@@ -70,16 +71,14 @@ namespace mfg {
 // arguments, and the run-time placement's global scratch. Context 0 serves
 // the batch's runs; contexts 1-6 the concurrent perturbed solves of the
 // material stiffness, which run at the same time on the same batch.
-constexpr int kMixedBuckets = 11;
-constexpr int kMaxCluster = 16;
 struct MixedRunCtx {
   int32_t* queues = nullptr;  // one claim counter per bucket (device)
   float* u_hl = nullptr;      // run-time placement scratch; null: the batch's own
   float* v = nullptr;
   float4* nrm = nullptr;
-  cudaStream_t side[kMixedBuckets] = {};
+  cudaStream_t side[kBuckets] = {};
   cudaEvent_t fork = nullptr;
-  cudaEvent_t join[kMixedBuckets] = {};
+  cudaEvent_t join[kBuckets] = {};
   cudaStream_t capture = nullptr;
   cudaGraphExec_t graph = nullptr;
   RunArgs graph_args{};
@@ -131,10 +130,10 @@ struct MixedState {
   // are order[bucket_off[q] .. bucket_off[q + 1]), solved by the launch
   // kind kKind[bucket_kind[q]] (cluster size and solve).
   int32_t* order = nullptr;
-  int bucket_off[kMixedBuckets + 1] = {};
-  int bucket_kind[kMixedBuckets] = {};
-  int bucket_grid[kMixedBuckets] = {};
-  int launch_order[kMixedBuckets] = {};  // buckets, largest clusters first
+  int bucket_off[kBuckets + 1] = {};
+  int bucket_kind[kBuckets] = {};
+  int bucket_grid[kBuckets] = {};
+  int launch_order[kBuckets] = {};  // buckets, largest clusters first
   // Run contexts (host memory; kernels never touch this pointer). A run is a
   // CUDA graph (queue reset, fork, one launch per bucket, join), captured
   // per context for the last run arguments and replayed while they stay
@@ -143,59 +142,6 @@ struct MixedState {
 };
 
 namespace {
-
-constexpr int kThreadsMixed = 1024;
-constexpr int kSmemBytesMixed = 220 * 1024;
-// Four lanes to a node: of the nonlinear RVEs of a bucket, or of every RVE of
-// a bucket that is all linear and all in small parts.
-enum { kSplitNone, kSplitNonlinear, kSplitLinear };
-// How the RVEs of a size bucket are solved.
-struct BucketKind {
-  int cl;      // CTAs per cluster
-  bool all;    // fiber-centric: force vectors in shared memory too
-  bool nodal;  // node-centric solve (node state in shared memory)
-  int ng;      // RVEs solved side by side by one CTA (fiber-centric, all on chip)
-  bool db;     // node-centric with two copies of the node records
-  bool stage;  // and the read-only data of the step in shared memory too
-  int split = kSplitNone;  // and four lanes to a node (nodal_kick_split)
-};
-constexpr int kBuckets = kMixedBuckets;
-// Launch kinds: each bucket's own (the same index), then the wider clusters a
-// bucket may take when the batch leaves SMs idle (choose_kinds).
-constexpr int kKinds = 24;
-constexpr BucketKind kKind[kKinds] = {
-    {8, false, true, 1, false, false}, {4, false, true, 1, true, false},
-    {4, false, true, 1, false, false}, {2, false, true, 1, true, false},
-    {2, false, true, 1, false, false}, {1, false, true, 1, false, false},
-    {1, false, true, 1, true, false},  {1, true, false, 1, false, false},
-    {1, true, false, 2, false, false}, {1, false, false, 1, false, false},
-    {1, false, true, 1, true, true},
-    // wider
-    {8, false, true, 1, true, false},  {16, false, true, 1, true, false},
-    {16, false, true, 1, false, false}, {2, false, true, 1, true, true},
-    {4, false, true, 1, true, true},   {8, false, true, 1, true, true},
-    {16, false, true, 1, true, true},
-    {4, false, true, 1, true, true, kSplitNonlinear},
-    {8, false, true, 1, true, true, kSplitNonlinear},
-    {16, false, true, 1, true, true, kSplitNonlinear},
-    {4, false, true, 1, true, true, kSplitLinear},
-    {8, false, true, 1, true, true, kSplitLinear},
-    {16, false, true, 1, true, true, kSplitLinear}};
-constexpr const BucketKind* kBucket = kKind;
-// Placement preference (bucket_of): the first bucket whose shared memory
-// holds the RVE, else the run-time placement. At each cluster size two
-// copies of the node records come first where they fit, on one CTA with the
-// step's read-only data before without.
-constexpr int kPref[] = {8, 7, 10, 6, 5, 3, 4, 1, 2, 0};
-// The single-CTA buckets with an RVE order of their own, by kind.
-constexpr int kQNodal1 = 5, kQNodalDB = 6, kQFiberAll = 7, kQFiberPair = 8, kQRuntime = 9,
-              kQNodalStage = 10;
-static_assert(kBucket[kQNodal1].cl == 1 && kBucket[kQNodal1].nodal, "bucket table");
-static_assert(kBucket[kQNodalDB].cl == 1 && kBucket[kQNodalDB].db, "bucket table");
-static_assert(kBucket[kQNodalStage].cl == 1 && kBucket[kQNodalStage].stage, "bucket table");
-static_assert(!kBucket[kQRuntime].all && !kBucket[kQRuntime].nodal, "bucket table");
-static_assert(kBucket[kQFiberAll].cl == 1 && kBucket[kQFiberAll].all, "bucket table");
-static_assert(kBucket[kQFiberPair].all && kBucket[kQFiberPair].ng == 2, "bucket table");
 
 __global__ void mixed_prepare_kernel(const DevBatch b, MixedState ms) {
   const int64_t i = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x;
@@ -665,34 +611,6 @@ __device__ __forceinline__ void mixed_stress(const DevBatch& b, const RunArgs& a
   }
 }
 
-// Node slots rounded up to an even count, so that an array of records after
-// another starts on a 16-byte boundary.
-__host__ __device__ inline int64_t even_slots(int64_t n) { return (n + 1) & ~static_cast<int64_t>(1); }
-
-// Shared-memory floats per CTA of an RVE solved by CL CTAs: 9 per node slot
-// (displacement hi, lo and velocity; ceil(NF/CL) free plus ceil(NB/CL)
-// boundary slots), 15 with two copies of the node records, plus 4 per fiber
-// slot (ceil(E/CL)) when the force vectors are kept in shared memory too
-// (all: the fiber-centric single CTA).
-__host__ __device__ inline int64_t cluster_floats(int n_nodes, int n_free, int n_fibers, int cl,
-                                                  bool all, bool two_copies = false) {
-  const int64_t nb = n_nodes - n_free;
-  const int64_t cap = even_slots((static_cast<int64_t>(n_free) + cl - 1) / cl + (nb + cl - 1) / cl);
-  const int64_t echunk = (static_cast<int64_t>(n_fibers) + cl - 1) / cl;
-  return (two_copies ? 15 : 9) * cap + (all ? 4 * echunk : 0);
-}
-
-// First float of the staged read-only data behind two record copies and the
-// velocities (16-byte aligned), and whether it fits: 16 bytes per incidence
-// record, 16 per free node (row and mass), 24 per boundary node (RAMP).
-__host__ __device__ inline int64_t stage_offset(int64_t slots) {
-  return (15 * slots + 3) & ~static_cast<int64_t>(3);
-}
-__host__ __device__ inline bool stage_fits(int64_t slots, int64_t n_free, int64_t n_bnd,
-                                           int64_t n_rec, int64_t smem_floats) {
-  return stage_offset(slots) + 4 * n_rec + 4 * n_free + 6 * n_bnd <= smem_floats;
-}
-
 // Prologue of a solve in FP64 for the CTA's own nodes: the affine predictor
 // (BatchedFiberRVEAnalysisExplicitBase.h:16-57) or, in RAMP mode, the
 // boundary's per-step increment; displacements split into (hi, lo); v = 0.
@@ -1108,8 +1026,6 @@ __device__ __forceinline__ double nodal_kick(const Law& law, const Nodes& u, con
 // L2 after each cluster barrier, and beside them cost more than is gained
 // (2.5 -> 2.9). Two lanes to a node for up to kThreadsMixed / 2 nodes lose
 // (nonlinear, 4,500 on 8: 4.5 -> 4.9).
-constexpr int kLanes = 4;
-constexpr int kSplitNodes = kThreadsMixed / kLanes;
 template <int kLaw, class Nodes>
 __device__ __forceinline__ void nodal_kick_split(const Law& law, const Nodes& u,
                                                  const LocalNodes& own, float* vel,
@@ -1506,7 +1422,6 @@ server_mixed_kernel(const DevBatch b, const MixedState ms, const ServerArgs sa, 
 // same number of times: every loop is bounded, and the decision to leave is
 // taken by the leader and broadcast before anyone acts on it. Shutdown is
 // collective as in server_loop, with clusters as the units.
-constexpr int kClusterServe = 4;
 constexpr int kSmallPerRound = 16;
 enum : int { kServeExit = 0, kServeBig = 1, kServeSmall = 2 };
 
@@ -1745,65 +1660,6 @@ void mixed_destroy(MixedState* ms) {
 
 namespace {
 
-// Incidence records that a CTA of a cluster of cl stages at most for its free
-// nodes: their degrees, and what slices of 32 nodes as wide as their widest
-// row add (the nodes are in falling degree within two groups, so a slice is
-// no wider than the mean row of the one before it but for each group's first
-// two).
-int64_t stage_records(const RveDesc& d, int cl, const int32_t* rowptr) {
-  const int NF = d.n_free, fchunk = (NF + cl - 1) / cl;
-  int64_t most = 0;
-  for (int lo = 0; lo < NF; lo += fchunk) {
-    const int hi = std::min(NF, lo + fchunk);
-    int widest = 0;
-    for (int j = lo; j < hi; ++j) widest = std::max(widest, rowptr[j + 1] - rowptr[j]);
-    most = std::max<int64_t>(most, rowptr[hi] - rowptr[lo] + 96LL * widest);
-  }
-  return most;
-}
-
-// Whether launch kind k holds an RVE in its CTAs' shared memory.
-bool holds(const BucketKind& k, const RveDesc& d, const int32_t* rowptr, int64_t smem_floats) {
-  if (cluster_floats(d.n_nodes, d.n_free, d.n_fibers, k.cl, k.all && !k.nodal, k.db) >
-      smem_floats / k.ng)
-    return false;
-  if (!k.stage) return true;
-  const int nb = d.n_nodes - d.n_free, fchunk = (d.n_free + k.cl - 1) / k.cl;
-  return stage_fits(even_slots(fchunk + (nb + k.cl - 1) / k.cl), fchunk, (nb + k.cl - 1) / k.cl,
-                    stage_records(d, k.cl, rowptr), smem_floats);
-}
-
-// Bucket of an RVE: the smallest of one CTA or a cluster of 2, 4 or 8 CTAs
-// whose shared memory holds its node state (node-centric solve; at that
-// size with two copies of the node records where they fit), else one
-// CTA that keeps what fits in shared memory and streams the rest from global
-// memory (fiber-centric solve). Clusters of 8 are the last resort: with
-// 220 KB per CTA only 15 of them (120 SMs) are resident at once, against 36
-// clusters of 4 (144 SMs). Clusters above max_cluster CTAs are not used,
-// nor clusters of 2 in the serving layout (the serving kernel solves in
-// clusters of 4 only).
-// With the fiber-centric small solve, RVEs whose whole state fits half a
-// CTA's shared memory come first (two of them share a CTA, at most
-// rves_per_cta), then those whose whole state fits one CTA; otherwise those
-// buckets are skipped and every RVE whose node state fits takes the
-// node-centric solve. small_solve (mfg_small_rve_solve) picks the solve;
-// AUTO takes the fiber-centric one for RVEs on the nonlinear law, whose
-// exponential the node-centric solve would evaluate at both ends of every
-// fiber, and the node-centric one for the linear law, where it runs 2 %
-// (500 - 1,300 nodes) to 37 % (1,300 - 3,300 nodes) faster.
-int bucket_of(const RveDesc& d, const int32_t* rowptr, int smem_floats, int max_cluster,
-              bool serving_layout, int small_solve, int rves_per_cta) {
-  const bool fiber_small =
-      small_solve == MFG_SMALL_FIBER_CENTRIC ||
-      (small_solve == MFG_SMALL_AUTO && d.law == MFG_LAW_NONLINEAR);
-  for (int q : kPref)
-    if ((fiber_small || !kBucket[q].all) && kBucket[q].cl <= max_cluster &&
-        !(serving_layout && kBucket[q].cl == 2) && kBucket[q].ng <= rves_per_cta &&
-        holds(kBucket[q], d, rowptr, smem_floats))
-      return q;
-  return kQRuntime;
-}
-
 // Calls fn(std::integral_constant<int, k>{}) for the run-time launch kind k.
 template <class Fn>
 cudaError_t with_kind(int k, Fn&& fn) {
@@ -1889,215 +1745,6 @@ cudaError_t setup_kind(const MixedState& ms, int* clusters) {
   return cudaSuccess;
 }
 
-// ---- width of the size buckets ------------------------------------------------
-
-// Time of a step of one RVE in launch kind k, in microseconds: fitted to
-// batches of 1 to 304 RVEs of one size at every cluster size, as they run side
-// by side. Linear law, nodes: us on 1, 2, 4, 8, 16 CTAs -- 1,000: 2.3, 2.3, 2.0,
-// 2.0, -; 2,500: 6.3, 3.8, 2.6, 2.4, 2.0; 4,500: 9.9, 5.8, 3.2, 2.6, 2.3; 9,000:
-// -, 11.5, 6.3, -, -; 20,000: (100 in global memory), -, 13, 7.0, 4.0.
-// Nonlinear -- 1,000: 4.9, 3.8, 2.9, 2.6, -; 4,500: 16, 9.6, 5.7, 4.5, 3.6;
-// 20,000: -, -, 21, 12, 7.4.
-double step_us(const RveDesc& d, const BucketKind& k) {
-  const bool nl = d.law == MFG_LAW_NONLINEAR;
-  if (k.all) return k.ng == 2 ? 0.0014 * d.n_fibers + 1.5 : 0.0011 * d.n_fibers + 2.0;
-  if (!k.nodal) return 0.002 * d.n_fibers;  // (part of) the state in global memory
-  // barriers and the tail of a part, by cluster size (1, 2, 4, 8, 16): one
-  // copy of the node records, two, and two with the read-only data staged
-  constexpr double fixed[3][5] = {
-      {1.2, 2.8, 3.5, 3.5, 4.5}, {1.2, 2.4, 2.3, 2.3, 1.8}, {0.6, 1.4, 1.2, 1.45, 1.6}};
-  int log2_cl = 0;
-  while (1 << log2_cl < k.cl) ++log2_cl;
-  const bool split = k.split == kSplitNonlinear && nl && d.n_free <= k.cl * kSplitNodes;
-  if (split) return 0.0019 * d.n_fibers / k.cl + 1.9;
-  const double per_fiber = nl ? (k.cl == 1 ? 0.0013 : 0.0015) : 0.0008;
-  return per_fiber * d.n_fibers / k.cl + fixed[k.db + k.stage][log2_cl] + (nl ? 0.9 : 0.0);
-}
-
-// Time of `copies` solves of the batch with the buckets in these kinds: RVE
-// after RVE, bucket by bucket with the largest clusters first and the longest
-// first in a bucket, each onto the SMs that are free first. No more than
-// clusters[k] of a kind run at once, whatever SMs are left beside them: 36 of
-// 4 CTAs and 15 of 8 on 152 SMs, which a share of whole SMs a cluster (5 and
-// 11) would take for 30 and 13 (36 RVEs of 19,500 nodes, then put on clusters
-// of 8 in three waves: 22.0 us a step, on 4 in one wave: 13.0).
-double batch_us(const std::vector<RveDesc>& desc, const std::vector<std::vector<int32_t>>& bucket,
-                const int* kind, const int* clusters, int sms, int copies) {
-  std::vector<int> order;
-  for (int q = 0; q < kBuckets; ++q)
-    if (!bucket[q].empty()) order.push_back(q);
-  std::stable_sort(order.begin(), order.end(),
-                   [&](int x, int y) { return kKind[kind[x]].cl > kKind[kind[y]].cl; });
-  std::vector<double> sm(sms, 0.0);  // when each SM is free, ascending
-  for (int q : order) {
-    const BucketKind& k = kKind[kind[q]];
-    const int share = std::min(k.cl, sms);
-    const size_t most = static_cast<size_t>(std::max(clusters[kind[q]], 1));
-    std::priority_queue<double, std::vector<double>, std::greater<double>> ends;
-    const size_t n = bucket[q].size() * copies;
-    for (size_t i = 0; i < n; i += k.ng) {
-      const RveDesc& d = desc[bucket[q][i / copies]];
-      // two RVEs side by side on a CTA take 1.4 times as long as one there
-      const double t = step_us(d, k) * d.max_steps * (i + 1 < n && k.ng == 2 ? 1.4 : 1.0);
-      double start = sm[share - 1];
-      if (ends.size() == most) {  // one of the kind has to end first
-        start = std::max(start, ends.top());
-        ends.pop();
-      }
-      ends.push(start + t);
-      // the SMs that come free last before then, so that the others stay free
-      const auto hi = std::upper_bound(sm.begin(), sm.end(), start);
-      sm.erase(hi - share, hi);
-      sm.insert(std::upper_bound(sm.begin(), sm.end(), start + t), share, start + t);
-    }
-  }
-  return sm.back();
-}
-
-// Widens buckets while the batch's estimated time falls: a batch that leaves
-// SMs idle solves its RVEs on larger clusters than they need. Starts from
-// each bucket's own kind in `kind`; RVEs in global memory (the run-time placement)
-// go to clusters of 16 where those hold them. Bucket by bucket, so that a
-// batch keeps one launch per size bucket.
-void choose_kinds(const std::vector<RveDesc>& desc,
-                  const std::vector<std::vector<int32_t>>& bucket,
-                  const std::vector<int32_t>& rowptr, int smem_floats, int max_cluster,
-                  bool keep_fiber_centric, const int* clusters, int sms,
-                  int copies, int* kind) {
-  auto fits = [&](int q, int k) {
-    for (int32_t r : bucket[q])
-      if (!holds(kKind[k], desc[r], rowptr.data() + desc[r].row_off, smem_floats)) return false;
-    return true;
-  };
-  // Four lanes to a node where the bucket has a nonlinear RVE whose parts are
-  // small enough (the kernel's linear steps are a tenth slower for it), or
-  // where every RVE is linear in such parts (a kernel without the other passes).
-  auto splits = [&](int q, int cl, int split) {
-    bool some = false, all = true;
-    for (int32_t r : bucket[q]) {
-      const bool small = desc[r].n_free <= cl * kSplitNodes;
-      some = some || (small && desc[r].law == MFG_LAW_NONLINEAR);
-      all = all && small && desc[r].law != MFG_LAW_NONLINEAR;
-    }
-    return split == kSplitNonlinear ? some : all;
-  };
-  // the kind of cl CTAs for bucket q: staged, else two record copies, else one
-  auto wider = [&](int q, int cl) {
-    for (int level = 3; level >= 0; --level)
-      for (int k = 0; k < kKinds; ++k)
-        if (kKind[k].nodal && kKind[k].cl == cl &&
-            (kKind[k].split != kSplitNone) + kKind[k].stage + kKind[k].db == level &&
-            clusters[k] > 0 && fits(q, k) &&
-            (kKind[k].split == kSplitNone || splits(q, cl, kKind[k].split)))
-          return k;
-    return -1;
-  };
-  // widen the bucket whose RVE takes longest, again and again; keep the best
-  // state met (a state no better than the one before it may lead to one)
-  int best[kBuckets], now[kBuckets];
-  std::copy(kind, kind + kBuckets, best);
-  std::copy(kind, kind + kBuckets, now);
-  double t_best = batch_us(desc, bucket, kind, clusters, sms, copies);
-  for (;;) {
-    int q_long = -1;
-    double longest = 0.0;
-    for (int q = 0; q < kBuckets; ++q)
-      for (int32_t r : bucket[q]) {
-        const double t = step_us(desc[r], kKind[now[q]]) * desc[r].max_steps;
-        if (t > longest) {
-          longest = t;
-          q_long = q;
-        }
-      }
-    if (q_long < 0 || (kKind[now[q_long]].all && keep_fiber_centric)) break;
-    int k = -1;
-    for (int cl = 2 * kKind[now[q_long]].cl; k < 0 && cl <= max_cluster; cl *= 2)
-      k = wider(q_long, cl);
-    if (k < 0) break;
-    now[q_long] = k;
-    const double t = batch_us(desc, bucket, now, clusters, sms, copies);
-    if (t < 0.97 * t_best) {  // a wider bucket has to pay
-      t_best = t;
-      std::copy(now, now + kBuckets, best);
-    } else if (t > 1.15 * t_best) {
-      break;
-    }
-  }
-  std::copy(best, best + kBuckets, kind);
-}
-
-// Serving layout: which of the RVEs that one CTA holds go to clusters of 4 all
-// the same. A wave of requests, one per RVE, ends with its longest chain, and
-// a single CTA takes two to three times as long for its RVE as a cluster, at
-// up to twice the SM time. Requests are taken in order, large ones first: the
-// wave's time is estimated so (clusters for the large, then CTA by CTA) for the
-// longest 0, 1, 2, 3, 4, 6, ... single-CTA RVEs moved, and the best is taken
-// where it saves a tenth. Two waves of 96 RVEs of 500 - 20,000 nodes, both laws,
-// 200 steps: 14.2 ms with every RVE on one CTA that fits one, 11.3 so; of 13
-// RVEs of 1,800 - 5,100 nodes, 344 steps: 10.5, 5.3; of 53 RVEs up to 2,200 nodes,
-// where nothing moves: 2.9, 2.9. Returns the bucket per RVE in rve_q.
-void serve_on_clusters(const std::vector<RveDesc>& desc, const std::vector<int32_t>& rowptr,
-                       int smem_floats, int clusters, std::vector<int>& rve_q) {
-  constexpr int kQCluster = 2, kQClusterDB = 1;
-  static_assert(kKind[kQCluster].cl == kClusterServe && kKind[kQClusterDB].cl == kClusterServe,
-                "bucket table");
-  const size_t n = rve_q.size();
-  // a wave that fills the CTAs several times over is better off on single ones
-  if (clusters < 1 || n > 4 * static_cast<size_t>(clusters) * kClusterServe) return;
-  std::vector<double> one(n), four(n);  // a request's time on one CTA and on a cluster
-  std::vector<int> movable;
-  for (size_t r = 0; r < n; ++r) {
-    int q = rve_q[r] == kQNodalStage ? kQNodalDB : rve_q[r];  // not staged there
-    one[r] = step_us(desc[r], kKind[q]) * desc[r].max_steps * (kKind[q].ng == 2 ? 1.3 : 1.0);
-    four[r] = step_us(desc[r], kKind[kQCluster]) * desc[r].max_steps;
-    if (kKind[q].cl == 1 && q != kQRuntime && four[r] < 0.8 * one[r] &&
-        holds(kKind[kQCluster], desc[r], rowptr.data() + desc[r].row_off, smem_floats))
-      movable.push_back(static_cast<int>(r));
-  }
-  std::stable_sort(movable.begin(), movable.end(), [&](int x, int y) { return one[x] > one[y]; });
-  using Heap = std::priority_queue<double, std::vector<double>, std::greater<double>>;
-  std::vector<char> moved(n, 0);
-  auto wave = [&] {
-    Heap by_cluster, by_cta;
-    for (int c = 0; c < clusters; ++c) by_cluster.push(0.0);
-    double end = 0.0;
-    for (size_t r = 0; r < n; ++r)
-      if (moved[r] || kKind[rve_q[r]].cl == kClusterServe) {
-        const double t = by_cluster.top() + four[r];
-        by_cluster.pop();
-        by_cluster.push(t);
-        end = std::max(end, t);
-      }
-    for (; !by_cluster.empty(); by_cluster.pop())
-      for (int k = 0; k < kClusterServe; ++k) by_cta.push(by_cluster.top());
-    for (size_t r = 0; r < n; ++r)
-      if (!moved[r] && kKind[rve_q[r]].cl != kClusterServe) {
-        const double t = by_cta.top() + one[r];
-        by_cta.pop();
-        by_cta.push(t);
-        end = std::max(end, t);
-      }
-    return end;
-  };
-  double best = 0.9 * wave();
-  size_t take = 0, m = 0;
-  while (m < movable.size()) {
-    const size_t next = std::min(movable.size(), m + 1 + m / 3);
-    for (; m < next; ++m) moved[movable[m]] = 1;
-    const double t = wave();
-    if (t < best) {
-      best = t;
-      take = m;
-    }
-  }
-  for (size_t k = 0; k < take; ++k) {
-    const int r = movable[k];
-    rve_q[r] = holds(kKind[kQClusterDB], desc[r], rowptr.data() + desc[r].row_off, smem_floats)
-                   ? kQClusterDB
-                   : kQCluster;
-  }
-}
-
 }  // namespace
 
 cudaError_t mixed_create(MixedState& ms, const DevBatch& b, const std::vector<RveDesc>& desc,
@@ -2143,18 +1790,7 @@ cudaError_t mixed_create(MixedState& ms, const DevBatch& b, const std::vector<Rv
                      [&](int32_t x, int32_t y) { return desc[x].n_fibers > desc[y].n_fibers; });
     ms.bucket_kind[q] = q;
   }
-  // Wider clusters: not in the serving layout (its kernels solve in clusters
-  // of 4), and not worth estimating for a batch that fills the GPU many times.
-  // For several solves at once only where they leave a third of the SMs idle:
-  // their clusters wait for neighbouring SMs to fall free (six solves of 32
-  // RVEs of 1,000 - 10,000 nodes, 200 steps: 4.2 ms widened, 3.7 not; of 8 RVEs
-  // of 500 - 20,000, 84 SMs of 152: 1.7 ms, 2.8 not).
-  size_t ctas = 0;
-  for (int q = 0; q < kBuckets; ++q) ctas += bucket[q].size() * copies * kBucket[q].cl;
-  const bool widen = !serving_layout &&
-                     (!bucket[kQRuntime].empty() ||
-                      (copies == 1 ? desc.size() <= 8 * static_cast<size_t>(sms)
-                                   : 3 * ctas <= 2 * static_cast<size_t>(sms)));
+  const bool widen = may_widen(bucket, sms, serving_layout, copies);
   for (int k = 0; k < kKinds; ++k) {
     const bool used = k < kBuckets && !bucket[k].empty();
     if (!used && !(widen && kKind[k].nodal && kKind[k].cl > 1 && kKind[k].cl <= max_cluster))
