@@ -204,7 +204,7 @@ void choose_kinds(const std::vector<RveDesc>& desc,
 }
 
 void serve_on_clusters(const std::vector<RveDesc>& desc, const std::vector<int32_t>& rowptr,
-                       int smem_floats, int clusters, std::vector<int>& rve_q) {
+                       int smem_floats, int clusters, int sms, std::vector<int>& rve_q) {
   constexpr int kQCluster = 2, kQClusterDB = 1;
   static_assert(kKind[kQCluster].cl == kClusterServe && kKind[kQClusterDB].cl == kClusterServe,
                 "bucket table");
@@ -213,46 +213,62 @@ void serve_on_clusters(const std::vector<RveDesc>& desc, const std::vector<int32
   if (clusters < 1 || n > 4 * static_cast<size_t>(clusters) * kClusterServe) return;
   std::vector<double> one(n), four(n);  // a request's time on one CTA and on a cluster
   std::vector<int> movable;
+  std::vector<char> big(n, 0);  // solved on a cluster
   for (size_t r = 0; r < n; ++r) {
-    int q = rve_q[r] == kQNodalStage ? kQNodalDB : rve_q[r];  // not staged there
+    // the serving kernels stage nothing and have no clusters of 8
+    const int q = rve_q[r] == kQNodalStage ? kQNodalDB
+                                           : (kKind[rve_q[r]].cl > kClusterServe ? kQRuntime : rve_q[r]);
     one[r] = step_us(desc[r], kKind[q]) * desc[r].max_steps * (kKind[q].ng == 2 ? 1.3 : 1.0);
     four[r] = step_us(desc[r], kKind[kQCluster]) * desc[r].max_steps;
+    big[r] = kKind[q].cl == kClusterServe;
     if (kKind[q].cl == 1 && q != kQRuntime && four[r] < 0.8 * one[r] &&
         holds(kKind[kQCluster], desc[r], rowptr.data() + desc[r].row_off, smem_floats))
       movable.push_back(static_cast<int>(r));
   }
   std::stable_sort(movable.begin(), movable.end(), [&](int x, int y) { return one[x] > one[y]; });
   using Heap = std::priority_queue<double, std::vector<double>, std::greater<double>>;
-  std::vector<char> moved(n, 0);
-  auto wave = [&] {
+  auto any_big = [&] { return std::find(big.begin(), big.end(), 1) != big.end(); };
+  // end of a wave when `share` CTAs of a cluster take small requests at a time
+  auto wave = [&](int share) {
     Heap by_cluster, by_cta;
-    for (int c = 0; c < clusters; ++c) by_cluster.push(0.0);
     double end = 0.0;
+    auto next = [&](Heap& heap, double time) {
+      const double t = heap.top() + time;
+      heap.pop();
+      heap.push(t);
+      end = std::max(end, t);
+    };
+    if (any_big()) {
+      for (int c = 0; c < clusters; ++c) by_cluster.push(0.0);
+      for (size_t r = 0; r < n; ++r)
+        if (big[r]) next(by_cluster, four[r]);
+      for (; !by_cluster.empty(); by_cluster.pop())
+        for (int k = 0; k < share; ++k) by_cta.push(by_cluster.top());
+    } else {
+      for (int c = 0; c < sms; ++c) by_cta.push(0.0);
+    }
     for (size_t r = 0; r < n; ++r)
-      if (moved[r] || kKind[rve_q[r]].cl == kClusterServe) {
-        const double t = by_cluster.top() + four[r];
-        by_cluster.pop();
-        by_cluster.push(t);
-        end = std::max(end, t);
-      }
-    for (; !by_cluster.empty(); by_cluster.pop())
-      for (int k = 0; k < kClusterServe; ++k) by_cta.push(by_cluster.top());
-    for (size_t r = 0; r < n; ++r)
-      if (!moved[r] && kKind[rve_q[r]].cl != kClusterServe) {
-        const double t = by_cta.top() + one[r];
-        by_cta.pop();
-        by_cta.push(t);
-        end = std::max(end, t);
-      }
+      if (!big[r]) next(by_cta, one[r]);
     return end;
   };
-  double best = 0.9 * wave();
+  // time of a request of every RVE when requests never run out: the SMs' or,
+  // since an RVE solves one request at a time, the RVEs' own
+  auto saturated = [&] {
+    double sm = 0.0, chain = 0.0;
+    for (size_t r = 0; r < n; ++r) {
+      sm += big[r] ? kClusterServe * four[r] : one[r];
+      chain += big[r] ? four[r] : one[r];
+    }
+    return std::max(sm / (any_big() ? kClusterServe * clusters : sms), chain / n);
+  };
+  double best = 0.9 * wave(kClusterServe);
+  const double spread = wave(1), busy = saturated();
   size_t take = 0, m = 0;
   while (m < movable.size()) {
     const size_t next = std::min(movable.size(), m + 1 + m / 3);
-    for (; m < next; ++m) moved[movable[m]] = 1;
-    const double t = wave();
-    if (t < best) {
+    for (; m < next; ++m) big[movable[m]] = 1;
+    const double t = wave(kClusterServe);
+    if (t < best && wave(1) <= spread && saturated() <= 1.05 * busy) {
       best = t;
       take = m;
     }

@@ -145,16 +145,27 @@ void choose_kinds(const std::vector<RveDesc>& desc,
 
 // Serving layout: which of the RVEs that one CTA holds go to clusters of 4 all
 // the same. A wave of requests, one per RVE, ends with its longest chain, and
-// a single CTA takes two to three times as long for its RVE as a cluster, at
-// up to twice the SM time. Requests are taken in order, large ones first: the
-// wave's time is estimated so (clusters for the large, then CTA by CTA) for the
-// longest 0, 1, 2, 3, 4, 6, ... single-CTA RVEs moved, and the best is taken
-// where it saves a tenth. Two waves of 96 RVEs of 500 - 20,000 nodes, both laws,
-// 200 steps: 14.2 ms with every RVE on one CTA that fits one, 11.3 so; of 13
-// RVEs of 1,800 - 5,100 nodes, 344 steps: 10.5, 5.3; of 53 RVEs up to 2,200 nodes,
-// where nothing moves: 2.9, 2.9. Returns the bucket per RVE in rve_q.
+// a single CTA takes two to three times as long for its RVE as a cluster, which
+// takes up to 3.2 times the SM time for it. Three estimates, for the longest 0,
+// 1, 2, 3, 4, 6, ... single-CTA RVEs moved:
+//  - the wave with large requests taken first and each CTA free for small ones
+//    has to be a tenth shorter;
+//  - the wave with one CTA of a cluster at work on small requests must not be
+//    longer: a cluster's CTAs that find no small request when they look wait
+//    for the one that did, so requests that come one by one occupy a cluster
+//    each (without clusters, all `sms` CTAs serve on their own);
+//  - the time of a request of every RVE in a stream that never runs dry must not
+//    grow by more than a twentieth.
+// The best by the first is taken. Requests/s of a stream with three waves queued,
+// and ms of two waves (200 steps), with every RVE on the smallest placement / by
+// the first estimate alone / so:
+//   150 RVEs of 3,000 - 6,000, linear  80,400, 7.3 / 42,200, 10.8 / 80,400, 7.3
+//   36 of these                        18,500, 5.8 / 27,000, 4.0 / 27,000, 4.0
+//   110 of 300 - 6,200, both laws      83,100, 9.5 / 58,800, 7.0 / 82,700, 9.5
+//   96 of 500 - 20,000, both laws      31,900, 12.6 / 31,600, 11.3 / 31,300, 11.2
+// Returns the bucket per RVE in rve_q.
 void serve_on_clusters(const std::vector<RveDesc>& desc, const std::vector<int32_t>& rowptr,
-                       int smem_floats, int clusters, std::vector<int>& rve_q);
+                       int smem_floats, int clusters, int sms, std::vector<int>& rve_q);
 
 }  // namespace mfg
 

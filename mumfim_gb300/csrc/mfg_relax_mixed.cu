@@ -1782,7 +1782,7 @@ cudaError_t mixed_create(MixedState& ms, const DevBatch& b, const std::vector<Rv
     rve_q[r] = bucket_of(desc[r], rowptr.data() + desc[r].row_off, smem_floats,
                          std::min(max_cluster, 8), serving_layout, small_solve, rves_per_cta);
   if (serving_layout && max_cluster >= kClusterServe && small_solve != MFG_SMALL_FIBER_CENTRIC)
-    serve_on_clusters(desc, rowptr, smem_floats, ms.server_grid / kClusterServe, rve_q);
+    serve_on_clusters(desc, rowptr, smem_floats, ms.server_grid / kClusterServe, sms, rve_q);
   for (size_t r = 0; r < desc.size(); ++r) bucket[rve_q[r]].push_back(static_cast<int32_t>(r));
   int clusters[kKinds] = {};
   for (int q = 0; q < kBuckets; ++q) {

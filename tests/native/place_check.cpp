@@ -39,7 +39,7 @@ int main() {
   for (int r = 0; r < n; ++r)
     rve_q[r] = bucket_of(desc[r], rowptr.data() + desc[r].row_off, smem_floats,
                          std::min(max_cluster, 8), serving, small_solve, 2);
-  if (serving) serve_on_clusters(desc, rowptr, smem_floats, held[2], rve_q);
+  if (serving) serve_on_clusters(desc, rowptr, smem_floats, held[2], sms, rve_q);
   std::vector<std::vector<int32_t>> bucket(kBuckets);
   for (int r = 0; r < n; ++r) bucket[rve_q[r]].push_back(r);
   int clusters[kKinds], kind[kBuckets];

@@ -108,6 +108,33 @@ def test_f64_cluster_size(place, rves, want):
     assert place(rves)[0] == want
 
 
+# ---- serving: RVEs that one CTA holds, on clusters of 4 ---------------------------------------
+
+def _spread(n, lo, hi):
+    return [int(round(lo * (hi / lo) ** ((i * 0.6180339887498949 + 0.5) % 1.0))) for i in range(n)]
+
+
+@pytest.mark.parametrize("n,lo,hi,both,want", [
+    # single CTAs keep the SMs busy: a cluster would take two to three times the
+    # SM time, and its CTAs wait for one another between small requests
+    (150, 3_000, 6_000, False, 0), (110, 300, 6_000, True, 0), (96, 2_000, 6_000, False, 0),
+    # fewer RVEs than clusters: nothing waits
+    (36, 3_000, 6_000, False, 36), (13, 1_800, 5_100, True, 10),
+    (53, 500, 2_200, True, 0),    # too small to be faster on four CTAs
+    (600, 1_000, 6_000, False, 0)])
+def test_served_on_clusters(place, n, lo, hi, both, want):
+    rves = [rve(x, int(both and i % 2 == 1)) for i, x in enumerate(_spread(n, lo, hi))]
+    assert ctas(place(rves, serving=True)[1]).count(4) == want
+
+
+def test_few_move_beside_rves_that_need_a_cluster(place):
+    sizes = _spread(96, 500, 20_000)
+    rves = [rve(x, i % 2) for i, x in enumerate(sizes)]
+    need = sum(9 * 4 * ((x + 1) // 2 * 2) > 220 * 1024 for x in sizes)
+    moved = ctas(place(rves, serving=True)[1]).count(4) - need
+    assert 1 <= moved <= 8  # the longest; all 30 that would be faster alone cost throughput
+
+
 # ---- the GPU tests that compare placements ----------------------------------------------------
 
 @pytest.mark.parametrize("sizes,law,narrow", [
