@@ -1257,7 +1257,7 @@ struct PendingReq {
   double t_submit;
 };
 
-// Device footprint of a batch's state (FP64 arrays, CSR, and the mixed
+// Device footprint of a server's state (FP64 arrays, CSR, and the mixed
 // working set when used), for admission against the HBM budget.
 double batch_bytes(int64_t nt, int64_t et, int64_t nbt, int64_t R, bool mixed) {
   double b = nt * (5 * 3 * 8.0 + 8 + 4) + et * (8.0 + 8 + 24 + 8) + nbt * (48.0 + 4) + R * 200.0;
@@ -1265,6 +1265,37 @@ double batch_bytes(int64_t nt, int64_t et, int64_t nbt, int64_t R, bool mixed) {
   if (mixed)  // + node-centric incidences (about 2.3 per fiber, with the set-up fiber ids)
     b += nt * (24.0 + 12 + 8 + 4 + 4 + 8 + 8) + et * (16.0 + 16 + 16 + 8 + 8 + 4 + 64) + R * 20.0;
   return b;
+}
+
+double server_bytes(const mfg_network* nets, int32_t n_rve, int32_t precision) {
+  int64_t nt = 0, et = 0;
+  for (int r = 0; r < n_rve; ++r) {
+    nt += std::max(nets[r].n_nodes, 0);
+    et += std::max(nets[r].n_fibers, 0);
+  }
+  return batch_bytes(nt, et, nt / 8, n_rve, precision == MFG_PREC_MIXED);
+}
+
+// What a batch may take above that: an FP64 batch that leaves SMs idle keeps
+// its RVEs' parts for the cluster solve (plan_f64_clusters), in which a fiber
+// between two CTAs counts twice. A mixed batch takes less than a server (no
+// run-time placement scratch but where an RVE needs it).
+double plan_bytes(const mfg_network* nets, int32_t n_rve, int32_t precision) {
+  if (precision == MFG_PREC_MIXED) return 0.0;
+  constexpr int kClusters[5] = {152, 76, 36, 15, 7};  // of 1, 2, 4, 8, 16 CTAs a GB300 holds
+  std::vector<mfg::RveDesc> desc(n_rve);
+  double b = 0.0;
+  for (int r = 0; r < n_rve; ++r) {
+    mfg::RveDesc& d = desc[r];
+    std::memset(&d, 0, sizeof(d));
+    d.n_nodes = std::max(nets[r].n_nodes, 0);
+    d.n_fibers = std::max(nets[r].n_fibers, 0);
+    d.max_steps = 1;
+    b += d.n_nodes * (sizeof(int32_t) * 2.0 + sizeof(mfg::F64Mass)) +
+         2.0 * d.n_fibers * (sizeof(int32_t) + sizeof(int2) + sizeof(mfg::F64Len)) +
+         16.0 * (sizeof(mfg::F64Part) + sizeof(int32_t));
+  }
+  return mfg::f64_cluster_size(desc, kClusters, 1) > 1 ? b : 0.0;
 }
 
 }  // namespace
@@ -1474,12 +1505,7 @@ mfg_status mfg_server_create(const mfg_network* nets, const mfg_strategy* strate
   bo.cluster_layout = MFG_LAYOUT_SERVING;
   // admission: the device state of every registered RVE must fit the budget
   if (nets && n_rve > 0) {
-    int64_t nt = 0, et = 0;
-    for (int r = 0; r < n_rve; ++r) {
-      nt += std::max(nets[r].n_nodes, 0);
-      et += std::max(nets[r].n_fibers, 0);
-    }
-    const double need = batch_bytes(nt, et, nt / 8, n_rve, opt.precision == MFG_PREC_MIXED);
+    const double need = server_bytes(nets, n_rve, opt.precision);
     double budget = opt.hbm_budget_bytes;
     if (budget <= 0) {
       size_t fr = 0, tot = 0;
@@ -1547,12 +1573,12 @@ mfg_status mfg_server_create(const mfg_network* nets, const mfg_strategy* strate
 
 double mfg_device_bytes_estimate(const mfg_network* nets, int32_t n_rve, int32_t precision) {
   if (!nets || n_rve < 1) return 0.0;
-  int64_t nt = 0, et = 0;
-  for (int r = 0; r < n_rve; ++r) {
-    nt += std::max(nets[r].n_nodes, 0);
-    et += std::max(nets[r].n_fibers, 0);
-  }
-  return batch_bytes(nt, et, nt / 8, n_rve, precision == MFG_PREC_MIXED);
+  return server_bytes(nets, n_rve, precision) + plan_bytes(nets, n_rve, precision);
+}
+
+double mfg_server_bytes_estimate(const mfg_network* nets, int32_t n_rve, int32_t precision) {
+  if (!nets || n_rve < 1) return 0.0;
+  return server_bytes(nets, n_rve, precision);
 }
 
 mfg_status mfg_server_submit(mfg_server* sv, int32_t rve, const double* F, int32_t update_coords,

@@ -42,8 +42,9 @@ def _lib():
         L.mfg_server_batch.argtypes = [vp]
         L.mfg_server_destroy.restype = i32
         L.mfg_server_destroy.argtypes = [vp]
-        L.mfg_device_bytes_estimate.restype = C.c_double
-        L.mfg_device_bytes_estimate.argtypes = [C.POINTER(_abi.mfg_network), i32, i32]
+        for n in ("mfg_device_bytes_estimate", "mfg_server_bytes_estimate"):
+            getattr(L, n).restype = C.c_double
+            getattr(L, n).argtypes = [C.POINTER(_abi.mfg_network), i32, i32]
         L._server_ready = True
     return L
 
@@ -155,6 +156,13 @@ def device_bytes_estimate(networks: Sequence, precision: str = "mixed") -> float
     return float(_lib().mfg_device_bytes_estimate(arr.nets, len(networks), prec))
 
 
+def server_bytes_estimate(networks: Sequence, precision: str = "mixed") -> float:
+    """mfg_server_bytes_estimate(): device memory of a server of `networks`."""
+    arr = NetworkArray(networks, [SolutionStrategy()] * len(networks))
+    prec = {"f64": MFG_PREC_F64, "mixed": MFG_PREC_MIXED}[precision]
+    return float(_lib().mfg_server_bytes_estimate(arr.nets, len(networks), prec))
+
+
 class PagedRVEServer:
     """Continuous-batching service over more RVEs than a device-memory budget
     holds: admission per request, eviction of idle RVEs to host memory.
@@ -163,7 +171,7 @@ class PagedRVEServer:
     is made resident -- its own RVEServer, so its RVEs' state lives on the
     device -- when a request for one of its RVEs arrives. If the estimated
     device memory of the resident pages and the new one
-    (mfg_device_bytes_estimate) would exceed `hbm_budget_bytes`, the least
+    (mfg_server_bytes_estimate) would exceed `hbm_budget_bytes`, the least
     recently used pages without a request in flight are evicted first: every
     RVE's persistent state (displacements, coordinates, volume, last stress)
     is exported to host memory and the page's device memory is freed. A
@@ -189,7 +197,7 @@ class PagedRVEServer:
         self.precision, self.device, self.idle_us = precision, device, idle_timeout_us
         self.pages = [list(range(i, min(i + page_size, self.n)))
                       for i in range(0, self.n, page_size)]
-        self.page_bytes = [device_bytes_estimate([self.networks[r] for r in pg], precision)
+        self.page_bytes = [server_bytes_estimate([self.networks[r] for r in pg], precision)
                            for pg in self.pages]
         self.budget = float(hbm_budget_bytes)
         if max(self.page_bytes) > self.budget:
