@@ -493,8 +493,13 @@ mfg_status plan_f64_clusters(mfg_batch* b, const std::vector<double>& m,
       len[e] = {l0[i], mfg::bits_of(l0[et + i])};
     }
   });
-  mfg_status st = upload(b->d_plan, blob, s);
-  if (st != MFG_OK) return st;
+  const cudaError_t e = b->d_plan.alloc(bytes);
+  if (e == cudaErrorMemoryAllocation) {  // every RVE on one CTA: no more than it needs
+    cudaGetLastError();
+    return MFG_OK;
+  }
+  MFG_CUDA(e);
+  MFG_CUDA(cudaMemcpyAsync(b->d_plan.p, blob.data(), bytes, cudaMemcpyHostToDevice, s));
   MFG_CUDA(cudaStreamSynchronize(s));  // the blob goes out of scope
   mfg::F64Plan& plan = b->f64_plan;
   plan.cl = cl;

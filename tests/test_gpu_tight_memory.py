@@ -1,0 +1,80 @@
+"""A device with room for a batch but not for what only speeds it up: the batch
+is created and solves with the same bits. Device memory is not used up for
+this: the library is linked once more from its objects, with a cudaMalloc that
+fails above a budget."""
+import os
+import subprocess
+import sys
+
+import pytest
+
+HERE = os.path.dirname(os.path.abspath(__file__))
+ROOT = os.path.dirname(HERE)
+
+pytestmark = pytest.mark.gpu
+
+PRELUDE = """
+import ctypes, sys
+import numpy as np
+import mumfim_gb300 as m
+from mumfim_gb300 import batched, synthetic as S
+L = batched.load_library(sys.argv[1])
+L.fake_memory_held.restype = ctypes.c_size_t
+L.fake_memory_more.argtypes = [ctypes.c_size_t]
+NO_LIMIT = 2 ** 62
+F = np.array([[1.02, 0.01, 0.0], [0.0, 0.99, 0.01], [0.01, 0.0, 1.01]])[None]
+
+def networks(sizes):
+    return [m.FiberNetwork(*S.knn_network(n, 4, S.geometry_seed(67, i)),
+                           [S._linear_params(67, i)]) for i, n in enumerate(sizes)]
+
+def batch(sizes, precision, steps=120, **options):
+    before = L.fake_memory_held()
+    g = m.BatchedFiberRVEAnalysisExplicit(networks(sizes), [m.SolutionStrategy.ramp(steps, 0.5)]
+                                          * len(sizes), precision=precision, **options)
+    return g, L.fake_memory_held() - before
+
+def stress(g, n):
+    s = np.zeros((n, 6))
+    assert g.run(F, s)
+    return s
+"""
+
+F64_PLAN = PRELUDE + """
+sizes = (300, 1_100, 2_000)
+g, wide = batch(sizes, "f64")
+want = stress(g, 3)
+g.close()
+g, narrow = batch(sizes, "f64", serving_layout=True)
+g.close()
+assert narrow < wide
+L.fake_memory_more(narrow)
+g, taken = batch(sizes, "f64")
+assert taken == narrow
+np.testing.assert_array_equal(stress(g, 3), want)
+"""
+
+
+@pytest.fixture(scope="module")
+def limited_library(lib_path, tmp_path_factory):
+    from mumfim_gb300.build import ARCH, OBJ_DIR, SOURCES, _cuda_home
+    cuda = _cuda_home()
+    d = tmp_path_factory.mktemp("tight")
+    wrap, lib = str(d / "fake_memory.o"), str(d / "libmumfim_gpu_limited.so")
+    subprocess.run(["g++", "-O1", "-std=c++17", "-fPIC", "-I" + os.path.join(cuda, "include"),
+                    "-c", os.path.join(HERE, "native", "fake_memory.cpp"), "-o", wrap], check=True)
+    objs = [os.path.join(OBJ_DIR, name + ".o") for name, _, _ in SOURCES]
+    subprocess.run([os.path.join(cuda, "bin", "nvcc"), *ARCH, "-shared", "-cudart", "static",
+                    "-Xlinker", "--wrap=cudaMalloc", "-Xlinker", "--wrap=cudaFree", *objs, wrap,
+                    "-o", lib, "-lpthread", "-ldl", "-lrt"], check=True)
+    return lib
+
+
+def _run(script, library):
+    r = subprocess.run([sys.executable, "-c", script, library], cwd=ROOT, capture_output=True,
+                       text=True, timeout=300)
+    assert r.returncode == 0, r.stdout + r.stderr
+
+
+def test_f64_batch_without_room_for_clusters(limited_library):
+    _run(F64_PLAN, limited_library)
