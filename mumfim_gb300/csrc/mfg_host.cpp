@@ -284,6 +284,13 @@ struct StiffSlots {
   }
 };
 
+// The networks' fiber ends and CSR rows, kept on the host until the concurrent
+// stiffness solves' own working set is made from them.
+struct StiffInputs {
+  std::vector<int2> conn;
+  std::vector<int32_t> rowptr, inc;
+};
+
 // The six perturbation gradients of the FD stiffness, row-major, h = 1e-5
 // (BatchedFiberRVEAnalysisExplicit.h:331-395).
 constexpr double kStiffH = 1E-5;
@@ -342,9 +349,13 @@ struct mfg_batch {
   bool f64_stiffness_clusters = false;
   DevArray<unsigned char> d_plan;
   std::unique_ptr<mfg::MixedState, mfg::MixedStateDeleter> mixed;
-  // the concurrent stiffness solves' own working set, when six solves at
-  // once fill the GPU where one leaves SMs idle and so takes wider clusters
+  // The concurrent stiffness solves' own working set, when six solves at once
+  // fill the GPU where one leaves SMs idle and so takes wider clusters; made
+  // by the first stiffness (stiff_state_ready) from the inputs kept until then,
+  // null where they share `mixed`.
   std::unique_ptr<mfg::MixedState, mfg::MixedStateDeleter> mixed_stiff;
+  std::unique_ptr<StiffInputs> stiff_inputs;
+  mfg_options opt{};
   int stiffness = MFG_STIFFNESS_AUTO;
   bool all_ramp = false;
   StiffSlots stiff;
@@ -540,6 +551,20 @@ cudaError_t launch_f64(const mfg_batch* b, const mfg::DevBatch& dev, const mfg::
   return mfg::launch_relax_f64(dev, a, 0, grid, s);
 }
 
+// The batch's mixed-precision working set for `copies` solves at once.
+cudaError_t make_mixed(const mfg_batch& b,
+                       std::unique_ptr<mfg::MixedState, mfg::MixedStateDeleter>& state,
+                       const std::vector<int2>& conn, const std::vector<int32_t>& rowptr,
+                       const std::vector<int32_t>& inc, int copies) {
+  state.reset(mfg::mixed_new());
+  if (!state) return cudaErrorMemoryAllocation;
+  return mfg::mixed_create(*state, b.dev, b.desc, conn, rowptr, inc, b.sms,
+                           b.opt.max_cluster_ctas > 0 ? b.opt.max_cluster_ctas : 16,
+                           b.opt.cluster_layout == MFG_LAYOUT_SERVING, b.opt.small_rve_solve,
+                           b.opt.small_rves_per_cta > 0 ? b.opt.small_rves_per_cta : 2, copies,
+                           b.stream);
+}
+
 mfg_status enqueue_run(mfg_batch* b, const double* F_dev, int32_t n_F, double* sigma_dev,
                        int32_t update_coords, cudaStream_t s) {
   MFG_CUDA(cudaMemsetAsync(b->d_queue.p, 0, sizeof(int32_t), s));
@@ -676,6 +701,7 @@ static mfg_status batch_create_impl(const mfg_network* nets, const mfg_strategy*
   b->device = opt.device;
   b->precision = opt.precision;
   b->stiffness = opt.stiffness;
+  b->opt = opt;
   b->all_ramp = true;
   for (int r = 0; r < n_rve; ++r) b->all_ramp = b->all_ramp && strategies[r].mode == MFG_MODE_RAMP;
   b->R = n_rve;
@@ -839,24 +865,13 @@ static mfg_status batch_create_impl(const mfg_network* nets, const mfg_strategy*
       return st;
   }
   if (b->precision == MFG_PREC_MIXED) {
-    auto make = [&](std::unique_ptr<mfg::MixedState, mfg::MixedStateDeleter>& state, int copies) {
-      state.reset(mfg::mixed_new());
-      return state ? mfg::mixed_create(*state, dv, b->desc, conn, rowptr, inc, b->sms,
-                                       opt.max_cluster_ctas > 0 ? opt.max_cluster_ctas : 16,
-                                       opt.cluster_layout == MFG_LAYOUT_SERVING,
-                                       opt.small_rve_solve,
-                                       opt.small_rves_per_cta > 0 ? opt.small_rves_per_cta : 2,
-                                       copies, s)
-                   : cudaErrorMemoryAllocation;
-    };
-    cudaError_t e = make(b->mixed, 1);
-    if (e == cudaSuccess && mfg::mixed_widened(*b->mixed) &&
-        opt.stiffness != MFG_STIFFNESS_SEQUENTIAL &&
-        (b->all_ramp || opt.stiffness == MFG_STIFFNESS_CONCURRENT))
-      e = make(b->mixed_stiff, kStiffSlots);
+    const cudaError_t e = make_mixed(*b, b->mixed, conn, rowptr, inc, 1);
     if (e != cudaSuccess)
       return fail(e == cudaErrorMemoryAllocation ? MFG_E_OOM : MFG_E_CUDA,
                   "mixed-precision set-up failed: %s", cudaGetErrorString(e));
+    if (mfg::mixed_widened(*b->mixed) && opt.stiffness != MFG_STIFFNESS_SEQUENTIAL &&
+        (b->all_ramp || opt.stiffness == MFG_STIFFNESS_CONCURRENT))
+      b->stiff_inputs.reset(new StiffInputs{std::move(conn), std::move(rowptr), std::move(inc)});
   }
   MFG_CUDA(cudaStreamSynchronize(s));
   *out = b.release();
@@ -980,6 +995,18 @@ static mfg_status batch_run_impl(mfg_batch* b, const double* F, int32_t n_F, dou
 
 namespace {
 
+// The concurrent stiffness solves' own working set with its run contexts;
+// without the memory for it the solves share the batch's.
+cudaError_t stiff_state_ready(mfg_batch* b) {
+  const std::unique_ptr<StiffInputs> in = std::move(b->stiff_inputs);
+  cudaError_t e = make_mixed(*b, b->mixed_stiff, in->conn, in->rowptr, in->inc, kStiffSlots);
+  if (e == cudaSuccess) e = mfg::mixed_prepare_contexts(*b->mixed_stiff, b->dev, kStiffSlots);
+  if (e != cudaSuccess) b->mixed_stiff.reset();
+  if (e != cudaErrorMemoryAllocation) return e;
+  cudaGetLastError();
+  return cudaSuccess;
+}
+
 // Allocates the concurrent stiffness solves' scratch on first use.
 mfg_status stiff_slots_ready(mfg_batch* b) {
   StiffSlots& sl = b->stiff;
@@ -1000,9 +1027,9 @@ mfg_status stiff_slots_ready(mfg_batch* b) {
     if (e == cudaSuccess) e = cudaEventCreateWithFlags(&sl.join[k], cudaEventDisableTiming);
   }
   if (e == cudaSuccess) e = cudaEventCreateWithFlags(&sl.fork, cudaEventDisableTiming);
-  if (e == cudaSuccess && b->precision == MFG_PREC_MIXED)
-    e = mfg::mixed_prepare_contexts(b->mixed_stiff ? *b->mixed_stiff : *b->mixed, b->dev,
-                                    kStiffSlots);
+  if (e == cudaSuccess && b->stiff_inputs) e = stiff_state_ready(b);
+  if (e == cudaSuccess && b->precision == MFG_PREC_MIXED && !b->mixed_stiff)
+    e = mfg::mixed_prepare_contexts(*b->mixed, b->dev, kStiffSlots);
   if (e != cudaSuccess) {
     sl.release();
     return fail(e == cudaErrorMemoryAllocation ? MFG_E_OOM : MFG_E_CUDA,

@@ -28,7 +28,8 @@ constexpr int kMixedContexts = 7;
 // the RVEs whose node state fits one CTA; with the fiber-centric one, up to
 // rves_per_cta (1 or 2) small RVEs share a CTA. A batch that leaves SMs idle
 // with `copies` solves of it at once takes wider clusters (up to max_cluster,
-// 16 at most), with the same results.
+// 16 at most), with the same results; with copies > 1 the state has no context
+// 0 (mixed_prepare_contexts makes the others).
 cudaError_t mixed_create(MixedState& ms, const DevBatch& b, const std::vector<RveDesc>& desc,
                          const std::vector<int2>& conn, const std::vector<int32_t>& rowptr,
                          const std::vector<int32_t>& inc, int sms, int max_cluster,

@@ -1812,8 +1812,10 @@ cudaError_t mixed_create(MixedState& ms, const DevBatch& b, const std::vector<Rv
   // The arrays whose sizes are known, in one allocation. The node records,
   // velocities and force vectors in global memory are the run-time
   // placement's, which the serving kernels may take for an RVE of any bucket.
-  const bool scratch = serving_layout || (!bucket[kQRuntime].empty() &&
-                                          ms.bucket_kind[kQRuntime] == kQRuntime);
+  // Several solves at once run on contexts 1, 2, ..., which have their own.
+  const bool scratch = copies == 1 &&
+                       (serving_layout || (!bucket[kQRuntime].empty() &&
+                                           ms.bucket_kind[kQRuntime] == kQRuntime));
   Arena arena;
   if (scratch) {
     arena.add(&ms.u_hl, 6 * nt);
@@ -1956,7 +1958,7 @@ cudaError_t mixed_create(MixedState& ms, const DevBatch& b, const std::vector<Rv
   std::stable_sort(ms.launch_order, ms.launch_order + kBuckets, [&](int x, int y) {
     return kKind[ms.bucket_kind[x]].cl > kKind[ms.bucket_kind[y]].cl;
   });
-  if ((e = ctx_init(ms, ms.ctx[0], nt, et, false)) != cudaSuccess) return e;
+  if (copies == 1 && (e = ctx_init(ms, ms.ctx[0], nt, et, false)) != cudaSuccess) return e;
 
   const int64_t n = std::max<int64_t>(b.nt, 1);
   mixed_prepare_kernel<<<static_cast<unsigned>((n + 255) / 256), 256, 0, s>>>(b, ms);

@@ -13,7 +13,7 @@ cudaError_t __real_cudaFree(void* p);
 
 static std::mutex mtx;
 static std::map<void*, size_t> held;
-static size_t total = 0, budget = ~static_cast<size_t>(0);
+static size_t total = 0, peak = 0, budget = ~static_cast<size_t>(0);
 
 cudaError_t __wrap_cudaMalloc(void** p, size_t n) {
   std::lock_guard<std::mutex> lock(mtx);
@@ -22,6 +22,7 @@ cudaError_t __wrap_cudaMalloc(void** p, size_t n) {
   if (e == cudaSuccess) {
     held[*p] = n;
     total += n;
+    if (total > peak) peak = total;
   }
   return e;
 }
@@ -37,5 +38,10 @@ cudaError_t __wrap_cudaFree(void* p) {
 }
 
 size_t fake_memory_held() { return total; }
+size_t fake_memory_peak() {  // the most held since the last call
+  const size_t most = peak;
+  peak = total;
+  return most;
+}
 void fake_memory_more(size_t n) { budget = total + n; }  // what may still be allocated
 }

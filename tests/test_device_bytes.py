@@ -40,7 +40,7 @@ def test_batches_take_no_more_than_their_estimate(lib_path, precision, n, nodes)
     def make(nets):
         g = m.BatchedFiberRVEAnalysisExplicit(nets, [m.SolutionStrategy.ramp(5, 0.5)] * len(nets),
                                               precision=precision)
-        g.run(F)
+        g.run(F, update_coords=False)
         return g
 
     nets = _networks(n, nodes)

@@ -19,7 +19,7 @@ import numpy as np
 import mumfim_gb300 as m
 from mumfim_gb300 import batched, synthetic as S
 L = batched.load_library(sys.argv[1])
-L.fake_memory_held.restype = ctypes.c_size_t
+L.fake_memory_held.restype = L.fake_memory_peak.restype = ctypes.c_size_t
 L.fake_memory_more.argtypes = [ctypes.c_size_t]
 NO_LIMIT = 2 ** 62
 F = np.array([[1.02, 0.01, 0.0], [0.0, 0.99, 0.01], [0.01, 0.0, 1.01]])[None]
@@ -36,7 +36,7 @@ def batch(sizes, precision, steps=120, **options):
 
 def stress(g, n):
     s = np.zeros((n, 6))
-    assert g.run(F, s)
+    assert g.run(np.repeat(F, n, axis=0), s)
     return s
 """
 
@@ -52,6 +52,37 @@ L.fake_memory_more(narrow)
 g, taken = batch(sizes, "f64")
 assert taken == narrow
 np.testing.assert_array_equal(stress(g, 3), want)
+"""
+
+MIXED_STIFFNESS = PRELUDE + """
+sizes = (500, 900, 1_300, 2_500, 4_000, 6_000, 9_000, 15_000) * 2
+n = len(sizes)
+L.fake_memory_peak()
+g, plain = batch(sizes, "mixed", stiffness="sequential")
+want = stress(g, n)
+g.close()
+# no memory for a second working set before a stiffness asks for one
+L.fake_memory_more(L.fake_memory_peak() - L.fake_memory_held())
+g, taken = batch(sizes, "mixed")
+assert taken == plain
+np.testing.assert_array_equal(stress(g, n), want)
+L.fake_memory_more(NO_LIMIT)
+C = g.computeMaterialStiffness()
+with_own = L.fake_memory_held()
+np.testing.assert_array_equal(g.computeMaterialStiffness(), C)
+assert L.fake_memory_held() == with_own
+g.close()
+start = L.fake_memory_held()
+# nor later: one byte too few for it, and the six solves share the batch's
+g, _ = batch(sizes, "mixed")
+stress(g, n)
+L.fake_memory_more(with_own - L.fake_memory_held() - 1)
+np.testing.assert_array_equal(g.computeMaterialStiffness(), C)
+assert start < L.fake_memory_held() < with_own
+np.testing.assert_array_equal(g.computeMaterialStiffness(), C)
+L.fake_memory_more(NO_LIMIT)
+stress(g, n)
+assert np.isfinite(g.computeMaterialStiffness()).all()
 """
 
 
@@ -78,3 +109,7 @@ def _run(script, library):
 
 def test_f64_batch_without_room_for_clusters(limited_library):
     _run(F64_PLAN, limited_library)
+
+
+def test_mixed_batch_without_room_for_a_second_working_set(limited_library):
+    _run(MIXED_STIFFNESS, limited_library)
