@@ -3,15 +3,17 @@
 The mixed solve places each RVE by rule: the smallest single CTA or
 thread-block cluster (2, 4, then 8 CTAs) whose shared memory holds the
 RVE's node state (node-centric solve), else one CTA streaming from global
-memory; on request, RVEs whose whole state fits one CTA (or half of one,
-two per CTA) take the fiber-centric solve first. Which shapes pay depends
+memory; a batch that leaves SMs idle, or has RVEs too large for 8 CTAs, takes
+wider clusters, up to 16 CTAs, unless a limit is set; on request, RVEs whose
+whole state fits one CTA (or half of one, two per CTA) take the fiber-centric
+solve first. Which shapes pay depends
 on the GPU and on the size mix: a cluster trades barrier and
 distributed-shared-memory costs for on-chip state, how many clusters of a
 size stay resident varies, and the fiber-centric solve of small RVEs trades
 half the fiber arithmetic against a stored force vector per fiber and a
 second pass. The tuner times short solves of a size-stratified sample of
 the batch under every candidate shape -- the largest cluster allowed
-(``max_cluster_ctas``), clusters of 4 instead of 2 (the serving layout) and
+(``max_cluster_ctas``; 0 sets no limit), clusters of 4 instead of 2 (the serving layout) and
 the solve of small RVEs (node-centric, or fiber-centric two per CTA) -- and
 keeps the fastest. Every candidate gives the same bits, so only the speed
 differs.
@@ -37,7 +39,7 @@ _PKG = os.path.dirname(os.path.abspath(__file__))
 
 @dataclasses.dataclass(frozen=True)
 class LaunchShape:
-    max_cluster_ctas: int = 0     # 1, 2, 4 or 8 (0 = 8)
+    max_cluster_ctas: int = 0     # 1, 2, 4 or 8 (0 = as many as pay, up to 16)
     serving_layout: bool = False  # clusters of 4 where the batch layout takes 2
     small_rves_per_cta: int = 0   # fiber-centric small solve: 1 or 2 (0 = 2)
     small_rve_solve: str = "auto"  # "auto" (= "node"), "node" or "fiber"
@@ -48,13 +50,14 @@ class LaunchShape:
                     small_rve_solve=self.small_rve_solve)
 
 
-DEFAULT_SHAPE = LaunchShape(8, False, 0, "auto")
-CANDIDATES_VERSION = 3  # small solve: auto (by law), node- or fiber-centric
+DEFAULT_SHAPE = LaunchShape(0, False, 0, "auto")  # as a batch without options
+CANDIDATES_VERSION = 4  # clusters without a limit; wide, staged and split kinds
 
 
 def candidate_shapes(nonlinear_frac: float = 0.0) -> List[LaunchShape]:
-    """Every distinct shape: the serving layout only differs from the batch
-    layout when clusters of 4 are allowed; the small solve "auto" (node-
+    """Every distinct shape: no limit on the cluster size (clusters of 16 where
+    they pay or an RVE needs them), 4, 2 or 1; the serving layout only differs
+    from the batch layout when clusters of 4 are allowed; the small solve "auto" (node-
     centric on the linear law, fiber-centric on the nonlinear one) is tried
     beside whichever of "node" and "fiber" differs from it on this law mix,
     the fiber-centric one with two small RVEs per CTA (one per CTA measured
@@ -66,9 +69,9 @@ def candidate_shapes(nonlinear_frac: float = 0.0) -> List[LaunchShape]:
         solves.append(("fiber", 2))
     out = []
     for solve, per_cta in solves:
-        for mc in (8, 4, 2, 1):
+        for mc in (0, 4, 2, 1):
             out.append(LaunchShape(mc, False, per_cta, solve))
-            if mc >= 4:
+            if mc in (0, 4):
                 out.append(LaunchShape(mc, True, per_cta, solve))
     return out
 
@@ -175,10 +178,10 @@ def tune_launch_shape(networks: Sequence, strategies: Sequence, F, steps: int = 
 
 
 def tune_cluster_limit(networks: Sequence, strategies: Sequence, F, steps: int = 100,
-                       candidates: Sequence[int] = (1, 2, 4, 8), repeats: int = 2,
+                       candidates: Sequence[int] = (1, 2, 4, 8, 0), repeats: int = 2,
                        device: int = 0) -> Tuple[int, Dict[int, float]]:
-    """The cluster-size limit alone, on the whole batch: (fastest limit,
-    {limit: fiber-steps/s})."""
+    """The cluster-size limit alone (0: none), on the whole batch: (fastest
+    limit, {limit: fiber-steps/s})."""
     strat = [SolutionStrategy.ramp(steps, s.visc_damp_coeff, s.crit_time_scale_factor)
              for s in strategies]
     F = np.ascontiguousarray(F, dtype=np.float64).reshape(len(networks), 3, 3)
