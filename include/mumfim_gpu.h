@@ -117,10 +117,9 @@ typedef struct mfg_options {
   int32_t precision;        /* mfg_precision */
   int32_t device;           /* CUDA device ordinal */
   int32_t threads_per_rve;  /* ignored: the CTA size is fixed per precision */
-  int32_t max_cluster_ctas; /* mixed precision: largest thread-block cluster an RVE
-                               may be split over (1, 2, 4 or 8; 0 = as many as pay,
-                               up to 16). 1 solves every RVE on one CTA, with the
-                               same results. */
+  int32_t max_cluster_ctas; /* largest thread-block cluster an RVE may be split over
+                               (1, 2, 4 or 8; 0 = as many as pay, up to 16). 1 solves
+                               every RVE on one CTA, with the same results. */
   int32_t cluster_layout;   /* mfg_cluster_layout. Mixed precision: MFG_LAYOUT_SERVING
                                places RVEs that need a cluster, and those that end a
                                wave of requests sooner there, on clusters of 4 (never

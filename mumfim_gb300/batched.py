@@ -119,7 +119,7 @@ class BatchedFiberRVEAnalysisExplicit:
     networks    sequence of network_io.FiberNetwork (reaction 0 drives the solve)
     strategies  one strategy.SolutionStrategy per network
     precision   "f64" (bit-identical to a serial CPU run) or "mixed"
-    max_cluster_ctas  mixed precision: largest thread-block cluster an RVE may be
+    max_cluster_ctas  largest thread-block cluster an RVE may be
                 split over (1, 2, 4 or 8; 0 = as many as pay, up to 16); results do
                 not depend on it
     serving_layout  the layout the serving kernel uses. Mixed precision: RVEs that

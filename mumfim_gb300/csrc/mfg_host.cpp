@@ -426,7 +426,8 @@ mfg_status plan_f64_clusters(mfg_batch* b, const std::vector<double>& m,
                              cudaStream_t s) {
   int clusters[5] = {b->sms, 0, 0, 0, 0};
   for (int k = 1; k < 5; ++k)
-    clusters[k] = mfg::relax_f64_max_clusters(1 << k, mfg::kF64ClusterSmem, b->sms);
+    if (b->opt.max_cluster_ctas == 0 || 1 << k <= b->opt.max_cluster_ctas)
+      clusters[k] = mfg::relax_f64_max_clusters(1 << k, mfg::kF64ClusterSmem, b->sms);
   const int64_t nt = b->nt, et = b->et;
   std::vector<mfg::F64Parts> parts(b->R);  // per RVE, offsets from its own start
   int cl = 1;

@@ -1,7 +1,7 @@
 """A device with room for a batch but not for what only speeds it up: the batch
 is created and solves with the same bits. Device memory is not used up for
 this: the library is linked once more from its objects, with a cudaMalloc that
-fails above a budget."""
+fails above a budget and counts what is held."""
 import os
 import subprocess
 import sys
@@ -52,6 +52,22 @@ L.fake_memory_more(narrow)
 g, taken = batch(sizes, "f64")
 assert taken == narrow
 np.testing.assert_array_equal(stress(g, 3), want)
+"""
+
+F64_LIMIT = PRELUDE + """
+sizes = (300, 1_100, 2_000)
+g, narrow = batch(sizes, "f64", serving_layout=True)
+want = stress(g, 3)
+C = g.computeMaterialStiffness()
+g.close()
+held = {}
+for limit in (1, 2, 8, 0):
+    g, held[limit] = batch(sizes, "f64", max_cluster_ctas=limit)
+    np.testing.assert_array_equal(stress(g, 3), want)
+    np.testing.assert_array_equal(g.computeMaterialStiffness(), C)
+    g.close()
+# a limit of 1 keeps no parts; wider parts share more fibers, and so take more
+assert narrow == held[1] < held[2] < held[8] < held[0]
 """
 
 MIXED_STIFFNESS = PRELUDE + """
@@ -109,6 +125,10 @@ def _run(script, library):
 
 def test_f64_batch_without_room_for_clusters(limited_library):
     _run(F64_PLAN, limited_library)
+
+
+def test_f64_clusters_keep_to_the_limit(limited_library):
+    _run(F64_LIMIT, limited_library)
 
 
 def test_mixed_batch_without_room_for_a_second_working_set(limited_library):
