@@ -583,19 +583,27 @@ __device__ __forceinline__ void mixed_stress(const DevBatch& b, const RunArgs& a
     const double* xj = b.x + cj * nt + no;
     const double* fi = b.fint + ci * nt + no;
     const double* fj = b.fint + cj * nt + no;
-    // virtual thread t + j kSize sums q = t + j kSize + m kThreadsMixed
+    // virtual thread t + j kSize sums q = t + j kSize + m kThreadsMixed; every
+    // rounding written out, and no more of them than the sum needs: the kernels
+    // that compile it would each contract it in a way of their own
     double acc[NG];
 #pragma unroll
     for (int j = 0; j < NG; ++j) acc[j] = 0.0;
-    for (int q = tid, j = 0; q < nb; q += Group<NG>::kSize, j = (j + 1 == NG ? 0 : j + 1)) {
-      const int i = bo[q];
-      // every rounding written out: the kernels that compile this sum would
-      // each contract it in a way of their own
-      const double t = k < 3 ? __dmul_rn(xi[i], fi[i])
-                             : 0.5 * __fma_rn(xj[i], fi[i], __dmul_rn(xi[i], fj[i]));
+    if (k < 3) {
+      for (int q = tid, j = 0; q < nb; q += Group<NG>::kSize, j = (j + 1 == NG ? 0 : j + 1)) {
+        const int i = bo[q];
 #pragma unroll
-      for (int jj = 0; jj < NG; ++jj)
-        if (jj == j) acc[jj] = __dadd_rn(acc[jj], t);
+        for (int jj = 0; jj < NG; ++jj)
+          if (jj == j) acc[jj] = __fma_rn(xi[i], fi[i], acc[jj]);
+      }
+    } else {
+      for (int q = tid, j = 0; q < nb; q += Group<NG>::kSize, j = (j + 1 == NG ? 0 : j + 1)) {
+        const int i = bo[q];
+        const double t = 0.5 * __fma_rn(xi[i], fj[i], __dmul_rn(xj[i], fi[i]));
+#pragma unroll
+        for (int jj = 0; jj < NG; ++jj)
+          if (jj == j) acc[jj] = __dadd_rn(acc[jj], t);
+      }
     }
     const double sk = group_sum<NG>(acc, red) * sc;
     bad = bad || !isfinite(sk);
