@@ -84,13 +84,15 @@ constexpr int kMulF64 = 2, kMulCluster = 2, kMulSmall = 0;
 struct LawF64 {
   bool nonlinear;
   bool exact;  // E A (half_E, below) and alpha (div_known) are far from underflow
-  double half_E, A;  // half_E = E / 2: the linear law's factor 1/2, moved to where it is exact
+  double E, A;
+  double half_E;  // E / 2: the linear law's factor 1/2, moved to where it is exact (with `exact`)
   double alpha, B, lt, kt, bt, kc, bc;
 };
 
 __device__ __forceinline__ LawF64 make_law_f64(const RveDesc& d) {
   LawF64 L;
   L.nonlinear = d.law == 1;
+  L.E = d.E;
   L.half_E = 0.5 * d.E;
   L.A = d.A;
   L.alpha = L.B = L.lt = L.kt = L.bt = L.kc = L.bc = 0.0;
@@ -140,7 +142,7 @@ __device__ __noinline__ double fiber_vector_general(const LawF64& L, const doubl
   const double l = sqrt(d[0] * d[0] + d[1] * d[1] + d[2] * d[2]);
   const double lr = l / l0;
   const double T = L.nonlinear ? reaction_force(L, lr, l0, L.alpha / l0)
-                               : lr * (2.0 * L.half_E) * L.A * (0.5 * (lr * lr - 1));
+                               : lr * L.E * L.A * (0.5 * (lr * lr - 1));
   const double q = T / l;
   for (int k = 0; k < 3; ++k) n[k] = d[k] * q;
   return l;
