@@ -59,16 +59,16 @@ namespace {
 
 constexpr int kThreadsF64 = 512;
 constexpr int kSumThreads = 256;  // partial sums of the residual
-// Which products run in integers: 1 the force vector's three, 2 also the
-// squares of the length, 3 also the linear law's, 4 also the nodes'. An FP64
-// product costs 19 cycles of the SM's pipe, an integer one 30 issue slots, so
-// it pays where warps are many. 304 RVEs of 4,500 nodes on single CTAs, levels
-// 0, 2, 3, 4: 1.20, 1.51, 1.54, 1.50e10 fiber-steps/s, but 1.08, 1.26, 1.20,
-// 1.18e10 for 152 (one CTA an SM); clusters of 512 threads, 36 RVEs, levels 1,
-// 2, 3, 4: 34, 28, 30, 31 us a step. A small part's warps are few, and a step
-// is a chain: 4.0 us with level 2 at 512 threads for one RVE of 1,000 nodes,
-// 3.7 with level 0 at 256.
-constexpr int kMulF64 = 2, kMulCluster = 2, kMulSmall = 0;
+// Whether the products of the length's squares and of the force vector run in
+// integers. An FP64 product costs 19 cycles of the SM's pipe, an integer one 30
+// issue slots, so it pays where warps are many. Fiber-steps/s without, with
+// these, with the linear law's too, and with the nodes' too: 304 RVEs of 4,500
+// nodes on single CTAs 1.20, 1.51, 1.54, 1.50e10, but 1.08, 1.26, 1.20, 1.18e10
+// for 152 (one CTA an SM); 36 on clusters of 512 threads -, 28, 30, 31 us a step
+// (34 with the force vector's alone). A small part's warps are few, and a step is
+// a chain: 4.0 us with them at 512 threads for one RVE of 1,000 nodes, 3.7
+// without at 256.
+constexpr bool kIntF64 = true, kIntCluster = true, kIntSmall = false;
 
 // Reaction law of one RVE with everything that does not depend on the fiber
 // formed once, by the expressions the reference forms per fiber.
@@ -123,12 +123,10 @@ __device__ __forceinline__ double product(double a, double b) {
 
 // Force at length ratio lr of a fiber of reference length l0; alpha_l0 =
 // alpha / l0 (nonlinear law only).
-template <int kMul = 0>
 __device__ __forceinline__ double reaction_force(const LawF64& L, double lr, double l0,
                                                  double alpha_l0) {
   if (!L.nonlinear)
-    return product<(kMul > 2)>(product<(kMul > 2)>(product<(kMul > 2)>(lr, L.half_E), L.A),
-                               product<(kMul > 2)>(lr, lr) - 1);
+    return lr * L.half_E * L.A * (lr * lr - 1);
   if (lr > L.lt) return alpha_l0 * L.kt * (lr - L.lt) * l0 + L.bt;
   if (lr < 1.0) return alpha_l0 * L.kc * (lr - 1.0) * l0 + L.bc;
   const double gs = 1.0 / 2.0 * (lr * lr - 1);
@@ -150,24 +148,24 @@ __device__ __noinline__ double fiber_vector_general(const LawF64& L, const doubl
 
 // The same, with the square root and the quotients of mfg_exact.cuh (R0 =
 // exact_reciprocal(l0), 0 to ask for the general operations): 16 FP64
-// instructions on the linear law instead of 45 (10 with kMul = 2), the same
+// instructions on the linear law instead of 45 (10 with kInt), the same
 // bits.
-template <int kMul>
+template <bool kInt>
 __device__ __forceinline__ double fiber_vector(const LawF64& L, const double d[3], double l0,
                                                uint64_t R0, double n[3]) {
-  const double s = product<(kMul > 1)>(d[0], d[0]) + product<(kMul > 1)>(d[1], d[1]) +
-                   product<(kMul > 1)>(d[2], d[2]);
+  const double s =
+      product<kInt>(d[0], d[0]) + product<kInt>(d[1], d[1]) + product<kInt>(d[2], d[2]);
   if (L.exact && in_range(s) && R0 != 0) {
     double l;
     uint64_t R;
     if (sqrt_recip(s, rsqrt_start(root_operand(s)), l, R)) {
-      const double T = reaction_force<kMul>(L, div_known(l, l0, R0), l0,
+      const double T = reaction_force(L, div_known(l, l0, R0), l0,
                                       L.nonlinear ? div_known(L.alpha, l0, R0) : 0.0);
       const bool zero = is_zero(T);
       if (zero || in_range(T)) {
         const double q = zero ? T : div_root(T, l, R);
 #pragma unroll
-        for (int k = 0; k < 3; ++k) n[k] = product<(kMul > 0)>(d[k], q);
+        for (int k = 0; k < 3; ++k) n[k] = product<kInt>(d[k], q);
         return l;
       }
     }
@@ -263,7 +261,7 @@ __device__ __forceinline__ double fiber_pass(const RveView& r, const RveDesc& d,
     const int2 c = __ldg(r.conn + e);
     const double dv[3] = {r.x0[c.y] - r.x0[c.x], r.x1[c.y] - r.x1[c.x], r.x2[c.y] - r.x2[c.x]};
     double n[3];
-    const double l = fiber_vector<kMulF64>(L, dv, __ldg(r.l0 + e), __ldg(r.rl0 + e), n);
+    const double l = fiber_vector<kIntF64>(L, dv, __ldg(r.l0 + e), __ldg(r.rl0 + e), n);
     if (kLen) lmin = fmin(lmin, l);
     r.n0[e] = n[0];
     r.n1[e] = n[1];
@@ -278,11 +276,10 @@ __device__ __forceinline__ double fiber_pass(const RveView& r, const RveDesc& d,
 // Between refreshes of the time step both half kicks add the same quotient
 // h f / m, formed once
 // (`same`).
-template <int kMul>
 __device__ __forceinline__ void kick(double a, double m, uint64_t rm, double mc, double h_prev,
                                      double h, bool first, bool same, double& w) {
-  const double f = -(a + product<(kMul > 3)>(mc, w));  // f = -f_int - c m v
-  const double q = over_mass(product<(kMul > 3)>(h, f), m, rm);
+  const double f = -(a + mc * w);  // f = -f_int - c m v
+  const double q = over_mass(h * f, m, rm);
   if (!first) w += same ? q : over_mass(h_prev * f, m, rm);
   w += q;
 }
@@ -419,13 +416,13 @@ __device__ void solve_rve(const DevBatch& b, const RunArgs& a, int rve, double* 
       const double mass = __ldg(r.m + i), mc = __ldg(r.mc + i);
       const uint64_t rm = __ldg(r.rm + i);
       double w0 = r.v0[i], w1 = r.v1[i], w2 = r.v2[i];
-      kick<kMulF64>(a0, mass, rm, mc, h_prev, h, step == 0, same, w0);
-      kick<kMulF64>(a1, mass, rm, mc, h_prev, h, step == 0, same, w1);
-      kick<kMulF64>(a2, mass, rm, mc, h_prev, h, step == 0, same, w2);
+      kick(a0, mass, rm, mc, h_prev, h, step == 0, same, w0);
+      kick(a1, mass, rm, mc, h_prev, h, step == 0, same, w1);
+      kick(a2, mass, rm, mc, h_prev, h, step == 0, same, w2);
       r.v0[i] = w0; r.v1[i] = w1; r.v2[i] = w2;
-      r.x0[i] = r.x0[i] + product<(kMulF64 > 3)>(h2, w0);
-      r.x1[i] = r.x1[i] + product<(kMulF64 > 3)>(h2, w1);
-      r.x2[i] = r.x2[i] + product<(kMulF64 > 3)>(h2, w2);
+      r.x0[i] = r.x0[i] + h2 * w0;
+      r.x1[i] = r.x1[i] + h2 * w1;
+      r.x2[i] = r.x2[i] + h2 * w2;
     }
     if (ramp) {
       const double alpha = div_known(done + 1.0, cap_d, d.r_steps);
@@ -512,7 +509,6 @@ __global__ void __launch_bounds__(kThreadsF64, 2) server_f64_kernel(const DevBat
 // copied into shared memory as far as it fits: the barrier's acquire drops
 // the L1 cache, and a step of a small part is a chain of loads.
 
-template <int CL>
 struct ClusterX {
   uint32_t base;     // shared address of the copy being read, in this CTA
   uint32_t stride;   // bytes from one component to the next
@@ -554,7 +550,7 @@ __device__ __forceinline__ const T* stage(const T* src, int n, unsigned char*& a
   return dst;
 }
 
-template <int CL, int NT, int kMul>
+template <int CL, int NT, bool kInt>
 __device__ void solve_rve_cluster(const DevBatch& b, const RunArgs& a, const F64Plan& plan,
                                   int rve, double* red, double* cred, double* alpha_s,
                                   double* terms,
@@ -628,7 +624,7 @@ __device__ void solve_rve_cluster(const DevBatch& b, const RunArgs& a, const F64
   }
   const uint32_t xs_addr = static_cast<uint32_t>(__cvta_generic_to_shared(xs));
   int cur = 0;  // the copy that holds the current positions
-  ClusterX<CL> x{xs_addr, 8u * static_cast<uint32_t>(S)};
+  ClusterX x{xs_addr, 8u * static_cast<uint32_t>(S)};
 
   // fiber pass over the part's fibers; with kLen also the shortest length,
   // for which the fibers between boundary nodes count too
@@ -643,7 +639,7 @@ __device__ void solve_rve_cluster(const DevBatch& b, const RunArgs& a, const F64
       x.load(c.x, xa);
       x.load(c.y, xb);
       const double dv[3] = {xb[0] - xa[0], xb[1] - xa[1], xb[2] - xa[2]};
-      const double l = fiber_vector<kMul>(L, dv, q.l0, q.r, nv);
+      const double l = fiber_vector<kInt>(L, dv, q.l0, q.r, nv);
       if (kLen) {
         lmin = fmin(lmin, l);
         if (e >= part.n_fib) continue;
@@ -722,9 +718,9 @@ __device__ void solve_rve_cluster(const DevBatch& b, const RunArgs& a, const F64
         if (t < nfo) {
           const F64Mass mm = mass[t];
           double w = vel[k * nfo + t];
-          kick<kMul>(gather(t, k), mm.m, mm.rm, mm.mc, h_prev, h, step == 0, same, w);
+          kick(gather(t, k), mm.m, mm.rm, mm.mc, h_prev, h, step == 0, same, w);
           vel[k * nfo + t] = w;
-          xn[k * S + t] = xc[k * S + t] + product<(kMul > 3)>(h2, w);
+          xn[k * S + t] = xc[k * S + t] + h2 * w;
         }
       } else {
         const int q = item - 3 * W;
@@ -781,7 +777,7 @@ __device__ void solve_rve_cluster(const DevBatch& b, const RunArgs& a, const F64
 #pragma unroll
       for (int k = 0; k < 3; ++k)
         dv[k] = __ldcg(b.x + k * nt + no + c.y) - __ldcg(b.x + k * nt + no + c.x);
-      fiber_vector<0>(L, dv, b.l0[e], b.rl0[e], nv);
+      fiber_vector<false>(L, dv, b.l0[e], b.rl0[e], nv);
 #pragma unroll
       for (int k = 0; k < 3; ++k) f[k] = f[k] + flip_sign(nv[k], !(code & 1));
     }
@@ -792,7 +788,7 @@ __device__ void solve_rve_cluster(const DevBatch& b, const RunArgs& a, const F64
   if (rank == 0) cauchy_stress<NT>(b, a, d, rve, status, step, residual, terms);
 }
 
-template <int CL, int NT, int kMul>
+template <int CL, int NT, bool kInt>
 __global__ void __launch_bounds__(NT, 1)
 relax_f64_cluster_kernel(const DevBatch b, const RunArgs a, const F64Plan plan) {
   extern __shared__ double4 smem_f64[];
@@ -810,20 +806,20 @@ relax_f64_cluster_kernel(const DevBatch b, const RunArgs a, const F64Plan plan) 
     const int rve = *cluster.map_shared_rank(&s_rve, 0);
     cluster.sync();  // also: no CTA overwrites what a slower one still reads
     if (rve < 0) break;
-    solve_rve_cluster<CL, NT, kMul>(b, a, plan, rve, red, &cred, &alpha, terms,
+    solve_rve_cluster<CL, NT, kInt>(b, a, plan, rve, red, &cred, &alpha, terms,
                           reinterpret_cast<unsigned char*>(smem_f64), plan.smem_bytes);
   }
 }
 
 using ClusterKernel = void (*)(DevBatch, RunArgs, F64Plan);
 
-template <int NT, int kMul>
+template <int NT, bool kInt>
 ClusterKernel cluster_kernel_of(int cl) {
   switch (cl) {
-    case 2: return relax_f64_cluster_kernel<2, NT, kMul>;
-    case 4: return relax_f64_cluster_kernel<4, NT, kMul>;
-    case 8: return relax_f64_cluster_kernel<8, NT, kMul>;
-    case 16: return relax_f64_cluster_kernel<16, NT, kMul>;
+    case 2: return relax_f64_cluster_kernel<2, NT, kInt>;
+    case 4: return relax_f64_cluster_kernel<4, NT, kInt>;
+    case 8: return relax_f64_cluster_kernel<8, NT, kInt>;
+    case 16: return relax_f64_cluster_kernel<16, NT, kInt>;
     default: return nullptr;
   }
 }
@@ -831,8 +827,8 @@ ClusterKernel cluster_kernel_of(int cl) {
 cudaError_t cluster_config(int cl, int threads, int grid, int smem_bytes, cudaStream_t s,
                            ClusterKernel* kernel, cudaLaunchConfig_t* cfg,
                            cudaLaunchAttribute* attr) {
-  *kernel = threads == kF64ClusterThreads ? cluster_kernel_of<kF64ClusterThreads, kMulCluster>(cl)
-                                          : cluster_kernel_of<kF64SmallThreads, kMulSmall>(cl);
+  *kernel = threads == kF64ClusterThreads ? cluster_kernel_of<kF64ClusterThreads, kIntCluster>(cl)
+                                          : cluster_kernel_of<kF64SmallThreads, kIntSmall>(cl);
   if (!*kernel) return cudaErrorInvalidValue;
   cudaError_t e = cudaFuncSetAttribute(*kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                        kF64ClusterSmem);
