@@ -101,25 +101,32 @@ MFG_HD int32_t exponent_bits(uint64_t u) { return static_cast<int32_t>(u >> 52) 
 // Reciprocal of a divisor for div_known(): floor(2^127 / D) for its
 // significand D at bit 63 (2^64 - 1 for a power of two), or 0 when the divisor
 // is outside 2^-100 .. 2^100 and its quotients need the general division.
-// Host set-up.
-inline uint64_t exact_reciprocal(double d) {
-  if (!(d >= std::ldexp(1.0, -100) && d <= std::ldexp(1.0, 100))) return 0;
-  uint64_t u;
-  std::memcpy(&u, &d, 8);
-  const uint64_t D = significand(u) << 11;
+// Set-up, on the device too.
+//
+// From the FP64 quotient, off by less than 2^12, and its exact remainder
+// 2^127 - R D in two words (a 128-bit division takes ten times as long): the
+// remainder over D corrects R to the last unit or the one beside it, and the
+// loops below settle that.
+MFG_HD uint64_t exact_reciprocal(double d) {
+  if (!(d >= 0x1p-100 && d <= 0x1p100)) return 0;
+  const uint64_t D = significand(bits_of(d)) << 11;
   if (D == 0x8000000000000000ull) return ~0ull;
-  // from the FP64 quotient, corrected by its exact remainder (a 128-bit
-  // division takes ten times as long)
-  using i128 = __int128;
   const double Df = static_cast<double>(D);  // exact: 53 bits
-  uint64_t R = static_cast<uint64_t>(std::ldexp(1.0, 127) / Df);
-  i128 rem = static_cast<i128>((static_cast<unsigned __int128>(1) << 127) -
-                               static_cast<unsigned __int128>(R) * D);
-  const int64_t step = static_cast<int64_t>(std::floor(static_cast<double>(rem) / Df));
-  R += static_cast<uint64_t>(step);
-  rem -= static_cast<i128>(step) * static_cast<i128>(D);
-  for (; rem < 0; rem += D) --R;
-  for (; rem >= static_cast<i128>(D); rem -= D) ++R;
+  uint64_t R = static_cast<uint64_t>(0x1p127 / Df);  // below 2^64 - 2^10: D is 2^63 + 2^11 or more
+  uint64_t lo = 0 - R * D;
+  int64_t hi = static_cast<int64_t>(0x8000000000000000ull - mul_high(R, D) - (R * D != 0));
+  const double rest = static_cast<double>(hi) * 0x1p64 + static_cast<double>(lo);
+  R += static_cast<uint64_t>(static_cast<int64_t>(floor(rest / Df)));
+  lo = 0 - R * D;
+  hi = static_cast<int64_t>(0x8000000000000000ull - mul_high(R, D) - (R * D != 0));
+  for (; hi < 0; --R) {  // remainder below 0: D more
+    lo += D;
+    hi += lo < D;
+  }
+  for (; hi > 0 || lo >= D; ++R) {
+    hi -= lo < D;
+    lo -= D;
+  }
   return R;
 }
 

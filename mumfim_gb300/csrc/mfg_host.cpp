@@ -409,26 +409,23 @@ mfg_status check_reaction(const mfg_reaction& rc, int r) {
   return MFG_OK;
 }
 
+// An array `times` as long as h on the device, h in front.
 template <typename T>
-mfg_status upload(DevArray<T>& d, const std::vector<T>& h, cudaStream_t s) {
-  MFG_CUDA(d.alloc(h.size()));
+mfg_status upload(DevArray<T>& d, const std::vector<T>& h, cudaStream_t s, size_t times = 1) {
+  MFG_CUDA(d.alloc(times * h.size()));
   if (!h.empty()) MFG_CUDA(cudaMemcpyAsync(d.p, h.data(), h.size() * sizeof(T), cudaMemcpyHostToDevice, s));
   return MFG_OK;
 }
 
 // FP64: chooses the cluster size for the batch (f64_cluster_size) and, when
-// it is above 1, builds and uploads the RVEs' parts (f64_parts). `m` holds
-// the masses, their reciprocals and m c, `l0` the lengths and their
-// reciprocals, `nt` and `et` apart.
-mfg_status plan_f64_clusters(mfg_batch* b, const std::vector<double>& m,
-                             const std::vector<double>& l0, const std::vector<int2>& conn,
+// it is above 1, builds and uploads the RVEs' parts (f64_parts).
+mfg_status plan_f64_clusters(mfg_batch* b, const std::vector<int2>& conn,
                              const std::vector<int32_t>& rowptr, const std::vector<int32_t>& inc,
                              cudaStream_t s) {
   int clusters[5] = {b->sms, 0, 0, 0, 0};
   for (int k = 1; k < 5; ++k)
     if (b->opt.max_cluster_ctas == 0 || 1 << k <= b->opt.max_cluster_ctas)
       clusters[k] = mfg::relax_f64_max_clusters(1 << k, mfg::kF64ClusterSmem, b->sms);
-  const int64_t nt = b->nt, et = b->et;
   std::vector<mfg::F64Parts> parts(b->R);  // per RVE, offsets from its own start
   int cl = 1;
   for (;;) {
@@ -469,12 +466,16 @@ mfg_status plan_f64_clusters(mfg_batch* b, const std::vector<double>& m,
   };
   const size_t o_part = take(static_cast<int64_t>(b->R) * cl, sizeof(mfg::F64Part));
   const size_t o_gnode = take(n.node, sizeof(int32_t));
-  const size_t o_mass = take(n.node, sizeof(mfg::F64Mass));
   const size_t o_rows = take(n.row, sizeof(int32_t));
   const size_t o_inc = take(n.inc, sizeof(int32_t));
   const size_t o_ends = take(n.fib, sizeof(int2));
+  // filled on the device; the fibers' slots, which it takes for that, go through
+  // the force vectors' scratch (24 bytes a fiber, at most two entries of 4 here)
+  const size_t uploaded = bytes;
+  const size_t o_mass = take(n.node, sizeof(mfg::F64Mass));
   const size_t o_len = take(n.fib, sizeof(mfg::F64Len));
-  std::vector<unsigned char> blob(bytes);
+  std::vector<unsigned char> blob(uploaded);
+  std::vector<int32_t> slot(n.fib);
   parallel_for(b->R, [&](int r) {
     mfg::F64Parts& p = parts[r];
     const mfg::RveDesc& d = b->desc[r];
@@ -494,16 +495,7 @@ mfg_status plan_f64_clusters(mfg_batch* b, const std::vector<double>& m,
     put(o_rows, at[r].row, p.rows);
     put(o_inc, at[r].inc, p.inc);
     put(o_ends, at[r].fib, p.ends);
-    mfg::F64Mass* mass = reinterpret_cast<mfg::F64Mass*>(&blob[o_mass]) + at[r].node;
-    for (size_t t = 0; t < p.gnode.size(); ++t) {
-      const int64_t i = d.node_off + p.gnode[t];
-      mass[t] = {m[i], mfg::bits_of(m[nt + i]), m[2 * nt + i]};
-    }
-    mfg::F64Len* len = reinterpret_cast<mfg::F64Len*>(&blob[o_len]) + at[r].fib;
-    for (size_t e = 0; e < p.slot.size(); ++e) {
-      const int64_t i = d.fiber_off + p.slot[e];
-      len[e] = {l0[i], mfg::bits_of(l0[et + i])};
-    }
+    std::copy(p.slot.begin(), p.slot.end(), slot.begin() + at[r].fib);
   });
   const cudaError_t e = b->d_plan.alloc(bytes);
   if (e == cudaErrorMemoryAllocation) {  // every RVE on one CTA: no more than it needs
@@ -511,8 +503,10 @@ mfg_status plan_f64_clusters(mfg_batch* b, const std::vector<double>& m,
     return MFG_OK;
   }
   MFG_CUDA(e);
-  MFG_CUDA(cudaMemcpyAsync(b->d_plan.p, blob.data(), bytes, cudaMemcpyHostToDevice, s));
-  MFG_CUDA(cudaStreamSynchronize(s));  // the blob goes out of scope
+  MFG_CUDA(cudaMemcpyAsync(b->d_plan.p, blob.data(), uploaded, cudaMemcpyHostToDevice, s));
+  int32_t* slots = reinterpret_cast<int32_t*>(b->d_nrm.p);
+  MFG_CUDA(cudaMemcpyAsync(slots, slot.data(), slot.size() * sizeof(int32_t),
+                           cudaMemcpyHostToDevice, s));
   mfg::F64Plan& plan = b->f64_plan;
   plan.cl = cl;
   plan.smem_bytes = mfg::kF64ClusterSmem;
@@ -526,13 +520,17 @@ mfg_status plan_f64_clusters(mfg_batch* b, const std::vector<double>& m,
   plan.threads = squares > mfg::kF64SmallParts * sum ? mfg::kF64ClusterThreads
                                                      : mfg::kF64SmallThreads;
   const unsigned char* base = b->d_plan.p;
+  mfg::F64Mass* mass = reinterpret_cast<mfg::F64Mass*>(b->d_plan.p + o_mass);
+  mfg::F64Len* len = reinterpret_cast<mfg::F64Len*>(b->d_plan.p + o_len);
   plan.part = reinterpret_cast<const mfg::F64Part*>(base + o_part);
   plan.gnode = reinterpret_cast<const int32_t*>(base + o_gnode);
-  plan.mass = reinterpret_cast<const mfg::F64Mass*>(base + o_mass);
+  plan.mass = mass;
   plan.rows = reinterpret_cast<const int32_t*>(base + o_rows);
   plan.inc = reinterpret_cast<const int32_t*>(base + o_inc);
   plan.ends = reinterpret_cast<const int2*>(base + o_ends);
-  plan.len = reinterpret_cast<const mfg::F64Len*>(base + o_len);
+  plan.len = len;
+  MFG_CUDA(mfg::launch_f64_plan(b->dev, plan, mass, len, slots, s));
+  MFG_CUDA(cudaStreamSynchronize(s));  // the blob and the slots go out of scope
   int k = 0;
   while (1 << k < cl) ++k;
   b->f64_clusters = clusters[k];
@@ -757,10 +755,8 @@ static mfg_status batch_create_impl(const mfg_network* nets, const mfg_strategy*
   const int64_t nt = no, et = fo;
 
   // ---- pack ------------------------------------------------------------
-  // FP64 batches: the masses' reciprocals (exact_reciprocal) and m c follow
-  // the masses, the lengths' reciprocals the lengths
   const bool f64 = b->precision == MFG_PREC_F64;
-  std::vector<double> X(3 * nt), m(f64 ? 3 * nt : nt), l0(f64 ? 2 * et : et);
+  std::vector<double> X(3 * nt), m(nt), l0(et);
   std::vector<int2> conn(et);
   std::vector<int32_t> rowptr(ro), inc(io), bnd(std::max<int64_t>(bo, 1));
   parallel_for(n_rve, [&](int r) {
@@ -774,14 +770,6 @@ static mfg_status batch_create_impl(const mfg_network* nets, const mfg_strategy*
     std::memcpy(&l0[d.fiber_off], s.l0.data(), s.n_fibers * sizeof(double));
     std::memcpy(&rowptr[d.row_off], s.rowptr.data(), (N + 1) * sizeof(int32_t));
     std::memcpy(&inc[d.inc_off], s.inc.data(), 2 * s.n_fibers * sizeof(int32_t));
-    if (f64) {
-      for (int i = 0; i < N; ++i) {
-        m[nt + d.node_off + i] = mfg::from_bits(mfg::exact_reciprocal(s.m[i]));
-        m[2 * nt + d.node_off + i] = s.m[i] * d.c;
-      }
-      for (int e = 0; e < s.n_fibers; ++e)
-        l0[et + d.fiber_off + e] = mfg::from_bits(mfg::exact_reciprocal(s.l0[e]));
-    }
     if (!s.bnd_order.empty())
       std::memcpy(&bnd[d.bnd_off], s.bnd_order.data(), s.bnd_order.size() * sizeof(int32_t));
   });
@@ -808,9 +796,11 @@ static mfg_status batch_create_impl(const mfg_network* nets, const mfg_strategy*
   MFG_CUDA(cudaMemsetAsync(b->d_v.p, 0, 3 * nt * sizeof(double), s));
   MFG_CUDA(b->d_fint.alloc(3 * nt));
   MFG_CUDA(cudaMemsetAsync(b->d_fint.p, 0, 3 * nt * sizeof(double), s));
-  if ((st = upload(b->d_m, m, s)) != MFG_OK) return st;
+  // FP64 batches: the masses' reciprocals and m c follow the masses, the
+  // lengths' reciprocals the lengths (launch_f64_divisors)
+  if ((st = upload(b->d_m, m, s, f64 ? 3 : 1)) != MFG_OK) return st;
   if ((st = upload(b->d_conn, conn, s)) != MFG_OK) return st;
-  if ((st = upload(b->d_l0, l0, s)) != MFG_OK) return st;
+  if ((st = upload(b->d_l0, l0, s, f64 ? 2 : 1)) != MFG_OK) return st;
   MFG_CUDA(b->d_nrm.alloc(3 * et));
   if ((st = upload(b->d_rowptr, rowptr, s)) != MFG_OK) return st;
   if ((st = upload(b->d_inc, inc, s)) != MFG_OK) return st;
@@ -860,9 +850,10 @@ static mfg_status batch_create_impl(const mfg_network* nets, const mfg_strategy*
     // so that mfg_batch_run_device_noalloc() never reserves it mid-solve.
     void* scratch = nullptr;
     MFG_CUDA(mfg::relax_f64_static_scratch_address(&scratch));
+    MFG_CUDA(mfg::launch_f64_divisors(dv, b->d_m.p, b->d_l0.p, s));
     // the serving kernel solves on single CTAs
     if (opt.cluster_layout != MFG_LAYOUT_SERVING &&
-        (st = plan_f64_clusters(b.get(), m, l0, conn, rowptr, inc, s)) != MFG_OK)
+        (st = plan_f64_clusters(b.get(), conn, rowptr, inc, s)) != MFG_OK)
       return st;
   }
   if (b->precision == MFG_PREC_MIXED) {

@@ -176,6 +176,13 @@ constexpr int kF64ClusterThreads = 512, kF64SmallThreads = 256;
 constexpr double kF64SmallParts = 288;  // fibers of a small part, at most
 cudaError_t launch_relax_f64_cluster(const DevBatch& b, const RunArgs& a, const F64Plan& plan,
                                      int grid, cudaStream_t s);
+// Set-up of a batch's divisors: the masses' reciprocals (exact_reciprocal) and
+// m c behind the nt masses at `m`, the lengths' behind the et lengths at `l0`;
+// and then a plan's masses and lengths from them, in the order of its nodes and
+// of `slot`, the fibers' slots in their RVE's storage order.
+cudaError_t launch_f64_divisors(const DevBatch& b, double* m, double* l0, cudaStream_t s);
+cudaError_t launch_f64_plan(const DevBatch& b, const F64Plan& plan, F64Mass* mass, F64Len* len,
+                            const int32_t* slot, cudaStream_t s);
 // Clusters of cl CTAs with smem_bytes of shared memory each that the device
 // holds at once (0 when it cannot run them).
 int relax_f64_max_clusters(int cl, int smem_bytes, int sms);
