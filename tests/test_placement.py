@@ -135,6 +135,15 @@ def test_few_move_beside_rves_that_need_a_cluster(place):
     assert 1 <= moved <= 8  # the longest; all 30 that would be faster alone cost throughput
 
 
+@pytest.mark.parametrize("sizes,need", [  # tests/test_gpu_serve_laws.py
+    (tuple(1_800 + 270 * i for i in range(13)), 0),
+    ((9_000, 5_900, 6_800, 5_000, 500, 700, 1_100, 4_100), 2)])
+def test_served_batches_of_both_laws_move_some(place, sizes, need):
+    placed = ctas(place([rve(n, i % 2, 3 + i % 3, 103) for i, n in enumerate(sizes)],
+                        serving=True)[1])
+    assert need < placed.count(4) < len(sizes)
+
+
 # ---- the GPU tests that compare placements ----------------------------------------------------
 
 @pytest.mark.parametrize("sizes,law,narrow", [
