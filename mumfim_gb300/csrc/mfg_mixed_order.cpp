@@ -37,6 +37,10 @@ void spread_banks(int32_t* order, int n, int owner_lo, int owner_hi, const int2*
     widest = std::max(widest, deg);
     total += deg;
   }
+  // a table of groups by widest row: mostly empty where one row is far wider
+  // than the others, whose nodes then read mostly one record anyway
+  const size_t sets = static_cast<size_t>((n + 7) / 8) * widest;
+  if (sets > 4 * static_cast<size_t>(total)) return;
   // the sets that each node's record is in: the k-th other ends of the group
   // of a neighbour of whose row it is the k-th; groups never change
   w.first.assign(n + 1, 0);
@@ -54,7 +58,7 @@ void spread_banks(int32_t* order, int n, int owner_lo, int owner_hi, const int2*
     }
   }
   // count[set]: its members by slot mod 8, one byte each (at most 8)
-  w.count.assign(static_cast<size_t>((n + 7) / 8) * widest, 0);
+  w.count.assign(sets, 0);
   auto add = [&](int j, uint64_t member) {
     for (int q = w.first[j - owner_lo]; q < end[j - owner_lo]; ++q) w.count[w.set[q]] += member;
   };
