@@ -108,6 +108,25 @@ def test_f64_cluster_size(place, rves, want):
     assert place(rves)[0] == want
 
 
+def test_staged_records_stay_within_their_bound(tmp_path):
+    gxx = shutil.which("g++")
+    if gxx is None:
+        pytest.skip("g++ not found")
+    from mumfim_gb300.build import _cuda_home
+    try:
+        cuda = _cuda_home()
+    except RuntimeError:
+        pytest.skip("CUDA headers not found")
+    exe = str(tmp_path / "stage_bound_check")
+    subprocess.run([gxx, "-O1", "-std=c++17", "-I" + CSRC, "-I" + os.path.join(ROOT, "include"),
+                    "-I" + os.path.join(cuda, "include"),
+                    os.path.join(HERE, "native", "stage_bound_check.cpp"),
+                    os.path.join(CSRC, "mfg_mixed_order.cpp"), "-o", exe], check=True)
+    r = subprocess.run([exe], capture_output=True, text=True, timeout=120)
+    assert r.returncode == 0, r.stdout + r.stderr
+    assert "bad=0" in r.stdout
+
+
 # ---- serving: RVEs that one CTA holds, on clusters of 4 ---------------------------------------
 
 def _spread(n, lo, hi):
