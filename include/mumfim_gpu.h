@@ -108,7 +108,8 @@ typedef struct mfg_strategy {
 /* Arithmetic of the solve. F64 is IEEE FP64 with the
  * reference's operation order and no contraction, bit-identical to a serial
  * CPU run of the same algorithm (on one CTA per RVE, or on clusters of 2 to 16
- * where the batch leaves SMs idle). MIXED runs fiber forces and the integrator in
+ * where the batch leaves SMs idle and they hold each of its RVEs: up to about
+ * 30,000 nodes). MIXED runs fiber forces and the integrator in
  * FP32 on top of FP64 reference coordinates plus Kahan-compensated FP32
  * displacements, and keeps FP64 for the stress, the residual and dt. */
 typedef enum mfg_precision { MFG_PREC_F64 = 0, MFG_PREC_MIXED = 1 } mfg_precision;

@@ -105,7 +105,7 @@ double f64_step_us(const RveDesc& d, int k) {
 
 }  // namespace
 
-double f64_batch_step_us(const std::vector<RveDesc>& desc, int k, int clusters, int copies) {
+double f64_batch_us(const std::vector<RveDesc>& desc, int k, int clusters, int copies) {
   // longest first onto the cluster that is free first, as the kernel's queue does
   std::vector<double> t;
   t.reserve(desc.size() * copies);
@@ -129,7 +129,7 @@ int f64_cluster_size(const std::vector<RveDesc>& desc, const int clusters[5], in
   double t_best = 0.0;
   for (int k = 0; k < 5; ++k) {
     if (clusters[k] < 1) continue;
-    const double t = f64_batch_step_us(desc, k, clusters[k], copies);
+    const double t = f64_batch_us(desc, k, clusters[k], copies);
     // a larger cluster has to be clearly faster
     if (k == 0 || t < 0.95 * t_best) {
       best = k;

@@ -40,12 +40,12 @@ inline int64_t f64_part_bytes(const F64Part& p) {
 }
 
 // Cluster size for the FP64 solve of `copies` solves each of these RVEs at
-// once, by an estimate of the time of a step (f64_order.cpp); `clusters[k]`
-// is the number of clusters of 2^k CTAs the device holds at once (0: not
-// available).
+// once, by the estimate below; `clusters[k]` is the number of clusters of 2^k
+// CTAs the device holds at once (0: not available).
 int f64_cluster_size(const std::vector<RveDesc>& desc, const int clusters[5], int copies);
-// The estimate: time of a step of the whole batch in clusters of 2^k CTAs.
-double f64_batch_step_us(const std::vector<RveDesc>& desc, int k, int clusters, int copies);
+// The estimate: time of the solves of the whole batch, all their steps, in
+// clusters of 2^k CTAs, `clusters` at once.
+double f64_batch_us(const std::vector<RveDesc>& desc, int k, int clusters, int copies);
 
 }  // namespace mfg
 

@@ -535,8 +535,8 @@ mfg_status plan_f64_clusters(mfg_batch* b, const std::vector<int2>& conn,
   while (1 << k < cl) ++k;
   b->f64_clusters = clusters[k];
   b->f64_stiffness_clusters =
-      mfg::f64_batch_step_us(b->desc, k, clusters[k], kStiffSlots) <
-      mfg::f64_batch_step_us(b->desc, 0, b->sms, kStiffSlots);
+      mfg::f64_batch_us(b->desc, k, clusters[k], kStiffSlots) <
+      mfg::f64_batch_us(b->desc, 0, b->sms, kStiffSlots);
   return MFG_OK;
 }
 
