@@ -44,10 +44,10 @@
 // cluster run fiber-centric on one CTA, placed by size at run time down to
 // global memory.
 #include <algorithm>
+#include <atomic>
 #include <cfloat>
 #include <cmath>
-#include <functional>
-#include <queue>
+#include <numeric>
 #include <thread>
 #include <type_traits>
 #include <vector>
@@ -1853,17 +1853,29 @@ cudaError_t mixed_create(MixedState& ms, const DevBatch& b, const std::vector<Rv
     // fiber order and codes of the cluster-solved RVEs
     std::vector<int2> econn(et);
     std::vector<int32_t> icode(2 * et), mslot(et), gnode(nt), mrowptr(rowptr.size());
-    std::vector<std::thread> pool;
-    const int nthr = static_cast<int>(std::max<size_t>(
-        1, std::min<size_t>({16, std::thread::hardware_concurrency(), desc.size()})));
-    for (int t = 0; t < nthr; ++t)
-      pool.emplace_back([&, t] {
-        for (size_t r = t; r < desc.size(); r += nthr)
-          cluster_order(desc[r], kind_of(r).cl, kind_of(r).all || kind_of(r).nodal,
-                        kind_of(r).nodal, conn, rowptr, inc, econn, icode, mslot, gnode,
-                        mrowptr);
-      });
-    for (auto& th : pool) th.join();
+    // RVE after RVE on the host's cores, the largest first: a batch of few has
+    // some many times as large as others (32 RVEs of 500 - 20,000 nodes dealt out
+    // in turn took 6.5 ms here, 5.1 so)
+    std::vector<int32_t> by_size(desc.size());
+    std::iota(by_size.begin(), by_size.end(), 0);
+    std::stable_sort(by_size.begin(), by_size.end(),
+                     [&](int32_t x, int32_t y) { return desc[x].n_fibers > desc[y].n_fibers; });
+    const size_t nthr = std::max<size_t>(
+        1, std::min<size_t>({16, std::thread::hardware_concurrency(), desc.size()}));
+    auto each_rve = [&](auto fn) {
+      std::atomic<size_t> next{0};
+      std::vector<std::thread> pool;
+      for (size_t t = 0; t < nthr; ++t)
+        pool.emplace_back([&] {
+          for (size_t k = next++; k < by_size.size(); k = next++)
+            fn(static_cast<size_t>(by_size[k]));
+        });
+      for (auto& th : pool) th.join();
+    };
+    each_rve([&](size_t r) {
+      cluster_order(desc[r], kind_of(r).cl, kind_of(r).all || kind_of(r).nodal, kind_of(r).nodal,
+                    conn, rowptr, inc, econn, icode, mslot, gnode, mrowptr);
+    });
     if ((e = cudaMemcpy(ms.econn, econn.data(), et * sizeof(int2), cudaMemcpyHostToDevice)) !=
             cudaSuccess ||
         (e = cudaMemcpy(ms.icode, icode.data(), 2 * et * sizeof(int32_t),
@@ -1878,34 +1890,22 @@ cudaError_t mixed_create(MixedState& ms, const DevBatch& b, const std::vector<Rv
 
     // SELL incidence blocks of the node-centric RVEs
     std::vector<int64_t> sell_off(desc.size() + 1, 0);
-    {
-      std::vector<std::thread> sp;
-      for (int t = 0; t < nthr; ++t)
-        sp.emplace_back([&, t] {
-          for (size_t r = t; r < desc.size(); r += nthr)
-            if (kind_of(r).nodal)
-              sell_off[r + 1] = sell_layout(desc[r], kind_of(r).cl, conn, rowptr, inc,
-                                            gnode, 0, nullptr, nullptr, nullptr);
-        });
-      for (auto& th : sp) th.join();
-    }
+    each_rve([&](size_t r) {
+      if (kind_of(r).nodal)
+        sell_off[r + 1] = sell_layout(desc[r], kind_of(r).cl, conn, rowptr, inc, gnode, 0, nullptr,
+                                      nullptr, nullptr);
+    });
     for (size_t r = 0; r < desc.size(); ++r) sell_off[r + 1] += sell_off[r];
     const int64_t n_sell = sell_off[desc.size()];
     ms.n_sell = n_sell;
     std::vector<int2> nsell(nt, make_int2(0, 0));
     std::vector<int32_t> ncode(static_cast<size_t>(n_sell), 0);
     std::vector<int64_t> nfib(static_cast<size_t>(n_sell), -1);
-    {
-      std::vector<std::thread> sp;
-      for (int t = 0; t < nthr; ++t)
-        sp.emplace_back([&, t] {
-          for (size_t r = t; r < desc.size(); r += nthr)
-            if (kind_of(r).nodal)
-              sell_layout(desc[r], kind_of(r).cl, conn, rowptr, inc, gnode, sell_off[r],
-                          nsell.data(), ncode.data(), nfib.data());
-        });
-      for (auto& th : sp) th.join();
-    }
+    each_rve([&](size_t r) {
+      if (kind_of(r).nodal)
+        sell_layout(desc[r], kind_of(r).cl, conn, rowptr, inc, gnode, sell_off[r], nsell.data(),
+                    ncode.data(), nfib.data());
+    });
     // the incidence records of each CTA's free nodes
     std::vector<int2> sell_cta(desc.size() * kMaxCluster, make_int2(0, 0));
     for (size_t r = 0; r < desc.size(); ++r) {
