@@ -12,7 +12,7 @@ pytestmark = pytest.mark.gpu
     ((60, 1_400), 0),                # 8 CTAs, split, linear
     ((60, 500, 1_400, 1_400), 2),    # 4 CTAs, not split; 16, split, nonlinear
     ((60,) + (1_400,) * 20, 0),      # 4 CTAs, not split
-    ((300, 300), 1),                 # 16 CTAs, split, nonlinear
+    ((200, 200), 1),                 # 8 CTAs, split, nonlinear
 ])
 @pytest.mark.parametrize("relax", [False, True])
 def test_tiny_parts_match_one_cta(lib_path, sizes, law, relax):

@@ -81,6 +81,20 @@ def test_batches_that_fill_the_gpu_are_not_widened(place):
     assert ctas(place([rve(19_500)] * 36)[1]) == [4] * 36  # one wave
 
 
+@pytest.mark.parametrize("n", [150, 300])
+def test_small_nonlinear_rves_share_ctas_where_clusters_of_2_remain(place, n):
+    # 38 to 76 RVEs leave room for 2 CTAs each, on which the longest row's chain
+    # takes longer than two RVEs side by side on one
+    for rves in (48, 64, 76):
+        assert ctas(place([rve(n, 1)] * rves)[1]) == [1] * rves
+    assert ctas(place([rve(n, 1)] * 32)[1]) == [4] * 32  # four lanes to a node
+
+
+def test_few_steps_do_not_pay_for_a_cluster(place):
+    assert ctas(place([rve(300, 1, steps=20)])[1]) == [1]
+    assert ctas(place([rve(300, 1, steps=400)])[1]) == [8]
+
+
 def test_widest_cluster_is_limited(place):
     for limit in (1, 2, 4, 8):
         for rves in ([rve(4_500)], [rve(900, 1), rve(3_000, 1)], [rve(20_000)] * 3):
@@ -193,7 +207,7 @@ def test_tiny_rves_alone_stay_on_one_cta(place):
 
 @pytest.mark.parametrize("sizes,law,split,cl", [  # tests/test_gpu_tiny_parts.py
     ((60, 1_400), 0, LINEAR, 8), ((60, 500, 1_400, 1_400), 2, NONE, 4),
-    ((60,) + (1_400,) * 20, 0, NONE, 4), ((300, 300), 1, NONLINEAR, 16)])
+    ((60,) + (1_400,) * 20, 0, NONE, 4), ((200, 200), 1, NONLINEAR, 8)])
 def test_parts_of_fewer_nodes_than_a_warp(place, sizes, law, split, cl):
     placed = place([rve(n, i % 2 if law == 2 else law, 4, 202) for i, n in enumerate(sizes)])[1]
     assert placed[0][0] == cl and placed[0][4] == split and sizes[0] / cl < 32
