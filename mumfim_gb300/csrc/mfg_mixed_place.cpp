@@ -82,16 +82,7 @@ double step_us(const RveDesc& d, const BucketKind& k) {
       per_fiber * d.n_fibers / k.cl + fixed[k.db + k.stage][log2_cl] + (nl ? 0.9 : 0.0);
   // the nonlinear law along the longest row, however few nodes a part has: 48
   // RVEs of 150, 300, 450 nodes on 2 CTAs 3.8 us a step each; two to a CTA 2.5, 3.4, 4.2
-  return nl ? std::max(t, 3.8) : t;
-}
-
-// The same for all its steps, with what a solve costs besides: node-centric on
-// the nonlinear law 28 us more than fiber-centric (one RVE of 300 nodes, one
-// step: 69 us on its CTA, 96, 99, 107 on 4, 8, 16).
-double solve_us(const RveDesc& d, const BucketKind& k) {
-  const bool nl = d.law == MFG_LAW_NONLINEAR;
-  return step_us(d, k) * d.max_steps + (k.nodal && nl ? 28.0 : 0.0) +
-         (k.cl == 16 ? 11.0 : (k.cl == 8 ? 3.0 : 0.0));
+  return nl && k.cl == 2 ? std::max(t, 3.8) : t;
 }
 
 // Time of `copies` solves of the batch with the buckets in these kinds: RVE
@@ -118,7 +109,7 @@ double batch_us(const std::vector<RveDesc>& desc, const std::vector<std::vector<
     for (size_t i = 0; i < n; i += k.ng) {
       const RveDesc& d = desc[bucket[q][i / copies]];
       // two RVEs side by side on a CTA take 1.4 times as long as one there
-      const double t = solve_us(d, k) * (i + 1 < n && k.ng == 2 ? 1.4 : 1.0);
+      const double t = step_us(d, k) * d.max_steps * (i + 1 < n && k.ng == 2 ? 1.4 : 1.0);
       double start = sm[share - 1];
       if (ends.size() == most) {  // one of the kind has to end first
         start = std::max(start, ends.top());
@@ -193,7 +184,7 @@ void choose_kinds(const std::vector<RveDesc>& desc,
     double longest = 0.0;
     for (int q = 0; q < kBuckets; ++q)
       for (int32_t r : bucket[q]) {
-        const double t = solve_us(desc[r], kKind[now[q]]);
+        const double t = step_us(desc[r], kKind[now[q]]) * desc[r].max_steps;
         if (t > longest) {
           longest = t;
           q_long = q;

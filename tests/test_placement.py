@@ -90,11 +90,6 @@ def test_small_nonlinear_rves_share_ctas_where_clusters_of_2_remain(place, n):
     assert ctas(place([rve(n, 1)] * 32)[1]) == [4] * 32  # four lanes to a node
 
 
-def test_few_steps_do_not_pay_for_a_cluster(place):
-    assert ctas(place([rve(300, 1, steps=20)])[1]) == [1]
-    assert ctas(place([rve(300, 1, steps=400)])[1]) == [8]
-
-
 def test_widest_cluster_is_limited(place):
     for limit in (1, 2, 4, 8):
         for rves in ([rve(4_500)], [rve(900, 1), rve(3_000, 1)], [rve(20_000)] * 3):
