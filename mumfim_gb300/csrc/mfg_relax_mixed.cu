@@ -332,7 +332,11 @@ struct ClusterOps {
   }
   // Combines a block-reduced value over the cluster in fixed rank order, so
   // every CTA gets the same bits.
-  template <bool kMin>
+  // kRolled: one CTA's value after another. For clusters above 4 with two record
+  // copies the unrolled loop costs a hundredth of a step (spills); with one copy
+  // the rolled one costs 6 to 8 (one RVE of 80,000 nodes on 16 CTAs, 400 steps:
+  // 5.74 ms, 5.40 unrolled; of 30,000 on 8: 4.48, 4.12).
+  template <bool kMin, bool kRolled = false>
   __device__ static double combine(double part, double* slot) {
     if constexpr (CL == 1) {
       return part;
@@ -341,7 +345,7 @@ struct ClusterOps {
       if (threadIdx.x == 0) *slot = part;
       cl.sync();
       double t = kMin ? DBL_MAX : 0.0;
-#pragma unroll(CL <= 4 ? CL : 1)
+#pragma unroll(kRolled ? 1 : CL)
       for (int o = 0; o < CL; ++o) {
         const double v = *cl.map_shared_rank(slot, o);
         t = kMin ? fmin(t, v) : t + v;
@@ -1228,7 +1232,7 @@ __device__ void solve_rve_nodal(const DevBatch& b, const MixedState& ms, const R
     Rve fibers;
     fibers.conn = kStage ? r.conn : ms.econn + dr.fiber_off;
     fibers.fcon = kStage ? r.fcon : ms.fconc + dr.fiber_off;
-    const double dt_crit = Ops::template combine<true>(
+    const double dt_crit = Ops::template combine<true, (kDB && CL > 4)>(
                                block_min<kThreadsMixed>(length_pass(fibers, u, e_lo, e_hi), red),
                                cred) /
                            dr.sound_speed;
@@ -1270,7 +1274,7 @@ __device__ void solve_rve_nodal(const DevBatch& b, const MixedState& ms, const R
                                         &nxt, h2);
     }
     if (res_step) {
-      residual = sqrt(Ops::template combine<false>(block_sum<kThreadsMixed>(part, red), cred));
+      residual = sqrt(Ops::template combine<false, (kDB && CL > 4)>(block_sum<kThreadsMixed>(part, red), cred));
       // a break keeps the copy of the step's start: the drift is dropped
       if (!isfinite(residual)) {
         status = 4;
