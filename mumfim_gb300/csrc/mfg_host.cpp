@@ -861,7 +861,7 @@ static mfg_status batch_create_impl(const mfg_network* nets, const mfg_strategy*
     if (e != cudaSuccess)
       return fail(e == cudaErrorMemoryAllocation ? MFG_E_OOM : MFG_E_CUDA,
                   "mixed-precision set-up failed: %s", cudaGetErrorString(e));
-    if (mfg::mixed_widened(*b->mixed) && opt.stiffness != MFG_STIFFNESS_SEQUENTIAL &&
+    if (mfg::mixed_contexts_differ(*b->mixed) && opt.stiffness != MFG_STIFFNESS_SEQUENTIAL &&
         (b->all_ramp || opt.stiffness == MFG_STIFFNESS_CONCURRENT))
       b->stiff_inputs.reset(new StiffInputs{std::move(conn), std::move(rowptr), std::move(inc)});
   }

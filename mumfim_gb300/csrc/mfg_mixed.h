@@ -50,8 +50,9 @@ void mixed_destroy(MixedState* ms);
 // `small` ring CTA by CTA.
 cudaError_t launch_server_mixed(MixedState& ms, const DevBatch& b, const ServerArgs& small,
                                 const ServerArgs* big, cudaStream_t s);
-// Whether some bucket of the batch took wider clusters than its RVEs need.
-bool mixed_widened(const MixedState& ms);
+// Whether the batch's own runs take other launch kinds than runs on contexts 1,
+// 2, ... all at once should: wider clusters than six solves side by side.
+bool mixed_contexts_differ(const MixedState& ms);
 // Cluster size of an RVE's batch bucket, and whether the serving kernel
 // solves it as a cluster.
 int mixed_rve_cluster(const MixedState& ms, int rve);

@@ -139,6 +139,7 @@ struct MixedState {
   // per context for the last run arguments and replayed while they stay
   // the same.
   MixedRunCtx* ctx = nullptr;
+  bool contexts_differ = false;  // mixed_contexts_differ()
 };
 
 namespace {
@@ -1818,6 +1819,15 @@ cudaError_t mixed_create(MixedState& ms, const DevBatch& b, const std::vector<Rv
   if (widen)
     choose_kinds(desc, bucket, rowptr, smem_floats, max_cluster, small_solve == MFG_SMALL_FIBER_CENTRIC,
                  clusters, sms, copies, ms.bucket_kind);
+  if (widen && copies == 1) {  // and as many solves at once as there are further contexts
+    int kind[kBuckets];
+    for (int q = 0; q < kBuckets; ++q) kind[q] = q;
+    if (may_widen(bucket, sms, serving_layout, kMixedContexts - 1))
+      choose_kinds(desc, bucket, rowptr, smem_floats, max_cluster,
+                   small_solve == MFG_SMALL_FIBER_CENTRIC, clusters, sms, kMixedContexts - 1, kind);
+    for (int q = 0; q < kBuckets; ++q)
+      ms.contexts_differ = ms.contexts_differ || (!bucket[q].empty() && kind[q] != ms.bucket_kind[q]);
+  }
   ms.h_cl = new int32_t[std::max<size_t>(desc.size(), 1)];
   for (size_t r = 0; r < desc.size(); ++r) ms.h_cl[r] = kKind[ms.bucket_kind[rve_q[r]]].cl;
   auto kind_of = [&](size_t r) -> const BucketKind& { return kKind[ms.bucket_kind[rve_q[r]]]; };
@@ -1995,13 +2005,7 @@ cudaError_t mixed_create(MixedState& ms, const DevBatch& b, const std::vector<Rv
   return cudaSuccess;
 }
 
-bool mixed_widened(const MixedState& ms) {
-  for (int q = 0; q < kBuckets; ++q)
-    if (ms.bucket_off[q + 1] > ms.bucket_off[q] && ms.bucket_kind[q] != q &&
-        kKind[ms.bucket_kind[q]].cl > kKind[q].cl)
-      return true;
-  return false;
-}
+bool mixed_contexts_differ(const MixedState& ms) { return ms.contexts_differ; }
 
 int mixed_rve_cluster(const MixedState& ms, int rve) { return ms.h_cl ? ms.h_cl[rve] : 1; }
 

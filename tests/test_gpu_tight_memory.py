@@ -101,6 +101,22 @@ stress(g, n)
 assert np.isfinite(g.computeMaterialStiffness()).all()
 """
 
+# one RVE: six solves of it fit beside one another on the clusters that one takes,
+# so they need the batch's working set and six sets of what a solve writes
+ONE_RVE_STIFFNESS = PRELUDE + """
+g, plain = batch((4_500,), "mixed")
+stress(g, 1)
+before = L.fake_memory_held()
+C = g.computeMaterialStiffness()
+nodes, fibers = g.n_nodes(0), g.n_fibers(0)
+scratch = 6 * (72 * nodes + 24 * fibers + 48 * nodes)  # (boundary: at most every node)
+assert L.fake_memory_held() - before < scratch + 4096
+g.close()
+g, _ = batch((4_500,), "mixed", max_cluster_ctas=1)
+stress(g, 1)
+np.testing.assert_array_equal(g.computeMaterialStiffness(), C)
+"""
+
 
 @pytest.fixture(scope="module")
 def limited_library(lib_path, tmp_path_factory):
@@ -125,6 +141,10 @@ def _run(script, library):
 
 def test_f64_batch_without_room_for_clusters(limited_library):
     _run(F64_PLAN, limited_library)
+
+
+def test_stiffness_of_one_rve_shares_the_working_set(limited_library):
+    _run(ONE_RVE_STIFFNESS, limited_library)
 
 
 def test_f64_clusters_keep_to_the_limit(limited_library):
